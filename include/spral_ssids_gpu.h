@@ -291,6 +291,19 @@ int spral_ssids_gpu_tc_gemm_f32_bn(int M, int N, int K, const float* A, int lda,
                                    int ldb, float* C, int ldc, int lower, int chunk, int reps,
                                    float* ms, int bn);
 
+/* FP64 trailing update on the tensor cores, the kernel of the numeric
+ * factorisation's FP64 contribution blocks, exposed for tests and
+ * measurements: C (M x N, N <= M, column-major, ldc) -= A B^T on the lower
+ * trapezoid (row >= column) with A (M x K) and B (N x K) column-major FP64
+ * device arrays, applied reps times on the caller's stream.  The products are
+ * exact bf16 slice products summed exactly; the result differs from the exact
+ * update by about 2^-62 sqrt(K) of (row maximum of A) x (row maximum of B)
+ * and the rounding of C.  Allocates its workspace and synchronises the
+ * stream.  Returns 0, -1 bad argument, -50 allocation, -51 CUDA error, -52
+ * pipeline timeout.  No reference counterpart. */
+int spral_ssids_gpu_slice_gemm_f64(int M, int N, int K, const double* A, int lda, const double* B,
+                                   int ldb, double* C, int ldc, int reps, void* stream);
+
 /* Per-node inertia of the last factorisation: out[3*node + {0, 1, 2}] =
  * (negative eigenvalues, 2x2 pivots, zero pivots) of each node's D, nodes
  * numbered 0-based as in the symbolic subtree.  Batched factorisations of

@@ -110,6 +110,7 @@ def _declare(L):
       ctypes.POINTER(CpuFactorOptions), P)
     f("spral_ssids_gpu_tc_gemm_f32", I, I, I, I, P, I, P, I, P, I, I, I, I, P)
     f("spral_ssids_gpu_tc_gemm_f32_bn", I, I, I, I, P, I, P, I, P, I, I, I, I, P, I)
+    f("spral_ssids_gpu_slice_gemm_f64", I, I, I, I, P, I, P, I, P, I, I, P)
     f("spral_ssids_gpu_tune_table", I, P, I)
     f("spral_ssids_gpu_group_bwd_errors", I, P, P, I)
     f("spral_ssids_gpu_tune_device_key", I, ctypes.c_char_p, I)

@@ -991,6 +991,16 @@ struct Numeric : NumericBase {
   // refinement a step)
   int panel_min_n = 4096;
   DevBuf<int> panel_list;   // fronts ending a panel (eager mode)
+  // FP64 factors: contribution blocks and panels' trailing updates from exact
+  // bf16 slice products on the tensor cores (slice_gemm.cu).  From
+  // slice_min_k pivots on they beat the SIMT kernel at every block size: a
+  // 64 x 64 SIMT tile takes 39 us for 32 columns whatever the block, the
+  // three slice launches 31 us (one block of 32 .. 1024 rows; 2048 rows:
+  // 44 us against 143 us, and 227 us against 4125 us for 1024 columns).
+  bool use_slices = false;
+  int slice_min_cm = 16, slice_min_k = 32;
+  DevBuf<char> slice_tab, slice_scratch;
+  static constexpr size_t kSliceScratch = size_t(256) << 20;
   int* d_tc_status = nullptr;
   int* d_ncount = nullptr;  // per-node inertia counts (neg, two, zero)
 
@@ -1013,7 +1023,7 @@ struct Numeric : NumericBase {
   // runs once per panel on the tensor cores with the panel's pivots as its
   // depth.  Returns the panel width of front f, or 0.
   int panel_cols(int f) const {
-    if (!std::is_same<T, float>::value || !use_tc || panel_nb <= 0) return 0;
+    if (!(std::is_same<T, float>::value ? use_tc : use_slices) || panel_nb <= 0) return 0;
     if (tpp_front(f) || S->copts.pivot_method == 3) return 0;
     return n_[f] >= std::max(panel_min_n, panel_nb + 1) ? panel_nb : 0;
   }
@@ -1048,6 +1058,7 @@ struct Numeric : NumericBase {
   }
   // end of panels in eager mode: the panels' geometry is read back (failed
   // columns move panel boundaries), then the trailing updates and the close
+  // (the slice kernels take it from the device: FP64 factors read nothing back)
   void panel_end_eager(const std::vector<int>& fl, cudaStream_t s) {
     const int nfl = (int)fl.size();
     panel_list.ensure(nfl);
@@ -1055,6 +1066,11 @@ struct Numeric : NumericBase {
     int max_n = 0;
     for (int f : fl) max_n = std::max(max_n, n_[f]);
     launch_panel_end<T>(d_fd, d_st, panel_list.p, nfl, max_n, panel_nb, s);
+    if (use_slices) {
+      slice_run(slice_panels(fl), s);
+      launch_panel_close<T>(d_fd, d_st, panel_list.p, nfl, s);
+      return;
+    }
     for (int f : fl)
       CK(cudaMemcpyAsync(&hst[f], &d_st[f], sizeof(FrontState), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
@@ -1076,6 +1092,123 @@ struct Numeric : NumericBase {
       if (profile) { prof_tc_ms += ms_gemm; prof_tc_launches += 1; prof_tc_flops += fl_tc; }
     }
     launch_panel_close<T>(d_fd, d_st, panel_list.p, nfl, s);
+  }
+
+  // Slice jobs in launch groups: fronts in list order, a group's buffers
+  // within kSliceScratch (or one job alone), the k ranges of a deep front in
+  // consecutive rounds.  Grouping never changes a front's result.
+  struct SliceBatch {
+    std::vector<SliceJob> jobs;
+    std::vector<size_t> first;  // of each group, then jobs.size()
+    size_t scratch = 0, table = 0;
+  };
+  void slice_groups(SliceBatch& b) const {
+    b.first.clear();
+    b.scratch = b.table = 0;
+    size_t used = 0;
+    for (size_t i = 0; i < b.jobs.size(); ++i) {
+      const SliceJob& j = b.jobs[i];
+      const size_t need = slice_job_bytes(j.mcap, j.ncap, j.kcap);
+      if (b.first.empty() || used + need > kSliceScratch || j.k0 != b.jobs[i - 1].k0 ||
+          i - b.first.back() >= 32768) {
+        b.first.push_back(i);
+        used = 0;
+      }
+      used += need;
+      b.scratch = std::max(b.scratch, used);
+    }
+    b.first.push_back(b.jobs.size());
+    for (size_t g = 0; g + 1 < b.first.size(); ++g)
+      b.table += slice_table_bytes((int)(b.first[g + 1] - b.first[g]));
+  }
+  int cm_of(int f) const { return S->nrow[S->node_of[f]] - S->ncol[S->node_of[f]]; }
+  bool slice_front(int f) const {
+    return use_slices && !tpp_front(f) && cm_of(f) >= slice_min_cm && n_[f] >= slice_min_k;
+  }
+  SliceBatch slice_contrib(int f0, int f1) const {
+    SliceBatch b;
+    int deep = 0;
+    for (int f = f0; f < f1; ++f)
+      if (slice_front(f)) deep = std::max(deep, n_[f]);
+    for (int k0 = 0; k0 < deep; k0 += kSliceMaxK)
+      for (int f = f0; f < f1; ++f) {
+        if (!slice_front(f) || k0 >= n_[f]) continue;
+        SliceJob j{};
+        j.front = f;
+        j.kind = kSliceContrib;
+        j.k0 = k0;
+        j.kcap = std::min(kSliceMaxK, n_[f] - k0);
+        j.mcap = j.ncap = cm_of(f);
+        b.jobs.push_back(j);
+      }
+    slice_groups(b);
+    return b;
+  }
+  SliceBatch slice_panels(const std::vector<int>& fl) const {
+    SliceBatch b;
+    for (int f : fl) {
+      SliceJob j{};
+      j.front = f;
+      j.kind = kSlicePanel;
+      j.kcap = panel_nb;
+      j.mcap = m_[f];
+      j.ncap = n_[f];
+      b.jobs.push_back(j);
+    }
+    slice_groups(b);
+    return b;
+  }
+  // lays the batch out in slice_scratch and returns its tables' image
+  std::vector<char> slice_place(SliceBatch& b) const {
+    std::vector<char> img(b.table, 0);
+    size_t off = 0;
+    for (size_t g = 0; g + 1 < b.first.size(); ++g) {
+      char* q = slice_scratch.p;
+      for (size_t i = b.first[g]; i < b.first[g + 1]; ++i) {
+        slice_job_place(b.jobs[i], q);
+        q += slice_job_bytes(b.jobs[i].mcap, b.jobs[i].ncap, b.jobs[i].kcap);
+      }
+      const size_t cnt = b.first[g + 1] - b.first[g];
+      memcpy(img.data() + off, &b.jobs[b.first[g]], cnt * sizeof(SliceJob));
+      off += slice_table_bytes((int)cnt);
+    }
+    return img;
+  }
+  void slice_enqueue(const SliceBatch& b, char* table, cudaStream_t s) {
+    if constexpr (std::is_same<T, double>::value) {
+      for (size_t g = 0; g + 1 < b.first.size(); ++g) {
+        const size_t cnt = b.first[g + 1] - b.first[g];
+        if (launch_slice_gemm(table, b.jobs, b.first[g], cnt, d_fd, d_st, d_tc_status, s) != 0)
+          throw CudaFail{cudaGetLastError(), __LINE__};
+        table += slice_table_bytes((int)cnt);
+      }
+    }
+  }
+  // The slices' memory for the fronts of a level whose sizes are known; a
+  // device too full for it keeps the SIMT kernels (false, for this handle).
+  bool slice_reserve(int f0, int f1) {
+    std::vector<int> pf;
+    for (int f = f0; f < f1; ++f)
+      if (panel_cols(f)) pf.push_back(f);
+    const size_t need = std::max(slice_contrib(f0, f1).scratch, slice_panels(pf).scratch);
+    try {
+      slice_scratch.ensure(need + 1);
+    } catch (CudaFail const& e) {
+      if (e.err != cudaErrorMemoryAllocation) throw;
+      cudaGetLastError();
+      slice_scratch.cap = 0;
+      return false;
+    }
+    return true;
+  }
+  // eager mode: tables uploaded now, then the launches
+  void slice_run(SliceBatch b, cudaStream_t s) {
+    if (b.jobs.empty()) return;
+    slice_scratch.ensure(b.scratch);
+    slice_tab.ensure(b.table);
+    const std::vector<char> img = slice_place(b);
+    CK(cudaMemcpyAsync(slice_tab.p, img.data(), img.size(), cudaMemcpyHostToDevice, s));
+    slice_enqueue(b, slice_tab.p, s);
   }
 
   // shared-memory staging of a small leaf front (k_tpp_small): the front,
@@ -1119,6 +1252,7 @@ struct Numeric : NumericBase {
 
   std::vector<TcProblem> tc_problems(int f0, int f1) const {
     std::vector<TcProblem> ps;
+    if (use_slices) return ps;
     for (int f = f0; f < f1; ++f) {
       const FrontDesc<T>& d = hfd[f];
       if (!d.tc) continue;
@@ -1180,7 +1314,7 @@ struct Numeric : NumericBase {
 
   std::vector<const void*> graph_key() const {
     return {aval_buf.p, scale_buf.p, ws_W.p, ws_swap.p, ws_LD.p, ws_step.p, ws_lperm.p,
-            contrib.p,  tc_scratch.p, d_fd,  d_st,      d_stats, d_ncount};
+            contrib.p,  tc_scratch.p, d_fd,  d_st,      d_stats, d_ncount, slice_scratch.p};
   }
 
   void build_fgraph(bool scaled) {
@@ -1240,7 +1374,7 @@ struct Numeric : NumericBase {
         d.LD = ws_LD.p + oL; oL += (size_t)std::max(d.cm, panel_cols(f)) * d.n;
         d.step = ws_step.p + (size_t)(f - f0) * (kBlk * kBlk + 2 * kBlk + 64);
         d.lperm = ws_lperm.p + (size_t)(f - f0) * kBlk;
-        d.tc = (use_tc && d.cm >= tc_min_cm && d.n >= tc_min_k) ? 1 : 0;
+        d.tc = (slice_front(f) || (use_tc && d.cm >= tc_min_cm && d.n >= tc_min_k)) ? 1 : 0;
         d.panel = panel_cols(f);
       }
     }
@@ -1254,6 +1388,7 @@ struct Numeric : NumericBase {
     std::vector<PanelStep> psteps;
     std::vector<int> plist;
     std::vector<std::vector<TcProblem>> pps;
+    std::vector<SliceBatch> sps;  // FP64: slice jobs per panel end, then per level
     {
       const int per = std::max(panel_nb / kBlk, 1);
       std::vector<int> pfl;
@@ -1272,9 +1407,13 @@ struct Numeric : NumericBase {
             ps.max_n = std::max(ps.max_n, n_[f]);
             const int j = st / per, pstart = j * panel_nb;
             const int q = std::min((j + 1) * panel_nb, n_[f]);
-            if (q < n_[f]) pr.push_back(panel_problem(f, pstart, q, q - pstart));
+            if (q < n_[f] && !use_slices) pr.push_back(panel_problem(f, pstart, q, q - pstart));
           }
           if (!pr.empty()) { ps.pp = (int)pps.size(); pps.push_back(pr); }
+          if (use_slices) {
+            ps.pp = (int)sps.size();
+            sps.push_back(slice_panels(pfl));
+          }
           psteps.push_back(ps);
         }
       }
@@ -1311,6 +1450,31 @@ struct Numeric : NumericBase {
       for (int l = 0; l < S->nlev; ++l)
         if (!lps[l].empty()) tblob[l] = upload_plan(lps[l], tplans[l]);
       for (size_t i = 0; i < pps.size(); ++i) pblob[i] = upload_plan(pps[i], pplans[i]);
+    }
+    // slice job tables (FP64), one device blob for all of them
+    const size_t npsl = sps.size();
+    std::vector<size_t> soff;
+    char* sblob = nullptr;
+    if (use_slices) {
+      for (int l = 0; l < S->nlev; ++l)
+        sps.push_back(slice_contrib(S->lvl_start[l], S->lvl_start[l + 1]));
+      size_t scr = 0, tab = 0;
+      for (auto& b : sps) {
+        scr = std::max(scr, b.scratch);
+        soff.push_back(tab);
+        tab += b.table;
+      }
+      slice_scratch.ensure(scr + 1);
+      void* b = nullptr;
+      CK(cudaMalloc(&b, std::max<size_t>(tab, 1)));
+      fgraph_blobs.push_back(b);
+      sblob = static_cast<char*>(b);
+      std::vector<char> img(tab);
+      for (size_t i = 0; i < sps.size(); ++i) {
+        const std::vector<char> one = slice_place(sps[i]);
+        if (!one.empty()) memcpy(img.data() + soff[i], one.data(), one.size());
+      }
+      if (tab) CK(cudaMemcpy(b, img.data(), tab, cudaMemcpyHostToDevice));
     }
     size_t pstep_i = 0;
     const double* d_scale = scaled ? scale_buf.p : nullptr;
@@ -1363,7 +1527,8 @@ struct Numeric : NumericBase {
           if (pstep_i < psteps.size() && psteps[pstep_i].l == l && psteps[pstep_i].st == st) {
             const PanelStep& ps = psteps[pstep_i++];
             launch_panel_end<T>(d_fd, d_st, d_plist + ps.off, ps.nl, ps.max_n, panel_nb, s);
-            if (ps.pp >= 0 &&
+            if (use_slices) slice_enqueue(sps[ps.pp], sblob + soff[ps.pp], s);
+            else if (ps.pp >= 0 &&
                 tc_gemm_launch(pplans[ps.pp], pblob[ps.pp], d_tc_status, s, tc_chunk) != 0)
               throw CudaFail{cudaErrorUnknown, __LINE__};
             launch_panel_close<T>(d_fd, d_st, d_plist + ps.off, ps.nl, s);
@@ -1377,6 +1542,7 @@ struct Numeric : NumericBase {
         launch_contrib_gemm<T>(d_fd, d_st, fr, napp, max_app_cm, s);
         if (tblob[l] && tc_gemm_launch(tplans[l], tblob[l], d_tc_status, s, tc_chunk) != 0)
           throw CudaFail{cudaErrorUnknown, __LINE__};
+        if (use_slices) slice_enqueue(sps[npsl + l], sblob + soff[npsl + l], s);
         launch_stats<T>(d_fd, d_st, fr, nf, max_n, d_stats, d_ncount, s);
       }
     } catch (...) {
@@ -1542,6 +1708,21 @@ struct Numeric : NumericBase {
       const char* bi = getenv("SPRAL_GB300_SOLVE_BINV");
       use_binv = std::is_same<T, float>::value && !(bi && bi[0] == '0');
     }
+    const char* pm = getenv("SPRAL_GB300_PANEL_MIN_N");
+    if (std::is_same<T, double>::value) {
+      const char* env = getenv("SPRAL_GB300_TENSOR_CORES");
+      use_slices = !(env && env[0] == '0');
+      // FP64 panels: 128 columns are one exact accumulation of the slice
+      // kernel and leave least to the FP64 pipe inside the panel (57^3
+      // Laplacian, a factorisation and 40 solves: 97.8 ms with 128 columns,
+      // 99.5 / 101.3 / 105.4 ms with 192 / 256 / 384).  From 576 columns on:
+      // narrower fronts would gain little more (105 ms from 768 columns) and
+      // keep the bookkeeping of failed columns of the unpaneled steps.
+      panel_nb = 128;
+      panel_min_n = pm ? std::max(0, atoi(pm)) : 576;
+    }
+    const char* pn = getenv("SPRAL_GB300_PANEL");
+    if (pn) panel_nb = std::max(0, atoi(pn)) / kBlk * kBlk;
     if (std::is_same<T, float>::value) {
       const char* env = getenv("SPRAL_GB300_TENSOR_CORES");
       use_tc = !(env && env[0] == '0');
@@ -1552,9 +1733,6 @@ struct Numeric : NumericBase {
       else if (use_tc) tc_min_cm = autotune_tc_min_cm();
       const char* mk = getenv("SPRAL_GB300_TC_MIN_K");
       if (mk) tc_min_k = std::max(0, atoi(mk));
-      const char* pn = getenv("SPRAL_GB300_PANEL");
-      if (pn) panel_nb = std::max(0, atoi(pn)) / kBlk * kBlk;
-      const char* pm = getenv("SPRAL_GB300_PANEL_MIN_N");
       if (pm) panel_min_n = std::max(0, atoi(pm));
     }
     contrib.ensure(std::max<int64_t>(S->contrib_total, 1));
@@ -1662,10 +1840,11 @@ struct Numeric : NumericBase {
         max_ent = std::max<int>(max_ent, (int)(S->nptr[node + 1] - S->nptr[node]));
         wsW += (size_t)ld * kBlk;
         wsSwap += (size_t)ld * 64 + 256;
-        wsLD += (size_t)std::max(cm, panel_cols(f)) * n;
         maxfront = std::max(maxfront, m);
         maxsn = std::max(maxsn, n);
       }
+      if (use_slices) use_slices = slice_reserve(f0, f1);
+      for (int f = f0; f < f1; ++f) wsLD += (size_t)std::max(cm_of(f), panel_cols(f)) * n_[f];
       for (int f = f0; f < f1; ++f) {
         if (tpp_front(f)) continue;
         max_app_n = std::max(max_app_n, n_[f]);
@@ -1697,7 +1876,7 @@ struct Numeric : NumericBase {
         d.LD = ws_LD.p + oL; oL += (size_t)std::max(d.cm, panel_cols(f)) * n;
         d.step = ws_step.p + (size_t)(f - f0) * (kBlk * kBlk + 2 * kBlk + 64);
         d.lperm = ws_lperm.p + (size_t)(f - f0) * kBlk;
-        d.tc = (use_tc && d.cm >= tc_min_cm && d.n >= tc_min_k) ? 1 : 0;
+        d.tc = (slice_front(f) || (use_tc && d.cm >= tc_min_cm && d.n >= tc_min_k)) ? 1 : 0;
         d.panel = panel_cols(f);
       }
       CK(cudaMemcpyAsync(d_fd + f0, hfd.data() + f0, nf * sizeof(FrontDesc<T>),
@@ -1766,6 +1945,7 @@ struct Numeric : NumericBase {
       if (profile) CK(cudaEventRecord(pev[2 * l], s));
       launch_contrib_gemm<T>(d_fd, d_st, fr, napp, max_app_cm, s);
       run_tc_contrib(f0, f1, s);
+      if (use_slices) slice_run(slice_contrib(f0, f1), s);
       if (profile) CK(cudaEventRecord(pev[2 * l + 1], s));
       pmark(tm(), kPhStats, s);
       launch_stats<T>(d_fd, d_st, fr, nf, max_n, d_stats, d_ncount, s);
@@ -1809,7 +1989,7 @@ struct Numeric : NumericBase {
           if (hfd[f].tc) prof_tc_flops += (double)nelim_[f] * cm * (cm + 1.0);
         }
       }
-      if (use_tc) {
+      if (use_tc || use_slices) {
         int tcs = 0;
         CK(cudaMemcpy(&tcs, d_tc_status, sizeof(int), cudaMemcpyDeviceToHost));
         if (tcs != 0) bad = true;

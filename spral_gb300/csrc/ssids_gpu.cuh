@@ -79,7 +79,7 @@ struct FrontDesc {
   int panel;     // > 0: APP in panels of this many candidate columns (see below)
 };
 
-// Panels (FP32 factors, fronts wider than FrontDesc::panel): the APP block
+// Panels (wide fronts, see Numeric::panel_cols): the APP block
 // steps draw their candidates from a panel of `panel` columns [pstart, qend)
 // and update only the panel's columns; at the panel's end the trailing
 // fully-summed columns [qend, n) take the panel's pk pivots in one
@@ -245,6 +245,34 @@ int tc_gemm_launch(const TcPlan& plan, const void* d_blob, int* status, cudaStre
 int tc_gemm_run(const std::vector<TcProblem>& ps, void* scratch, TcBuffers& buf, int* status,
                 cudaStream_t s, int chunk = kTcChunk, float* ms_split = nullptr,
                 float* ms_gemm = nullptr, int bn = 0);
+
+// ---------------- FP64 updates on the tensor cores (slice_gemm.cu) ----------------
+// C -= A B^T (r >= c), all FP64, from exact bf16 slice products.  A job is
+// one front's contribution block (pivots [k0, k0 + kcap)), one closed panel's
+// trailing update, or operands given by the caller; k_slice_plan completes it
+// on the device from the front's state.
+constexpr int kSlices = 8;         // base-256 digits of an operand
+constexpr int kSliceMaxK = 2048;   // deepest job (bounds the slices' memory)
+enum SliceKind : int { kSliceContrib = 0, kSlicePanel, kSliceGiven };
+struct SliceJob {
+  int front, kind, k0, kcap;  // kcap: columns the buffers hold
+  int mcap, ncap;             // rows of A and of B the buffers hold
+  char *sA, *sB;              // slices
+  int *eA, *eB;               // row exponents
+  // completed on the device (kSliceGiven: by the host)
+  const double *A, *B, *D;    // D: D^{-1} for the column balance, or nullptr
+  double* C;
+  int lda, ldb, ldc, M, N, K;
+  int c0, dlast;              // first pivot column, end of the pivots
+};
+size_t slice_job_bytes(int mcap, int ncap, int kcap);
+void slice_job_place(SliceJob& j, char* base);  // lays the job's buffers out at base
+size_t slice_table_bytes(int njobs);
+// plan, slice and GEMM launches of jobs[first, first + count), whose copies
+// are at `table` in device memory (slice_table_bytes(count)); enqueues only
+int launch_slice_gemm(void* table, const std::vector<SliceJob>& jobs, size_t first, size_t count,
+                      const FrontDesc<double>* fds, const FrontState* sts, int* status,
+                      cudaStream_t s);
 
 // syrk-like lower update C(r,c) -= sum_k A(r,k) B(c,k), r >= c
 template <typename T>

@@ -69,6 +69,11 @@ def estimate_bytes(akeep, precision=ssids.PRECISION_FP64, nrhs=1):
     factors = 1.25 * (nrow * ncol).sum() * s
     contrib = (cm * cm).sum() * s
     work = (nrow.max() * 160 + 16 * nrow.sum()) * s + akeep.nnz * 8 * 3
+    if precision != ssids.PRECISION_MIXED:
+        # digit slices of the tensor-core updates: one launch group of 256 MiB,
+        # or the largest front alone
+        sl = 32 * (cm + 128) * np.minimum(ncol, 2048)
+        work += max(sl.max(), min(sl.sum(), 256 << 20))
     solve = 4 * akeep.n * max(nrhs, 16) * 8
     return int(factors + contrib + work + solve + (192 << 20))
 
