@@ -34,37 +34,60 @@ __global__ void k_zero_fronts(FrontDesc<T>* fds, const int* fronts) {
   zero_range(fd.D, 2 * (int64_t)fd.n, i0, stride);
 }
 
-__device__ __forceinline__ void atomic_max_pos(double* a, double v) {
-  // non-negative doubles order like their bit patterns
-  atomicMax(reinterpret_cast<unsigned long long*>(a), (unsigned long long)__double_as_longlong(v));
+// Maxima of magnitudes as integers: non-negative doubles order like their bit
+// patterns, and an FP64 maximum issues some 30 times slower than an integer
+// one on GB300.
+typedef unsigned long long u64;
+__device__ __forceinline__ u64 mag_bits(double v) {  // a NaN counts as 0, as in fmax
+  const u64 k = (u64)__double_as_longlong(v) & 0x7fffffffffffffffULL;
+  return k > 0x7ff0000000000000ULL ? 0ULL : k;
+}
+__device__ __forceinline__ u64 warp_max(u64 k) {
+  const unsigned hi = (unsigned)(k >> 32), lo = (unsigned)k;
+  const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+  return ((u64)mh << 32) | ml;
+}
+__device__ __forceinline__ void atomic_max_pos(double* a, u64 bits) {
+  atomicMax(reinterpret_cast<u64*>(a), bits);
 }
 
 // r = b - A x and the maxima of the scaled backward error in one pass.
-// kResG lanes share a row (its non-zeros strided over the lanes); each
-// non-zero is applied to kResQC right-hand sides at once (chunk
-// blockIdx.y), so the row's index and value loads are shared by the chunk.
-// Every lane of a warp runs the same number of row iterations, so the lane
-// reductions use full-warp shuffles.  work: [0] ||A||_inf, then per rhs
-// (||x||, ||b||, ||r||) at 1 + 3q (maxima, order-independent).
-constexpr int kResG = 4;
+// G lanes share a row (its non-zeros strided over the lanes); each non-zero
+// is applied to kResQC right-hand sides at once (chunk blockIdx.y), so the
+// row's index and value loads are shared by the chunk.  Every lane of a warp
+// runs the same number of row iterations, so the lane reductions use
+// full-warp shuffles.  work: [0] ||A||_inf, then per rhs (||x||, ||b||,
+// ||r||) at 1 + 3q (maxima, order-independent).
+//
+// Bound by FP64 issue (about 75 cycles a warp instruction): a non-zero costs
+// one multiply-add per right-hand side and, in the first chunk, one addition
+// for the row sum.  One lane per row needs the fewest (short rows: no partial
+// sums to add over lanes); four lanes per row where rows average more than
+// kResShort non-zeros and a warp would wait for its longest.  320 stacked 2D
+// Laplacians (n = 0.93M, one right-hand side): 751 -> 123 us, 48^3 Laplacian
+// with 8 right-hand sides 127 -> 62 us, with the maxima in integers.
 constexpr int kResQC = 4;
+constexpr int kResShort = 12;
 // With row groups (row_group != nullptr: the group of each row, e.g. the
 // matrix of a batch it belongs to) the maxima are kept per group, at
 // work[g * kResStride ...], so the backward error can be judged per group.
+template <int G>
 __global__ void __launch_bounds__(256) k_resid_norms(const int64_t* aptr, const int* acol,
                                                      const int64_t* asrc, const double* aval,
                                                      int n, const double* x, const double* b,
                                                      double* r, int nrhs, int ld, double* work,
                                                      const int* row_group) {
-  constexpr int G = kResG, QC = kResQC, RPW = 32 / G;
+  constexpr int QC = kResQC, RPW = 32 / G, NV = 1 + 3 * QC;
   const int lane = threadIdx.x & 31, sub = lane & (G - 1);
   const int q0 = blockIdx.y * QC;
   const int nq = min(QC, nrhs - q0);
+  const bool norm = blockIdx.y == 0;  // this chunk forms ||A||
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarp = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  double an = 0.0, mx[QC], mb[QC], mr[QC];
+  u64 m[NV];  // ||A||, then (x, b, r) per right-hand side
 #pragma unroll
-  for (int q = 0; q < QC; ++q) mx[q] = mb[q] = mr[q] = 0.0;
+  for (int v = 0; v < NV; ++v) m[v] = 0;
   for (int64_t base = warp * RPW; base < n; base += nwarp * RPW) {
     const int64_t i = base + lane / G;
     const bool ok = i < n;
@@ -76,7 +99,7 @@ __global__ void __launch_bounds__(256) k_resid_norms(const int64_t* aptr, const 
       for (int64_t k = aptr[i] + sub; k < k1; k += G) {
         const double a = aval[asrc[k]];
         const int64_t c = acol[k];
-        ra += fabs(a);
+        if (norm) ra += fabs(a);
 #pragma unroll
         for (int q = 0; q < QC; ++q)
           if (q < nq) s[q] = fma(a, x[(int64_t)(q0 + q) * ld + c], s[q]);
@@ -84,109 +107,64 @@ __global__ void __launch_bounds__(256) k_resid_norms(const int64_t* aptr, const 
     }
 #pragma unroll
     for (int off = G / 2; off > 0; off >>= 1) {
-      ra += __shfl_xor_sync(0xffffffffu, ra, off);
+      if (norm) ra += __shfl_xor_sync(0xffffffffu, ra, off);
 #pragma unroll
-      for (int q = 0; q < QC; ++q) s[q] += __shfl_xor_sync(0xffffffffu, s[q], off);
+      for (int q = 0; q < QC; ++q)
+        if (q < nq) s[q] += __shfl_xor_sync(0xffffffffu, s[q], off);
     }
     if (row_group) {
-      // grouped maxima: a warp whose rows share one group reduces them and
-      // makes one atomic per value; otherwise each row makes its own
-      double vx[QC], vb[QC], vr[QC];
 #pragma unroll
-      for (int q = 0; q < QC; ++q) vx[q] = vb[q] = vr[q] = 0.0;
-      const int g = ok ? row_group[i] : -1;
-      if (ok && sub == 0) {
-#pragma unroll
-        for (int q = 0; q < QC; ++q) {
-          if (q < nq) {
-            const int64_t e = (int64_t)(q0 + q) * ld + i;
-            const double bi = b[e], ri = bi - s[q];
-            r[e] = ri;
-            vx[q] = fabs(x[e]);
-            vb[q] = fabs(bi);
-            vr[q] = fabs(ri);
-          }
-        }
-      }
-      const double va = ok ? ra : 0.0;
-      const int g0 = __shfl_sync(0xffffffffu, g, 0);
-      if (__all_sync(0xffffffffu, g == g0 || g < 0)) {
-        double wa = va;
-        for (int off = 16; off > 0; off >>= 1) wa = fmax(wa, __shfl_xor_sync(0xffffffffu, wa, off));
-#pragma unroll
-        for (int q = 0; q < QC; ++q)
-          for (int off = 16; off > 0; off >>= 1) {
-            vx[q] = fmax(vx[q], __shfl_xor_sync(0xffffffffu, vx[q], off));
-            vb[q] = fmax(vb[q], __shfl_xor_sync(0xffffffffu, vb[q], off));
-            vr[q] = fmax(vr[q], __shfl_xor_sync(0xffffffffu, vr[q], off));
-          }
-        if (lane == 0 && g0 >= 0) {
-          double* w = work + (int64_t)g0 * kResStride;
-          if (blockIdx.y == 0) atomic_max_pos(&w[0], wa);
-          for (int q = 0; q < nq; ++q) {
-            atomic_max_pos(&w[1 + 3 * (q0 + q)], vx[q]);
-            atomic_max_pos(&w[2 + 3 * (q0 + q)], vb[q]);
-            atomic_max_pos(&w[3 + 3 * (q0 + q)], vr[q]);
-          }
-        }
-      } else if (ok && sub == 0) {
-        double* w = work + (int64_t)g * kResStride;
-        if (blockIdx.y == 0) atomic_max_pos(&w[0], va);
-        for (int q = 0; q < nq; ++q) {
-          atomic_max_pos(&w[1 + 3 * (q0 + q)], vx[q]);
-          atomic_max_pos(&w[2 + 3 * (q0 + q)], vb[q]);
-          atomic_max_pos(&w[3 + 3 * (q0 + q)], vr[q]);
-        }
-      }
-      continue;
+      for (int v = 0; v < NV; ++v) m[v] = 0;
     }
     if (ok && sub == 0) {
-      an = fmax(an, ra);
+      m[0] = max(m[0], mag_bits(ra));
 #pragma unroll
       for (int q = 0; q < QC; ++q) {
         if (q < nq) {
           const int64_t e = (int64_t)(q0 + q) * ld + i;
           const double bi = b[e], ri = bi - s[q];
           r[e] = ri;
-          mx[q] = fmax(mx[q], fabs(x[e]));
-          mb[q] = fmax(mb[q], fabs(bi));
-          mr[q] = fmax(mr[q], fabs(ri));
+          m[1 + 3 * q] = max(m[1 + 3 * q], mag_bits(x[e]));
+          m[2 + 3 * q] = max(m[2 + 3 * q], mag_bits(bi));
+          m[3 + 3 * q] = max(m[3 + 3 * q], mag_bits(ri));
         }
       }
+    }
+    if (!row_group) continue;
+    // grouped maxima: a warp whose rows share one group reduces them and
+    // makes one atomic per value; otherwise each row makes its own
+    const int g = ok ? row_group[i] : -1;
+    const int g0 = __shfl_sync(0xffffffffu, g, 0);
+    if (__all_sync(0xffffffffu, g == g0 || g < 0)) {
+      double* w = work + (int64_t)g0 * kResStride;  // g0 >= 0: the warp's first row exists
+#pragma unroll
+      for (int v = 0; v < NV; ++v) {
+        if (v == 0 ? !norm : (v - 1) / 3 >= nq) continue;
+        const u64 k = warp_max(m[v]);
+        if (lane == 0) atomic_max_pos(&w[v == 0 ? 0 : 3 * q0 + v], k);
+      }
+    } else if (ok && sub == 0) {
+      double* w = work + (int64_t)g * kResStride;
+#pragma unroll
+      for (int v = 0; v < NV; ++v)
+        if (v == 0 ? norm : (v - 1) / 3 < nq) atomic_max_pos(&w[v == 0 ? 0 : 3 * q0 + v], m[v]);
     }
   }
   if (row_group) return;
   // warp maxima -> block maxima in shared memory -> one atomic per value
   // and block (same-address atomics from every warp would serialise)
-  constexpr int NV = 1 + 3 * QC;
-  __shared__ double red[256 / 32][NV];
-  const int warp_in_block = threadIdx.x >> 5;
-  for (int off = 16; off > 0; off >>= 1) an = fmax(an, __shfl_xor_sync(0xffffffffu, an, off));
-  if (lane == 0) red[warp_in_block][0] = an;
+  __shared__ u64 red[256 / 32][NV];
 #pragma unroll
-  for (int q = 0; q < QC; ++q) {
-    double v0 = mx[q], v1 = mb[q], v2 = mr[q];
-    for (int off = 16; off > 0; off >>= 1) {
-      v0 = fmax(v0, __shfl_xor_sync(0xffffffffu, v0, off));
-      v1 = fmax(v1, __shfl_xor_sync(0xffffffffu, v1, off));
-      v2 = fmax(v2, __shfl_xor_sync(0xffffffffu, v2, off));
-    }
-    if (lane == 0) {
-      red[warp_in_block][1 + 3 * q] = v0;
-      red[warp_in_block][2 + 3 * q] = v1;
-      red[warp_in_block][3 + 3 * q] = v2;
-    }
+  for (int v = 0; v < NV; ++v) {
+    const u64 k = warp_max(m[v]);
+    if (lane == 0) red[threadIdx.x >> 5][v] = k;
   }
   __syncthreads();
   if (threadIdx.x < NV) {
     const int v = threadIdx.x;
-    double m = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) m = fmax(m, red[w][v]);
-    if (v == 0) {
-      if (blockIdx.y == 0) atomic_max_pos(&work[0], m);
-    } else if ((v - 1) / 3 < nq) {
-      atomic_max_pos(&work[1 + 3 * q0 + (v - 1)], m);
-    }
+    u64 k = 0;
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) k = max(k, red[w][v]);
+    if (v == 0 ? norm : (v - 1) / 3 < nq) atomic_max_pos(&work[v == 0 ? 0 : 3 * q0 + v], k);
   }
 }
 
@@ -239,18 +217,26 @@ template void launch_zero_fronts<float>(FrontDesc<float>*, const int*, int, int,
 // r = b - A x and the scaled backward error of each right-hand side, the
 // largest over the row groups when row_group is given (work must hold
 // nrhs + max(ngroups, 1) * (1 + 3*kSolveRhs) doubles; the result per rhs is
-// written to work[0 .. nrhs)).
+// written to work[0 .. nrhs)).  nnz: entries of the full CSR.
 void launch_resid_bwd_err(const int64_t* aptr, const int* acol, const int64_t* asrc,
-                          const double* aval, int n, const double* x, const double* b, double* r,
-                          int nrhs, int ld, double* work, const int* row_group, int ngroups,
+                          const double* aval, int n, int64_t nnz, const double* x,
+                          const double* b, double* r, int nrhs, int ld, double* work,
+                          const int* row_group, int ngroups,
                           cudaStream_t s) {
   double* acc = work + nrhs;
   const int ng = row_group ? std::max(ngroups, 1) : 1;
   cudaMemsetAsync(acc, 0, (size_t)ng * kResStride * sizeof(double), s);
-  const int rows_per_block = 256 / 32 * (32 / kResG);
+  const bool small = nnz <= (int64_t)kResShort * n;
+  const int rows_per_block = small ? 256 : 64;
   const int bx = std::max(1, std::min((n + rows_per_block - 1) / rows_per_block, 4 * 152));
-  const int by = (nrhs + kResQC - 1) / kResQC;
-  { k_resid_norms<<<dim3(bx, by), 256, 0, s>>>(aptr, acol, asrc, aval, n, x, b, r, nrhs, ld, acc, row_group); note_launches(1); }
+  const dim3 grid(bx, (nrhs + kResQC - 1) / kResQC);
+  if (small)
+    k_resid_norms<1><<<grid, 256, 0, s>>>(aptr, acol, asrc, aval, n, x, b, r, nrhs, ld, acc,
+                                          row_group);
+  else
+    k_resid_norms<4><<<grid, 256, 0, s>>>(aptr, acol, asrc, aval, n, x, b, r, nrhs, ld, acc,
+                                          row_group);
+  note_launches(1);
   { k_bwd_finish<<<1, 256, 0, s>>>(acc, nrhs, ng, work); note_launches(1); }
 }
 

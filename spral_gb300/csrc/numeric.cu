@@ -341,6 +341,7 @@ struct Symbolic {
   std::vector<int64_t> contrib_off;  // per front, elements
   int64_t contrib_total = 0;
   int64_t nnz = 0;
+  int64_t nnz_full = 0;  // entries of the full CSR of A (both triangles)
   std::vector<int> rdir_h;
   std::vector<int64_t> rdir_ptr_h;
   // device
@@ -576,6 +577,7 @@ static Symbolic* build_symbolic(int device, int n, int sa, int en, const int* sp
       if (pr[k] != pc[k]) aptr[pc[k] + 1]++;
     }
     for (int i = 0; i < n; ++i) aptr[i + 1] += aptr[i];
+    S->nnz_full = aptr[n];
     std::vector<int> acol(aptr[n]);
     std::vector<int64_t> asrc(aptr[n]);
     std::vector<int64_t> fill(aptr.begin(), aptr.end() - 1);
@@ -680,9 +682,9 @@ template <typename T>
 void launch_zero_fronts(FrontDesc<T>* fd, const int* fronts, int nf, int max_elems,
                         cudaStream_t s);
 void launch_resid_bwd_err(const int64_t* aptr, const int* acol, const int64_t* asrc,
-                          const double* aval, int n, const double* x, const double* b, double* r,
-                          int nrhs, int ld, double* work, const int* row_group, int ngroups,
-                          cudaStream_t s);
+                          const double* aval, int n, int64_t nnz, const double* x,
+                          const double* b, double* r, int nrhs, int ld, double* work,
+                          const int* row_group, int ngroups, cudaStream_t s);
 void launch_axpy(int n, int nrhs, int ld, double* x, const double* d, cudaStream_t s,
                  const int* row_group = nullptr, const unsigned char* active = nullptr);
 
@@ -2387,8 +2389,8 @@ struct Numeric : NumericBase {
     group_prev.clear();
     for (;; ++it) {
       pmark(tm(), kPhResid, s);
-      launch_resid_bwd_err(S->d_aptr, S->d_acol, S->d_asrc, cur_aval, n, x, b, rbuf.p, q, ld,
-                           nbuf.p, S->d_row_group, S->ngroups, s);
+      launch_resid_bwd_err(S->d_aptr, S->d_acol, S->d_asrc, cur_aval, n, S->nnz_full, x, b,
+                           rbuf.p, q, ld, nbuf.p, S->d_row_group, S->ngroups, s);
       pmark(tm(), kPhHost, s);
       CK(cudaMemcpyAsync(h.data(), nbuf.p, q * sizeof(double), cudaMemcpyDeviceToHost, s));
       CK(cudaStreamSynchronize(s));
