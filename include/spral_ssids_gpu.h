@@ -241,8 +241,9 @@ int spral_ssids_gpu_recip_probe(const double* x_dev, double* y_dev, int n);
  *   upd ((m-n) x (m-n), ldupd >= m-n) or NULL: upd = beta*upd - L21 D L21^T
  *     (beta 0 or 1), e.g. the trailing block of a with ldupd = lda.
  * Returns nelim, or a negative SSIDS flag (-5 singular with action false,
- * -50 allocation, -51 CUDA).  Allocates its workspace with cudaMalloc and
- * synchronises the stream before returning. */
+ * -50 allocation, -51 CUDA).  Takes its workspace from the device blocks that
+ * numeric handles keep for reuse (spral_ssids_gpu_release_cache), or from
+ * cudaMalloc, and synchronises the stream before returning. */
 int spral_ssids_gpu_ldlt_app_factor(int m, int n, int* perm_dev, double* a_dev, int lda,
                                     double* d_dev, double beta, double* upd_dev, int ldupd,
                                     const struct spral_ssids_cpu_factor_options* options,
@@ -296,7 +297,7 @@ int spral_ssids_gpu_tc_gemm_f32_bn(int M, int N, int K, const float* A, int lda,
  * measurements: C (M x N, N <= M, column-major, ldc) -= A B^T on the lower
  * trapezoid (row >= column) with A (M x K) and B (N x K) column-major FP64
  * device arrays, applied reps times on the caller's stream.  The products are
- * exact bf16 slice products summed exactly; the result differs from the exact
+ * exact FP16 slice products summed exactly; the result differs from the exact
  * update by about 2^-62 sqrt(K) of (row maximum of A) x (row maximum of B)
  * and the rounding of C.  Allocates its workspace and synchronises the
  * stream.  Returns 0, -1 bad argument, -50 allocation, -51 CUDA error, -52

@@ -6,6 +6,9 @@
 // on one front held by the caller in device memory.
 #include <algorithm>
 #include <cstdio>
+#include <cstring>
+#include <new>
+#include <vector>
 
 #include "spral_ssids_gpu.h"
 #include "ssids_gpu.cuh"
@@ -42,6 +45,37 @@ struct DenseWorkspace {
   double* LD;
 };
 
+// Tensor-core update of the allocating entry point (slice_gemm.cu), with the
+// tree factorisation's rule: from 32 columns and 16 rows on.  The job tables
+// (one per k range) and the digit slices follow the front's workspace.
+struct DenseSlices {
+  std::vector<SliceJob> jobs;  // one per k range
+  size_t table = 0, scratch = 0;
+  char* base = nullptr;
+  bool any() const { return !jobs.empty(); }
+  size_t bytes() const { return table + scratch; }
+  int* status() const { return reinterpret_cast<int*>(base); }
+  char* job_table(size_t i) const { return base + 256 + i * slice_table_bytes(1); }
+};
+constexpr int kDenseSliceMinK = 32, kDenseSliceMinCm = 16;
+
+static DenseSlices dense_slices(int m, int n, bool update) {
+  DenseSlices d;
+  const int cm = m - n;
+  if (!update || cm < kDenseSliceMinCm || n < kDenseSliceMinK) return d;
+  for (int k0 = 0; k0 < n; k0 += kSliceMaxK) {
+    SliceJob j{};
+    j.kind = kSliceContrib;
+    j.k0 = k0;
+    j.kcap = std::min(kSliceMaxK, n - k0);
+    j.mcap = j.ncap = cm;
+    d.jobs.push_back(j);
+    d.scratch = std::max(d.scratch, slice_job_bytes(cm, cm, j.kcap));
+  }
+  d.table = 256 + d.jobs.size() * slice_table_bytes(1);
+  return d;
+}
+
 static size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
 
 size_t dense_workspace_bytes(int m, int n, int lda) {
@@ -72,10 +106,12 @@ DenseWorkspace dense_workspace_carve(void* base, int m, int n, int lda) {
 }
 
 // Enqueue the factorization of one front on stream s using workspace w and
-// return nelim (after a synchronisation) or a negative SSIDS flag.
+// return nelim (after a synchronisation) or a negative SSIDS flag.  sl: the
+// tensor-core update, or nullptr for the SIMT kernel.
 int dense_factor_run(const DenseWorkspace& w, int m, int n, int* perm, double* a, int lda,
                      double* d, double beta, double* upd, int ldupd,
-                     const spral_ssids_cpu_factor_options& co, cudaStream_t s) {
+                     const spral_ssids_cpu_factor_options& co, cudaStream_t s,
+                     DenseSlices* sl = nullptr) {
   FrontDesc<double> h{};
   h.L = a;
   h.D = d;
@@ -91,6 +127,20 @@ int dense_factor_run(const DenseWorkspace& w, int m, int n, int* perm, double* a
   h.nrow = m; h.ncol = n; h.ndelay_in = 0; h.cm = m - n;
   h.node = 0;
   h.ldc = ldupd;
+  const bool tc = sl && sl->any();
+  h.tc = tc ? 1 : 0;
+  if (tc) {
+    char* buf = sl->base + sl->table;
+    std::vector<char> img(sl->table - 256, 0);
+    for (size_t i = 0; i < sl->jobs.size(); ++i) {
+      slice_job_place(sl->jobs[i], buf);
+      memcpy(img.data() + i * slice_table_bytes(1), &sl->jobs[i], sizeof(SliceJob));
+    }
+    if (cudaMemcpyAsync(sl->base + 256, img.data(), img.size(), cudaMemcpyHostToDevice, s) !=
+        cudaSuccess)
+      return -51;
+    if (cudaMemsetAsync(sl->status(), 0, sizeof(int), s) != cudaSuccess) return -51;
+  }
   const int zero = 0;
   if (cudaMemcpyAsync(w.desc, &h, sizeof(h), cudaMemcpyHostToDevice, s) != cudaSuccess) return -51;
   if (cudaMemcpyAsync(w.front0, &zero, sizeof(int), cudaMemcpyHostToDevice, s) != cudaSuccess) return -51;
@@ -114,14 +164,25 @@ int dense_factor_run(const DenseWorkspace& w, int m, int n, int* perm, double* a
   launch_tpp<double>(w.desc, w.state, w.front0, 1, co.action, co.u, co.small, tpp_all, s);
   if (m > n && upd) {
     launch_calc_ld<double>(w.desc, w.state, w.front0, 1, m - n, n, s);
-    launch_contrib_gemm<double>(w.desc, w.state, w.front0, 1, m - n, s);
+    if (tc) {
+      for (size_t i = 0; i < sl->jobs.size(); ++i)
+        if (launch_slice_gemm(sl->job_table(i), sl->jobs, i, 1, w.desc, w.state, sl->status(),
+                              s) != 0)
+          return -51;
+    } else {
+      launch_contrib_gemm<double>(w.desc, w.state, w.front0, 1, m - n, s);
+    }
   }
   FrontState hs{};
+  int slice_status = 0;
+  if (tc && cudaMemcpyAsync(&slice_status, sl->status(), sizeof(int),
+                                         cudaMemcpyDeviceToHost, s) != cudaSuccess)
+    return -51;
   if (cudaMemcpyAsync(&hs, w.state, sizeof(FrontState), cudaMemcpyDeviceToHost, s) != cudaSuccess)
     return -51;
   if (cudaStreamSynchronize(s) != cudaSuccess) return -51;
   if (hs.status == kDevSingular) return -5;
-  if (hs.status != kDevOk) return -51;
+  if (hs.status != kDevOk || slice_status != 0) return -51;
   return hs.nelim;
 }
 
@@ -143,16 +204,30 @@ int spral_ssids_gpu_ldlt_app_factor(int m, int n, int* perm_dev, double* a_dev, 
   co.action = true; co.small = 1e-20; co.u = 0.01; co.pivot_method = 2; co.failed_pivot_method = 1;
   if (options) co = *options;
   cudaStream_t s = (cudaStream_t)stream;
-  void* base = nullptr;
-  const size_t bytes = dense_workspace_bytes(m, n, lda);
-  if (cudaMalloc(&base, bytes) != cudaSuccess) {
-    cudaGetLastError();
+  try {
+    DenseSlices sl = dense_slices(m, n, m > n && upd_dev);
+    void* base = nullptr;
+    size_t cls = 0;
+    int dev = -1;
+    // a device too full for the slices factors the front without them
+    for (int attempt = sl.any() ? 0 : 1; attempt < 2 && !base; ++attempt) {
+      if (attempt == 1) sl = DenseSlices{};
+      const size_t front = align256(dense_workspace_bytes(m, n, lda));
+      base = workspace_alloc(front + (sl.any() ? sl.bytes() : 0), &cls, &dev);
+      if (base && sl.any()) sl.base = static_cast<char*>(base) + front;
+    }
+    if (!base) return -50;
+    const DenseWorkspace w = dense_workspace_carve(base, m, n, lda);
+    const int r = dense_factor_run(w, m, n, perm_dev, a_dev, lda, d_dev, beta, upd_dev, ldupd, co,
+                                   s, sl.any() ? &sl : nullptr);
+    // nothing of this call is still running when the block goes back: the
+    // run synchronised its stream, unless it gave up on an error
+    if (r == -51 && cudaStreamSynchronize(s) != cudaSuccess) cudaGetLastError();
+    workspace_free(base, cls, dev);
+    return r;
+  } catch (std::bad_alloc const&) {
     return -50;
   }
-  DenseWorkspace w = dense_workspace_carve(base, m, n, lda);
-  int r = dense_factor_run(w, m, n, perm_dev, a_dev, lda, d_dev, beta, upd_dev, ldupd, co, s);
-  cudaFree(base);
-  return r;
 }
 
 }  // extern "C"

@@ -22,12 +22,14 @@
 // reference does (root fronts or failed_pivot_method = tpp); k_calc_ld and
 // k_syrk (contrib) form the contribution block; k_stats counts inertia.
 #include <algorithm>
+#include <atomic>
 #include <cfloat>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <type_traits>
 
+#include "slices.cuh"
 #include "ssids_gpu.cuh"
 
 namespace ssids300 {
@@ -979,15 +981,13 @@ __device__ void app_fixup_cta(const FrontDesc<T>& fd, FrontState* st, int p, int
 // the fixup rewrites the failed columns of the block), so one launch serves
 // both.  Every CTA derives npass from the apply's result itself.
 //
-// Update C -= A B^T (lower part) with K = npass <= kBlk: a TP x TP tile per
-// CTA round, thread (tx, ty) = (tid % 16, tid / 16) computing (TP/16)^2
+// Update C -= A B^T (lower part) with K = npass <= kBlk, FP32: a TP x TP tile
+// per CTA round, thread (tx, ty) = (tid % 16, tid / 16) computing (TP/16)^2
 // entries; a tile stages all of its A and B columns and reads its C entries
-// in one batch of loads (one memory round trip per tile).  FP32 uses 64 x 64
-// tiles (latency bound); FP64 32 x 32 tiles: a 64 x 64 tile is about 37 us
-// of work for one SM's FP64 pipe, and finer tiles balance the last wave.
+// in one batch of loads (one memory round trip per tile; latency bound).
+// FP64: k_app_panel_f64.
 // ------------------------------------------------------------------------
-template <typename T>
-constexpr int panel_tile() { return sizeof(T) == 8 ? 32 : 64; }
+constexpr int kPanelTile = 64;
 
 template <typename T, int TP>
 __global__ void __launch_bounds__(256) k_app_panel(FrontDesc<T>* fds, FrontState* sts,
@@ -1083,6 +1083,178 @@ __global__ void __launch_bounds__(256) k_app_panel(FrontDesc<T>* fds, FrontState
       }
     }
     __syncthreads();  // Ap/Bp are rewritten by the next tile
+  }
+}
+
+// ------------------------------------------------------------------------
+// k_app_panel_f64: the same launch for FP64 factors.  On the FP64 pipe a
+// 32 x 32 x 32 tile took 10 us of an SM; here a CTA of four warps forms a
+// 64 x 32 tile from exact products of FP16 digits (slices.cuh) with
+// mma.sync m16n8k16 (FP32 sums of at most 8 * 32 products of at most 2^14,
+// exact): it loads the tile's rows of A and B once, cuts them into digits in
+// shared memory (8-column groups of rows of 16 bytes: conflict-free ldmatrix),
+// a warp multiplies 16 rows by 32 columns for all 36 digit pairs, and one
+// FP64 subtraction per entry is left.  mma.sync rather than tcgen05: the
+// depth is a single block (32 columns), so a tile's operands are used once
+// and its sums leave the registers directly, without a pass through TMEM.
+// Bound by latency on one front (a tile is one round), by the digit
+// arithmetic when tiles fill the GPU.  48^3 Laplacian: 58 -> 17 us a launch.
+// ------------------------------------------------------------------------
+constexpr int PF_M = 64, PF_N = 32, PF_THREADS = 128;
+constexpr int PF_A_SLICE = PF_M * kBlk * 2, PF_B_SLICE = PF_N * kBlk * 2;  // bytes per digit
+constexpr int kEmptyRow = -(1 << 18);  // exponent of a row of zeros
+constexpr size_t kPanelF64Smem = (size_t)8 * (PF_A_SLICE + PF_B_SLICE);
+
+__device__ __forceinline__ void ldsm_x4(unsigned (&v)[4], const char* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
+               : "r"((unsigned)__cvta_generic_to_shared(p)));
+}
+__device__ __forceinline__ void ldsm_x2(unsigned (&v)[2], const char* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];"
+               : "=r"(v[0]), "=r"(v[1])
+               : "r"((unsigned)__cvta_generic_to_shared(p)));
+}
+__device__ __forceinline__ void mma_f16(float (&c)[4], const unsigned (&a)[4],
+                                         const unsigned (&b)[2]) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+      "{%0,%1,%2,%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+// sum of eight levels of exact digit products (each |v| <= 2^22) as FP64 * 2^e
+__device__ __forceinline__ double levels_to_double(const float (&v)[8], int e) {
+  // an integer |i| <= 2^22 plus 1.5 * 2^23 has i in its low mantissa bits; two
+  // levels make one 32-bit integer (below 2^30 + 2^22), modulo 2^32 throughout
+  int p[4];
+#pragma unroll
+  for (int l = 0; l < 4; ++l) {
+    const unsigned i0 = __float_as_uint(v[2 * l] + 12582912.0f);
+    const unsigned i1 = __float_as_uint(v[2 * l + 1] + 12582912.0f);
+    p[l] = (int)(i0 * 256u + i1 - 257u * 0x4B400000u);
+  }
+  return fixed_to_double((long long)p[0] * 65536 + p[1], (long long)p[2] * 65536 + p[3], e);
+}
+
+__global__ void __launch_bounds__(PF_THREADS, 4)
+    k_app_panel_f64(FrontDesc<double>* fds, FrontState* sts, const int* fronts, int ptiles) {
+  extern __shared__ __align__(16) char pf_smem[];
+  __shared__ int emA[3][PF_M], emB[5][PF_N];  // partial row exponents; last, the rows' own
+  __shared__ short hs[kBlk];
+  const int f = fronts[blockIdx.y];
+  const FrontDesc<double> fd = fds[f];  // written by the host before the launch
+  pdl_wait();
+  pdl_trigger();
+  FrontState* stp = &sts[f];
+  const int bs = stp->bs;
+  if (bs == 0) return;
+  const int p = stp->p;
+  const int np = adjust_npass(stp->npass_raw, bs, p, fd.D);
+  if ((int)blockIdx.x >= ptiles) {
+    double (*l11)[kBlk + 1] = reinterpret_cast<double (*)[kBlk + 1]>(pf_smem);
+    app_fixup_cta<double>(fd, stp, p, bs, np, blockIdx.x - ptiles, gridDim.x - ptiles, l11,
+                          l11 + kBlk);
+    return;
+  }
+  const int M = fd.m - (p + bs), N = stp->qend - (p + bs), K = np;
+  if (K <= 0 || M <= 0 || N <= 0) return;
+  double* C = fd.L + (int64_t)(p + bs) * fd.ld + (p + bs);
+  const double* A = fd.L + (int64_t)p * fd.ld + (p + bs);
+  const double* B = fd.W;
+  const int64_t ld = fd.ld;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  char* sA = pf_smem;
+  char* sB = pf_smem + 8 * PF_A_SLICE;
+  const int total = trapezoid_tiles<PF_N>(M, N);
+  if ((int)blockIdx.x >= total) return;
+  if (tid < K) hs[tid] = (short)slice_balance(fd.D, p + tid, p + np);
+  // this thread's row and column groups of the operands: 16 columns of a row
+  // of A, 8 columns of a row of B
+  const int ra = tid & 63, ka = (tid >> 6) * 16, rb = tid & 31, kb = warp * 8;
+  for (int t = blockIdx.x; t < total; t += ptiles) {
+    int ti, tj;
+    trapezoid_tile<PF_N>(t, N, ti, tj);
+    const int row0 = ti * PF_M, col0 = tj * PF_N;
+    unsigned long long a0[8], a1[8], b0[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const bool va = row0 + ra < M;
+      const double* s = A + row0 + ra;
+      a0[q] = (va && ka + q < K) ? (unsigned long long)__double_as_longlong(s[(ka + q) * ld]) : 0ULL;
+      a1[q] = (va && ka + 8 + q < K)
+                  ? (unsigned long long)__double_as_longlong(s[(ka + 8 + q) * ld]) : 0ULL;
+      b0[q] = (col0 + rb < N && kb + q < K)
+                  ? (unsigned long long)__double_as_longlong(B[(kb + q) * ld + col0 + rb]) : 0ULL;
+    }
+    __syncthreads();  // hs; the previous tile's digits have been read
+    int e0[8], e1[8], eb[8], ma = kEmptyRow, mb = kEmptyRow;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      e0[q] = slice_exponent(a0[q], ka + q < K ? hs[ka + q] : 0);
+      e1[q] = slice_exponent(a1[q], ka + 8 + q < K ? hs[ka + 8 + q] : 0);
+      eb[q] = slice_exponent(b0[q], kb + q < K ? -hs[kb + q] : 0);
+      if ((a0[q] << 1) != 0ULL) ma = max(ma, e0[q]);
+      if ((a1[q] << 1) != 0ULL) ma = max(ma, e1[q]);
+      if ((b0[q] << 1) != 0ULL) mb = max(mb, eb[q]);
+    }
+    emA[tid >> 6][ra] = ma;
+    emB[warp][rb] = mb;
+    __syncthreads();
+    ma = max(emA[0][ra], emA[1][ra]);
+    mb = max(max(emB[0][rb], emB[1][rb]), max(emB[2][rb], emB[3][rb]));
+    if (tid < PF_M) emA[2][ra] = ma;
+    if (tid < PF_N) emB[4][rb] = mb;
+    slice_store(a0, e0, ma, sA + (ka >> 3) * (PF_M * 16) + ra * 16, PF_A_SLICE);
+    slice_store(a1, e1, ma, sA + ((ka >> 3) + 1) * (PF_M * 16) + ra * 16, PF_A_SLICE);
+    slice_store(b0, eb, mb, sB + (kb >> 3) * (PF_N * 16) + rb * 16, PF_B_SLICE);
+    __syncthreads();
+    const int g = lane >> 2, c2 = (lane & 3) * 2;  // row and column pair of a fragment
+    const int ks = K > 16 ? 2 : 1;
+    // one column group of 8 at a time: 32 accumulators, so that four CTAs
+    // share an SM (two at a time and two CTAs: 31 us against 22 us a launch)
+#pragma unroll 1
+    for (int nt = 0; nt < PF_N / 8; ++nt) {
+      float acc[8][4];
+#pragma unroll
+      for (int l = 0; l < 8; ++l)
+#pragma unroll
+        for (int x = 0; x < 4; ++x) acc[l][x] = 0.f;
+      double cv[4];
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        const int rr = row0 + warp * 16 + g + (x >> 1) * 8, cc = col0 + nt * 8 + c2 + (x & 1);
+        cv[x] = (rr < M && cc < N && rr >= cc) ? C[cc * ld + rr] : 0.0;
+      }
+      for (int k = 0; k < ks; ++k) {
+        unsigned bf[8][2];
+#pragma unroll
+        for (int s = 0; s < 8; ++s)
+          ldsm_x2(bf[s], sB + s * PF_B_SLICE + (2 * k + ((lane >> 3) & 1)) * (PF_N * 16) +
+                             (nt * 8 + (lane & 7)) * 16);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          unsigned af[4];
+          ldsm_x4(af, sA + i * PF_A_SLICE + (2 * k + (lane >> 4)) * (PF_M * 16) +
+                          (warp * 16 + (lane & 15)) * 16);
+#pragma unroll
+          for (int j = 0; j < 8 - i; ++j) mma_f16(acc[i + j], af, bf[j]);
+        }
+      }
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        const int rt = warp * 16 + g + (x >> 1) * 8, ct = nt * 8 + c2 + (x & 1);
+        const int rr = row0 + rt, cc = col0 + ct;
+        if (rr < M && cc < N && rr >= cc) {
+          const float v[8] = {acc[0][x], acc[1][x], acc[2][x], acc[3][x],
+                              acc[4][x], acc[5][x], acc[6][x], acc[7][x]};
+          const int er = emA[2][rt], ec = emB[4][ct];
+          double pr = levels_to_double(v, slice_product_exponent(er, ec));
+          if (max(er, ec) >= kSliceNonFinite / 2) pr = dinf() - dinf();
+          C[cc * ld + rr] = cv[x] - pr;
+        }
+      }
+    }
   }
 }
 
@@ -2301,6 +2473,18 @@ static int diag_f32_warps() {
   return (v == 4 || v == 8) ? v : 17;
 }
 
+// the dynamic shared memory opt-in of k_app_panel_f64, once per device
+static void panel_f64_init() {
+  constexpr int kDevices = 64;
+  static std::atomic<bool> done[kDevices];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return;
+  if (dev < kDevices && done[dev].load()) return;
+  cudaFuncSetAttribute(k_app_panel_f64, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)kPanelF64Smem);
+  if (dev < kDevices) done[dev].store(true);
+}
+
 template <typename T>
 void launch_app_step(FrontDesc<T>* fd, FrontState* st, const int* fronts, int nf, int step,
                      int max_rows, int max_trail_rows, int max_trail_cols, bool action,
@@ -2335,12 +2519,21 @@ void launch_app_step(FrontDesc<T>* fd, FrontState* st, const int* fronts, int nf
   // trailing update and fixup in one launch (tile estimate assumes no failed
   // columns so far; after failures the trailing region is wider and the
   // kernel's tile loop covers it, so the launch is never skipped)
-  constexpr int tp = panel_tile<T>();
-  int tr = std::max(0, cdiv(max_trail_rows, tp)), tc = std::max(0, cdiv(max_trail_cols, tp));
-  const int ptiles = std::max(1, std::min(tc * tr - tc * (tc - 1) / 2, 4096));
   const int nfix = std::max(1, cdiv(max_rows, 256));
   pmark(tm, kPhPanel, s);
-  launch_pdl(k_app_panel<T, tp>, dim3(ptiles + nfix, nf), 256, 0, s, fd, st, fronts, ptiles);
+  if constexpr (std::is_same<T, double>::value) {
+    panel_f64_init();
+    const int ptiles = std::max(
+        1, std::min(trapezoid_tiles<PF_N>(std::max(max_trail_rows, 0), std::max(max_trail_cols, 0)),
+                    4096));
+    launch_pdl(k_app_panel_f64, dim3(ptiles + nfix, nf), PF_THREADS, kPanelF64Smem, s, fd, st,
+               fronts, ptiles);
+  } else {
+    constexpr int tp = kPanelTile;
+    const int tr = std::max(0, cdiv(max_trail_rows, tp)), tc = std::max(0, cdiv(max_trail_cols, tp));
+    const int ptiles = std::max(1, std::min(tc * tr - tc * (tc - 1) / 2, 4096));
+    launch_pdl(k_app_panel<T, tp>, dim3(ptiles + nfix, nf), 256, 0, s, fd, st, fronts, ptiles);
+  }
   note_launches(1);
   pmark(tm, kPhSwap, s);
   const int sx = 1 + std::max(1, std::min(cdiv(max_rows + step * kBlk, 256), 64));

@@ -208,6 +208,18 @@ void cache_free(void* p, size_t cls, int dev) {
   if (cur != dev && cur >= 0) cudaSetDevice(cur);
 }
 
+// the same for callers outside the numeric handles: nullptr when the device
+// has no room (or on another CUDA error)
+void* workspace_alloc(size_t bytes, size_t* cls, int* dev) {
+  try {
+    return cache_alloc(bytes, cls, dev);
+  } catch (CudaFail const&) {
+    cudaGetLastError();
+    return nullptr;
+  }
+}
+void workspace_free(void* p, size_t cls, int dev) { cache_free(p, cls, dev); }
+
 // cudaFree on the block's device (not cached)
 void release_now(void* p, int dev) {
   int cur = -1;
@@ -993,12 +1005,12 @@ struct Numeric : NumericBase {
   // refinement a step)
   int panel_min_n = 4096;
   DevBuf<int> panel_list;   // fronts ending a panel (eager mode)
-  // FP64 factors: contribution blocks and panels' trailing updates from exact
-  // bf16 slice products on the tensor cores (slice_gemm.cu).  From
-  // slice_min_k pivots on they beat the SIMT kernel at every block size: a
-  // 64 x 64 SIMT tile takes 39 us for 32 columns whatever the block, the
-  // three slice launches 31 us (one block of 32 .. 1024 rows; 2048 rows:
-  // 44 us against 143 us, and 227 us against 4125 us for 1024 columns).
+  // FP64 factors: contribution blocks from exact FP16 slice products on the
+  // tensor cores (slice_gemm.cu).  From slice_min_k pivots on they beat the
+  // SIMT kernel at every block size: a 64 x 64 SIMT tile takes 39 us for 32
+  // columns whatever the block, the three slice launches 31 us (one block of
+  // 32 .. 1024 rows; 2048 rows: 44 us against 143 us, and 227 us against
+  // 4125 us for 1024 columns).
   bool use_slices = false;
   int slice_min_cm = 16, slice_min_k = 32;
   DevBuf<char> slice_tab, slice_scratch;
@@ -1025,7 +1037,7 @@ struct Numeric : NumericBase {
   // runs once per panel on the tensor cores with the panel's pivots as its
   // depth.  Returns the panel width of front f, or 0.
   int panel_cols(int f) const {
-    if (!(std::is_same<T, float>::value ? use_tc : use_slices) || panel_nb <= 0) return 0;
+    if (!std::is_same<T, float>::value || !use_tc || panel_nb <= 0) return 0;
     if (tpp_front(f) || S->copts.pivot_method == 3) return 0;
     return n_[f] >= std::max(panel_min_n, panel_nb + 1) ? panel_nb : 0;
   }
@@ -1060,7 +1072,6 @@ struct Numeric : NumericBase {
   }
   // end of panels in eager mode: the panels' geometry is read back (failed
   // columns move panel boundaries), then the trailing updates and the close
-  // (the slice kernels take it from the device: FP64 factors read nothing back)
   void panel_end_eager(const std::vector<int>& fl, cudaStream_t s) {
     const int nfl = (int)fl.size();
     panel_list.ensure(nfl);
@@ -1068,11 +1079,6 @@ struct Numeric : NumericBase {
     int max_n = 0;
     for (int f : fl) max_n = std::max(max_n, n_[f]);
     launch_panel_end<T>(d_fd, d_st, panel_list.p, nfl, max_n, panel_nb, s);
-    if (use_slices) {
-      slice_run(slice_panels(fl), s);
-      launch_panel_close<T>(d_fd, d_st, panel_list.p, nfl, s);
-      return;
-    }
     for (int f : fl)
       CK(cudaMemcpyAsync(&hst[f], &d_st[f], sizeof(FrontState), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
@@ -1146,20 +1152,6 @@ struct Numeric : NumericBase {
     slice_groups(b);
     return b;
   }
-  SliceBatch slice_panels(const std::vector<int>& fl) const {
-    SliceBatch b;
-    for (int f : fl) {
-      SliceJob j{};
-      j.front = f;
-      j.kind = kSlicePanel;
-      j.kcap = panel_nb;
-      j.mcap = m_[f];
-      j.ncap = n_[f];
-      b.jobs.push_back(j);
-    }
-    slice_groups(b);
-    return b;
-  }
   // lays the batch out in slice_scratch and returns its tables' image
   std::vector<char> slice_place(SliceBatch& b) const {
     std::vector<char> img(b.table, 0);
@@ -1187,14 +1179,10 @@ struct Numeric : NumericBase {
     }
   }
   // The slices' memory for the fronts of a level whose sizes are known; a
-  // device too full for it keeps the SIMT kernels (false, for this handle).
+  // device too full for it keeps the SIMT kernel (false, for this handle).
   bool slice_reserve(int f0, int f1) {
-    std::vector<int> pf;
-    for (int f = f0; f < f1; ++f)
-      if (panel_cols(f)) pf.push_back(f);
-    const size_t need = std::max(slice_contrib(f0, f1).scratch, slice_panels(pf).scratch);
     try {
-      slice_scratch.ensure(need + 1);
+      slice_scratch.ensure(slice_contrib(f0, f1).scratch + 1);
     } catch (CudaFail const& e) {
       if (e.err != cudaErrorMemoryAllocation) throw;
       cudaGetLastError();
@@ -1390,7 +1378,6 @@ struct Numeric : NumericBase {
     std::vector<PanelStep> psteps;
     std::vector<int> plist;
     std::vector<std::vector<TcProblem>> pps;
-    std::vector<SliceBatch> sps;  // FP64: slice jobs per panel end, then per level
     {
       const int per = std::max(panel_nb / kBlk, 1);
       std::vector<int> pfl;
@@ -1409,13 +1396,9 @@ struct Numeric : NumericBase {
             ps.max_n = std::max(ps.max_n, n_[f]);
             const int j = st / per, pstart = j * panel_nb;
             const int q = std::min((j + 1) * panel_nb, n_[f]);
-            if (q < n_[f] && !use_slices) pr.push_back(panel_problem(f, pstart, q, q - pstart));
+            if (q < n_[f]) pr.push_back(panel_problem(f, pstart, q, q - pstart));
           }
           if (!pr.empty()) { ps.pp = (int)pps.size(); pps.push_back(pr); }
-          if (use_slices) {
-            ps.pp = (int)sps.size();
-            sps.push_back(slice_panels(pfl));
-          }
           psteps.push_back(ps);
         }
       }
@@ -1454,7 +1437,7 @@ struct Numeric : NumericBase {
       for (size_t i = 0; i < pps.size(); ++i) pblob[i] = upload_plan(pps[i], pplans[i]);
     }
     // slice job tables (FP64), one device blob for all of them
-    const size_t npsl = sps.size();
+    std::vector<SliceBatch> sps;  // per level
     std::vector<size_t> soff;
     char* sblob = nullptr;
     if (use_slices) {
@@ -1529,8 +1512,7 @@ struct Numeric : NumericBase {
           if (pstep_i < psteps.size() && psteps[pstep_i].l == l && psteps[pstep_i].st == st) {
             const PanelStep& ps = psteps[pstep_i++];
             launch_panel_end<T>(d_fd, d_st, d_plist + ps.off, ps.nl, ps.max_n, panel_nb, s);
-            if (use_slices) slice_enqueue(sps[ps.pp], sblob + soff[ps.pp], s);
-            else if (ps.pp >= 0 &&
+            if (ps.pp >= 0 &&
                 tc_gemm_launch(pplans[ps.pp], pblob[ps.pp], d_tc_status, s, tc_chunk) != 0)
               throw CudaFail{cudaErrorUnknown, __LINE__};
             launch_panel_close<T>(d_fd, d_st, d_plist + ps.off, ps.nl, s);
@@ -1544,7 +1526,7 @@ struct Numeric : NumericBase {
         launch_contrib_gemm<T>(d_fd, d_st, fr, napp, max_app_cm, s);
         if (tblob[l] && tc_gemm_launch(tplans[l], tblob[l], d_tc_status, s, tc_chunk) != 0)
           throw CudaFail{cudaErrorUnknown, __LINE__};
-        if (use_slices) slice_enqueue(sps[npsl + l], sblob + soff[npsl + l], s);
+        if (use_slices) slice_enqueue(sps[l], sblob + soff[l], s);
         launch_stats<T>(d_fd, d_st, fr, nf, max_n, d_stats, d_ncount, s);
       }
     } catch (...) {
@@ -1710,21 +1692,10 @@ struct Numeric : NumericBase {
       const char* bi = getenv("SPRAL_GB300_SOLVE_BINV");
       use_binv = std::is_same<T, float>::value && !(bi && bi[0] == '0');
     }
-    const char* pm = getenv("SPRAL_GB300_PANEL_MIN_N");
     if (std::is_same<T, double>::value) {
       const char* env = getenv("SPRAL_GB300_TENSOR_CORES");
       use_slices = !(env && env[0] == '0');
-      // FP64 panels: 128 columns are one exact accumulation of the slice
-      // kernel and leave least to the FP64 pipe inside the panel (57^3
-      // Laplacian, a factorisation and 40 solves: 97.8 ms with 128 columns,
-      // 99.5 / 101.3 / 105.4 ms with 192 / 256 / 384).  From 576 columns on:
-      // narrower fronts would gain little more (105 ms from 768 columns) and
-      // keep the bookkeeping of failed columns of the unpaneled steps.
-      panel_nb = 128;
-      panel_min_n = pm ? std::max(0, atoi(pm)) : 576;
     }
-    const char* pn = getenv("SPRAL_GB300_PANEL");
-    if (pn) panel_nb = std::max(0, atoi(pn)) / kBlk * kBlk;
     if (std::is_same<T, float>::value) {
       const char* env = getenv("SPRAL_GB300_TENSOR_CORES");
       use_tc = !(env && env[0] == '0');
@@ -1735,6 +1706,9 @@ struct Numeric : NumericBase {
       else if (use_tc) tc_min_cm = autotune_tc_min_cm();
       const char* mk = getenv("SPRAL_GB300_TC_MIN_K");
       if (mk) tc_min_k = std::max(0, atoi(mk));
+      const char* pn = getenv("SPRAL_GB300_PANEL");
+      if (pn) panel_nb = std::max(0, atoi(pn)) / kBlk * kBlk;
+      const char* pm = getenv("SPRAL_GB300_PANEL_MIN_N");
       if (pm) panel_min_n = std::max(0, atoi(pm));
     }
     contrib.ensure(std::max<int64_t>(S->contrib_total, 1));

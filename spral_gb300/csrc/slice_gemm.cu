@@ -2,19 +2,18 @@
 //
 //   C(r, c) -= sum_k A(r, k) B(c, k),   r >= c,   everything FP64
 //
-// with A = L21 and B = L21 D of a front (the contribution block), or the
-// rows below a panel and their L D (a panel's trailing update).  GB300 issues
-// about 1.06 TF/s of FP64 multiply-adds, and 1900 TF/s of bf16 on the tensor
-// cores; the update is therefore formed from exact bf16 products (the
+// with A = L21 and B = L21 D of a front (the contribution block).  GB300 issues
+// about 1.06 TF/s of FP64 multiply-adds, and 1900 TF/s of FP16 on the tensor
+// cores; the update is therefore formed from exact FP16 products (the
 // splitting of Ozaki, Ogita, Oishi and Rump, "Error-free transformations of
 // matrix multiplication", Numer. Algorithms 59, 2012, in the form with a
 // common exponent per row that Mukunoki, Ozaki, Ogita and Imamura, "DGEMM
 // using tensor cores", ISC 2020, use on FP16 tensor cores):
 //
 //   * every row of A and of B is scaled by a power of two so that its
-//     largest entry lies in [1/2, 1), rounded to a 62-bit integer and cut
+//     largest entry lies in [1/2, 1), truncated to a 62-bit integer and cut
 //     into kSlices = 8 balanced base-256 digits in [-128, 128], each exact in
-//     bf16.  Entries within a factor 2^10 of the row's largest keep all 53
+//     FP16.  Entries within a factor 2^10 of the row's largest keep all 53
 //     bits;
 //   * the digit products of equal weight (levels l = 0..7 of the two digits'
 //     indices) are summed by tcgen05.mma in FP32 accumulators in TMEM.  A
@@ -24,7 +23,7 @@
 //   * every chunk is added to 64-bit integers, and the total becomes one FP64
 //     number, rounded once, that is subtracted from C.
 //
-// What is lost are the rounding to 62 bits and the products below level 7,
+// What is lost are the bits past the 62nd and the products below level 7,
 // about 2^-62 sqrt(K) of (row maximum of A) x (row maximum of B) in all; an
 // FP64 accumulation over K columns loses about 2^-54 sqrt(K) of the size of
 // its partial sums.  (Seven digits, 2^-55, were up to three times less exact
@@ -34,7 +33,7 @@
 // the matrix exactly.  The result of an entry depends on nothing but its two
 // rows, so a front gives the same bits alone and in a batch.
 //
-// Bound: 36 bf16 products of 16 columns per tile (128 x 64, so that the eight
+// Bound: 36 FP16 products of 16 columns per tile (128 x 64, so that the eight
 // level accumulators fit the 512 TMEM columns) at 6 KiB of shared-memory
 // operands per 32 cycles of the tensor pipe, then the integer drain of the
 // accumulators.
@@ -45,6 +44,7 @@
 #include <vector>
 
 #include "spral_ssids_gpu.h"
+#include "slices.cuh"
 #include "ssids_gpu.cuh"
 #include "tcgen05.cuh"
 
@@ -55,48 +55,24 @@ namespace {
 constexpr int SL_M = 128, SL_N = 64, SL_K = 32;  // tile rows, columns, columns per stage
 constexpr int SL_CHUNK = 4;                      // stages per exact FP32 accumulation (128 columns)
 static_assert(kSlices * SL_CHUNK * SL_K <= 1024, "a level's sum of products must stay within 2^24");
-static_assert(kSlices == 8, "the integer layouts below are those of eight digits");
+static_assert(SL_M == 2 * SL_N, "tiles of a trapezoid");
 constexpr int SL_A_SLICE = SL_M * SL_K * 2;      // 8 KiB
 constexpr int SL_B_SLICE = SL_N * SL_K * 2;      // 4 KiB
 constexpr int SL_A_BYTES = kSlices * SL_A_SLICE;  // 64 KiB per stage
 constexpr int SL_B_BYTES = kSlices * SL_B_SLICE;  // 32 KiB per stage
 constexpr int SL_STAGES = 2;
-constexpr int SL_EPI_THREADS = 256;
+constexpr int SL_EPI_THREADS = 512;
 constexpr int SL_THREADS = 64 + SL_EPI_THREADS;
-constexpr int SL_HALF = SL_N / 2;                // columns of a tile per epilogue warp
-constexpr int kNonFinite = 1 << 19;              // row exponent of a row with Inf or NaN
-static_assert(kSlices * SL_N <= 512, "TMEM columns");
+constexpr int SL_PART = SL_N / 4;                // columns of a tile per epilogue warp
+static_assert(kSlices * SL_N <= 512 && SL_PART == 16, "TMEM columns");
 
 __host__ __device__ constexpr int pad_to(int x, int p) { return (x + p - 1) / p * p; }
-
-// Tiles of the lower trapezoid M x N (N <= M): row ti of tiles holds tile
-// columns 0 .. min(tn, 2 ti + 2) - 1.
-__host__ __device__ inline int tile_count(int M, int N) {
-  const int tm = (M + SL_M - 1) / SL_M, tn = (N + SL_N - 1) / SL_N;
-  const int q = tn / 2 < tm ? tn / 2 : tm;
-  return q * (q + 1) + (tm - q) * tn;
-}
-__device__ __forceinline__ void tile_at(int t, int N, int& ti, int& tj) {
-  const int tn = (N + SL_N - 1) / SL_N;
-  const int q = tn / 2;
-  if (t >= q * (q + 1)) {
-    const int s = t - q * (q + 1);
-    ti = q + s / tn;
-    tj = s % tn;
-    return;
-  }
-  int i = (int)((sqrtf(4.0f * t + 1.0f) - 1.0f) * 0.5f);
-  while (i > 0 && i * (i + 1) > t) --i;
-  while ((i + 1) * (i + 2) <= t) ++i;
-  ti = i;
-  tj = t - i * (i + 1);
-}
 
 }  // namespace
 
 // ---------------------------------------------------------------------------
 // The geometry of every job, from the fronts' states in device memory (the
-// elimination counts and panel bounds are known only there), and the first
+// elimination counts are known only there), and the first
 // tile of each job.  One CTA.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(1024) k_slice_plan(SliceJob* jobs, int njobs, int* tile0,
@@ -117,34 +93,19 @@ __global__ void __launch_bounds__(1024) k_slice_plan(SliceJob* jobs, int njobs, 
         const FrontState st = sts[j.front];
         j.D = fd.D;
         j.lda = fd.ld;
-        if (j.kind == kSliceContrib) {
-          j.dlast = st.nelim;
-          j.c0 = j.k0;
-          j.K = max(0, min(st.nelim - j.k0, j.kcap));
-          j.A = fd.L + (int64_t)j.k0 * fd.ld + fd.n;
-          j.B = fd.LD + (int64_t)j.k0 * fd.cm;
-          j.ldb = fd.cm;
-          j.C = fd.C;
-          j.ldc = fd.ldc;
-          j.M = j.N = fd.cm;
-        } else {
-          const int q = st.qend;
-          j.dlast = st.pstart + st.pk;
-          j.c0 = st.pstart;
-          j.K = st.status == kDevOk ? max(0, min(st.pk, j.kcap)) : 0;
-          j.A = fd.L + (int64_t)st.pstart * fd.ld + q;
-          j.B = fd.LD;
-          j.ldb = fd.n;
-          j.C = fd.L + (int64_t)q * fd.ld + q;
-          j.ldc = fd.ld;
-          j.M = max(fd.m - q, 0);
-          j.N = max(fd.n - q, 0);
-        }
+        j.dlast = st.nelim;
+        j.K = max(0, min(st.nelim - j.k0, j.kcap));
+        j.A = fd.L + (int64_t)j.k0 * fd.ld + fd.n;
+        j.B = fd.LD + (int64_t)j.k0 * fd.cm;
+        j.ldb = fd.cm;
+        j.C = fd.C;
+        j.ldc = fd.ldc;
+        j.M = j.N = fd.cm;
         // the buffers were sized for at most mcap rows and ncap columns
         if (j.M > j.mcap || j.N > j.ncap || j.M <= 0 || j.N <= 0) j.K = 0;
         jobs[i] = j;
       }
-      tiles = j.K > 0 ? tile_count(j.M, j.N) : 0;
+      tiles = j.K > 0 ? trapezoid_tiles<SL_N>(j.M, j.N) : 0;
     }
     int incl = tiles;
     for (int o = 1; o < 32; o <<= 1) {
@@ -194,23 +155,9 @@ __global__ void __launch_bounds__(256) k_slice(const SliceJob* jobs) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   __shared__ short hs[kSliceMaxK];
   __shared__ int emax[8][32];
-  // column balance from D^{-1}: 1x1 pivots by their entry, 2x2 pivots by
-  // their off-diagonal entry (exponents only)
   for (int k = threadIdx.x; k < K; k += 256) {
-    int h = 0;
-    if (j.D) {
-      const int c = j.c0 + k;
-      unsigned long long v = (unsigned long long)__double_as_longlong(j.D[2 * c]);
-      const unsigned long long inf = 0x7ff0000000000000ULL;
-      if (v == inf) v = (unsigned long long)__double_as_longlong(j.D[2 * c - 1]);
-      else if (c + 1 < j.dlast &&
-               (unsigned long long)__double_as_longlong(j.D[2 * c + 2]) == inf)
-        v = (unsigned long long)__double_as_longlong(j.D[2 * c + 1]);
-      const int e = (int)((v >> 52) & 0x7ff);
-      if (e > 0 && e < 0x7ff) h = (1023 - e) >> 1;
-      if (isb) h = -h;
-    }
-    hs[k] = (short)h;
+    const int h = j.D ? slice_balance(j.D, j.k0 + k, j.dlast) : 0;
+    hs[k] = (short)(isb ? -h : h);
   }
   __syncthreads();
   const int r = row0 + lane;
@@ -228,10 +175,7 @@ __global__ void __launch_bounds__(256) k_slice(const SliceJob* jobs) {
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int k = k0 + 8 * u;
-      if ((b[u] << 1) != 0ULL) {
-        const int e = (int)((b[u] >> 52) & 0x7ff);
-        em = max(em, e == 0x7ff ? kNonFinite : max(e, 1) + (int)hs[k]);
-      }
+      if ((b[u] << 1) != 0ULL) em = max(em, slice_exponent(b[u], hs[k]));
     }
   }
   emax[warp][lane] = em;
@@ -252,46 +196,11 @@ __global__ void __launch_bounds__(256) k_slice(const SliceJob* jobs) {
       b[q] = (valid && k0 + q < K)
                  ? (unsigned long long)__double_as_longlong(col[(int64_t)(k0 + q) * ld])
                  : 0ULL;
-    unsigned zl[8], zh[8];
+    int e[8];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const int e = (int)((b[q] >> 52) & 0x7ff);
-      unsigned long long m = b[q] & 0xfffffffffffffULL;
-      if (e) m |= 1ULL << 52;
-      // X = value * 2^62 / 2^(em - 1022), rounded to nearest
-      const int sh = 9 - (em - (max(e, 1) + (int)(k0 + q < K ? hs[k0 + q] : 0)));
-      unsigned long long X;
-      if (sh >= 0) X = m << min(sh, 9);
-      else X = sh < -55 ? 0ULL : (m + (1ULL << (-sh - 1))) >> -sh;
-      if (e == 0x7ff) X = 0ULL;
-      const long long Y = (b[q] >> 63) ? -(long long)X : (long long)X;
-      // balanced digits: the bytes of Y + 0x80808080808080, minus 128, below
-      // the signed top digit
-      const unsigned long long Z = (unsigned long long)(Y + 0x0080808080808080LL);
-      zl[q] = (unsigned)Z;
-      zh[q] = (unsigned)(Z >> 32);
-    }
-    char* d = dst + (int64_t)(o >> 2) * piece + (o & 3) * (pad * 16);
-#pragma unroll
-    for (int s = 0; s < kSlices; ++s) {
-      const int byte = kSlices - 1 - s;  // of Z, from the lowest
-      unsigned w[4];
-#pragma unroll
-      for (int p = 0; p < 4; ++p) {
-        float f[2];
-#pragma unroll
-        for (int t = 0; t < 2; ++t) {
-          const unsigned a = zl[2 * p + t], c = zh[2 * p + t];
-          if (byte == 7) f[t] = (float)((int)c >> 24);
-          else
-            f[t] = __uint_as_float(__byte_perm(byte < 4 ? a : c, 0x4B000000u,
-                                               0x7440u | (unsigned)(byte & 3))) -
-                   8388736.0f;  // 2^23 + 128
-        }
-        asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(w[p]) : "f"(f[1]), "f"(f[0]));
-      }
-      *reinterpret_cast<uint4*>(d + (int64_t)s * (pad * SL_K * 2)) = make_uint4(w[0], w[1], w[2], w[3]);
-    }
+    for (int q = 0; q < 8; ++q) e[q] = slice_exponent(b[q], k0 + q < K ? hs[k0 + q] : 0);
+    slice_store(b, e, em, dst + (int64_t)(o >> 2) * piece + (o & 3) * (pad * 16),
+                pad * SL_K * 2);
   }
 }
 
@@ -314,46 +223,8 @@ __device__ __forceinline__ uint64_t smem_desc_plain(uint32_t saddr, uint32_t lea
          ((uint64_t)(128 >> 4) << 32) | ((uint64_t)1 << 46);
 }
 
-// D = F32, A = B = BF16, both K-major, N = SL_N, M = SL_M
-constexpr uint32_t kIdescBf16 = (1u << 4) | (1u << 7) | (1u << 10) |
-                                ((uint32_t)(SL_N >> 3) << 17) | ((uint32_t)(SL_M >> 4) << 24);
-
-// The FP64 number nearest to (H 2^32 + L) 2^e, |H| < 2^63, |L| < 2^63
-__device__ __forceinline__ double fixed_to_double(long long H, long long L, int e) {
-  unsigned long long lo = (unsigned long long)H << 32;
-  long long hi = H >> 32;
-  const unsigned long long l = (unsigned long long)L;
-  lo += l;
-  hi += (L >> 63) + (lo < l ? 1 : 0);
-  const bool neg = hi < 0;
-  if (neg) {
-    hi = ~hi + (lo == 0ULL ? 1 : 0);
-    lo = 0ULL - lo;
-  }
-  // the leading 64 bits, the rest as a sticky bit
-  unsigned long long m = lo;
-  if (hi != 0) {
-    const int z = __clzll(hi);  // 1 <= z: the sign is gone
-    m = ((unsigned long long)hi << z) | (lo >> (64 - z)) | ((lo << z) != 0ULL ? 1ULL : 0ULL);
-    e += 64 - z;
-  }
-  if (m == 0ULL) return 0.0;
-  const int z = __clzll(m);
-  m <<= z;
-  e += 63 - z;
-  unsigned long long q = m >> 11;  // 53 bits
-  const unsigned rem = (unsigned)m & 0x7ffu;
-  q += (rem > 0x400u || (rem == 0x400u && (q & 1ULL))) ? 1ULL : 0ULL;
-  const int E = e + 1023;
-  if (E <= 0 || E >= 2046) {  // outside the normal range: rare
-    const double v = ldexp((double)q, e - 52);
-    return neg ? -v : v;
-  }
-  // a carry of the rounding runs into the exponent, as it should
-  const unsigned long long bits =
-      ((unsigned long long)(E - 1) << 52) + q + (neg ? 1ULL << 63 : 0ULL);
-  return __longlong_as_double((long long)bits);
-}
+// D = F32, A = B = F16, both K-major, N = SL_N, M = SL_M
+constexpr uint32_t kIdescF16 = (1u << 4) | ((uint32_t)(SL_N >> 3) << 17) | ((uint32_t)(SL_M >> 4) << 24);
 
 }  // namespace
 
@@ -363,9 +234,11 @@ __device__ __forceinline__ double fixed_to_double(long long H, long long L, int 
 //                   into a ring of two
 //   warp 1 lane 0   tcgen05.mma: 36 slice products per stage, summed by level
 //                   into eight TMEM accumulators
-//   warps 2..9      every chunk, the eight accumulators into 64-bit integers
+//   warps 2..17     every chunk, the eight accumulators into 64-bit integers
 //                   (levels 0..3 and 4..7), after the last one C
-// The next tile's products run while this tile's C is updated.
+// The next tile's products run while this tile's C is updated.  The drain is
+// bound by the latency of the TMEM loads: sixteen warps of 16 columns each
+// (eight of 32: 10,000 cycles a chunk beside 17,000 of products).
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(SL_THREADS, 1)
     k_slice_gemm(const SliceJob* jobs, const int* tile0, int njobs, int* status) {
@@ -425,7 +298,7 @@ __global__ void __launch_bounds__(SL_THREADS, 1)
         const int ji = job_of(t);
         const SliceJob& j = jobs[ji];
         int ti, tj;
-        tile_at(t - tile0[ji], j.N, ti, tj);
+        trapezoid_tile<SL_N>(t - tile0[ji], j.N, ti, tj);
         const int nkt = (j.K + SL_K - 1) / SL_K;
         const char* a = j.sA + (int64_t)ti * nkt * SL_A_BYTES;
         const char* b = j.sB + (int64_t)tj * nkt * SL_B_BYTES;
@@ -474,7 +347,7 @@ __global__ void __launch_bounds__(SL_THREADS, 1)
                       "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
                       " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(
                           tmem + l * SL_N),
-                      "l"(ad), "l"(bd), "r"(kIdescBf16), "r"(acc));
+                      "l"(ad), "l"(bd), "r"(kIdescF16), "r"(acc));
                 }
               }
             }
@@ -489,40 +362,37 @@ __global__ void __launch_bounds__(SL_THREADS, 1)
     }
   } else {
     // ---- drain and C ----
-    // warp w reads TMEM lane quarter w % 4 and owns the column half
-    // (w - 2) / 4: one row and 32 columns of the tile per thread
+    // warp w reads TMEM lane quarter w % 4 and owns the column quarter
+    // (w - 2) / 4: one row and 16 columns of the tile per thread
     const int q = warp & 3;
-    const int half = (warp - 2) >> 2;
+    const int part = (warp - 2) >> 2;
     uint32_t ch = 0;
     bool ok = true;
     for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
       const int ji = job_of(t);
       const SliceJob& j = jobs[ji];
       int ti, tj;
-      tile_at(t - tile0[ji], j.N, ti, tj);
+      trapezoid_tile<SL_N>(t - tile0[ji], j.N, ti, tj);
       const int nkt = (j.K + SL_K - 1) / SL_K;
-      long long H[SL_HALF], L[SL_HALF];
+      long long H[SL_PART], L[SL_PART];
 #pragma unroll
-      for (int c = 0; c < SL_HALF; ++c) H[c] = L[c] = 0;
+      for (int c = 0; c < SL_PART; ++c) H[c] = L[c] = 0;
       for (int k0 = 0; k0 < nkt; k0 += SL_CHUNK, ++ch) {
         // the TMEM loads below are warp-collective: decide as a warp
         const bool got = mbar_wait(accf, ch & 1, abort_flag);
         if (!__all_sync(0xffffffffu, got)) { *abort_flag = 1; ok = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;");
-        const uint32_t tbase = tmem + ((uint32_t)(q * 32) << 16) + half * SL_HALF;
+        const uint32_t tbase = tmem + ((uint32_t)(q * 32) << 16) + part * SL_PART;
 #pragma unroll
         for (int l = 0; l < kSlices; ++l) {
           const int w = 1 << (8 * (3 - l % 4));
+          uint32_t v[16];
+          tmem_ld16(tbase + (uint32_t)(l * SL_N), v);
 #pragma unroll
-          for (int cb = 0; cb < SL_HALF; cb += 16) {
-            uint32_t v[16];
-            tmem_ld16(tbase + (uint32_t)(l * SL_N + cb), v);
-#pragma unroll
-            for (int c = 0; c < 16; ++c) {
-              const long long p = (long long)__float2int_rn(__uint_as_float(v[c])) * w;
-              if (l < 4) H[cb + c] += p;
-              else L[cb + c] += p;
-            }
+          for (int c = 0; c < SL_PART; ++c) {
+            const long long p = (long long)__float2int_rn(__uint_as_float(v[c])) * w;
+            if (l < 4) H[c] += p;
+            else L[c] += p;
           }
         }
         asm volatile("tcgen05.fence::before_thread_sync;");
@@ -531,7 +401,7 @@ __global__ void __launch_bounds__(SL_THREADS, 1)
       if (!ok) break;
       const int r = ti * SL_M + q * 32 + lane;
       if (r >= j.M) continue;
-      const int col0 = tj * SL_N + half * SL_HALF;
+      const int col0 = tj * SL_N + part * SL_PART;
       const int er = j.eA[r];
       const int* eb = j.eB + col0;
       const int64_t ldc = j.ldc;
@@ -539,7 +409,7 @@ __global__ void __launch_bounds__(SL_THREADS, 1)
       const int N = j.N;
       // 4 columns at a time: all loads in flight before the stores
 #pragma unroll
-      for (int cb = 0; cb < SL_HALF; cb += 4) {
+      for (int cb = 0; cb < SL_PART; cb += 4) {
         double cv[4];
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
@@ -551,9 +421,8 @@ __global__ void __launch_bounds__(SL_THREADS, 1)
           const int cc = col0 + cb + c;
           if (cc < N && r >= cc) {
             const int ec = eb[cb + c];
-            // X_A X_B = T 2^56, each X = value 2^62 / 2^(exponent - 1022)
-            double p = fixed_to_double(H[cb + c], L[cb + c], er + ec - 2044 - 68);
-            if (max(er, ec) >= kNonFinite / 2) p = __longlong_as_double(0x7ff8000000000000LL);
+            double p = fixed_to_double(H[cb + c], L[cb + c], slice_product_exponent(er, ec));
+            if (max(er, ec) >= kSliceNonFinite / 2) p = __longlong_as_double(0x7ff8000000000000LL);
             crow[(cb + c) * ldc] = cv[c] - p;
           }
         }
@@ -614,7 +483,7 @@ int launch_slice_gemm(void* table, const std::vector<SliceJob>& jobs, size_t fir
   long long tiles = 0;
   for (size_t i = first; i < first + count; ++i) {
     rows = std::max(rows, std::max(pad_to(jobs[i].mcap, SL_M), pad_to(jobs[i].ncap, SL_N)));
-    tiles += tile_count(jobs[i].mcap, jobs[i].ncap);
+    tiles += trapezoid_tiles<SL_N>(jobs[i].mcap, jobs[i].ncap);
   }
   int dev = 0, nsm = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return -3;

@@ -1,0 +1,156 @@
+// FP64 operands as eight balanced base-256 digits (exact in FP16), and the
+// way back from exact digit-product sums to FP64: shared by the kernels that
+// form FP64 products on the tensor cores (the method is described in
+// slice_gemm.cu).  Integer instructions only: an FP64 instruction issues some
+// 70 times slower on GB300.
+#pragma once
+#include <climits>
+#include <cstdint>
+#include <cuda_runtime.h>
+
+namespace ssids300 {
+
+// exponent of a row with Inf or NaN: the products of the row become NaN
+constexpr int kSliceNonFinite = 1 << 19;
+
+// biased exponent of an entry after its column's balance 2^h
+__device__ __forceinline__ int slice_exponent(unsigned long long bits, int h) {
+  const int e = (int)((bits >> 52) & 0x7ff);
+  return e == 0x7ff ? kSliceNonFinite : max(e, 1) + h;
+}
+
+// Column balance 2^h ~ sqrt|D| of pivot column c from D^{-1}: a 1x1 pivot by
+// its entry, a 2x2 pivot by its off-diagonal entry (exponents only); dlast
+// ends the pivots.
+__device__ __forceinline__ int slice_balance(const double* D, int c, int dlast) {
+  const unsigned long long inf = 0x7ff0000000000000ULL;
+  unsigned long long v = (unsigned long long)__double_as_longlong(D[2 * c]);
+  if (v == inf) v = (unsigned long long)__double_as_longlong(D[2 * c - 1]);
+  else if (c + 1 < dlast && (unsigned long long)__double_as_longlong(D[2 * c + 2]) == inf)
+    v = (unsigned long long)__double_as_longlong(D[2 * c + 1]);
+  const int e = (int)((v >> 52) & 0x7ff);
+  return (e > 0 && e < 0x7ff) ? (1023 - e) >> 1 : 0;
+}
+
+// Digits of eight consecutive columns of one row (entries b, exponents e after
+// the balance, row exponent em): slice s (0 the leading digit) goes to the 16
+// bytes at d + s * stride, as eight FP16 values.
+__device__ __forceinline__ void slice_store(const unsigned long long (&b)[8], const int (&e)[8],
+                                            int em, char* d, int64_t stride) {
+  unsigned zl[8], zh[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const unsigned hi = (unsigned)(b[q] >> 32), lo = (unsigned)b[q];
+    const unsigned m = (hi & 0xfffffu) | ((hi & 0x7ff00000u) ? 0x100000u : 0u);
+    // |value| 2^62 / 2^(em - 1022), truncated; the mantissa's 53 bits start
+    // at bit 61 for the row's largest exponent.  (A zero's exponent may
+    // exceed em; entries of a row with Inf or NaN have no meaning.)
+    const unsigned long long M =
+        ((unsigned long long)__funnelshift_l(lo, m, 9) << 32) | (unsigned long long)(lo << 9);
+    const unsigned long long X = M >> min(max(em - e[q], 0), 63);
+    // balanced digits: the bytes of +-X + 0x8080808080808080, minus 128
+    const long long sg = (long long)((int)hi >> 31);
+    const unsigned long long Z =
+        (X ^ (unsigned long long)sg) + (0x8080808080808080ULL - (unsigned long long)sg);
+    zl[q] = (unsigned)Z;
+    zh[q] = (unsigned)(Z >> 32);
+  }
+#pragma unroll
+  for (int s = 0; s < 8; ++s) {
+    const int byte = (7 - s) & 3;  // of the upper (s < 4) or lower word
+    unsigned w[4];
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+      // FP16 1024 + byte for two columns, minus 1152: exact
+      const unsigned t = __byte_perm(s < 4 ? zh[2 * p] : zl[2 * p], s < 4 ? zh[2 * p + 1] : zl[2 * p + 1],
+                                     (unsigned)(byte | (byte << 4) | ((4 + byte) << 8) | ((4 + byte) << 12)));
+      asm("{\n .reg .b32 t;\n lop3.b32 t, %1, 0x00ff00ff, 0x64006400, 0xea;\n"
+          " sub.rn.f16x2 %0, t, %2;\n}\n"
+          : "=r"(w[p])
+          : "r"(t), "r"(0x64806480u));
+    }
+    *reinterpret_cast<uint4*>(d + s * stride) = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+}
+
+// The FP64 number nearest to (w2 2^64 + w1 2^32 + w0) 2^e, a 96-bit integer in
+// two's complement
+__device__ __forceinline__ double fixed_to_double(int w2, unsigned w1, unsigned w0, int e) {
+  const unsigned sg = (unsigned)(w2 >> 31);
+  // magnitude
+  unsigned long long lo = ((unsigned long long)(w1 ^ sg) << 32) | (unsigned long long)(w0 ^ sg);
+  const unsigned c = sg & 1u;
+  lo += c;
+  unsigned hi = ((unsigned)w2 ^ sg) + ((lo < (unsigned long long)c) ? 1u : 0u);
+  if (hi == 0) {
+    hi = (unsigned)(lo >> 32);
+    lo <<= 32;
+    e -= 32;
+  }
+  if (hi == 0) {
+    hi = (unsigned)(lo >> 32);
+    lo <<= 32;
+    e -= 32;
+    if (hi == 0) {
+      hi = (unsigned)(lo >> 32);
+      lo = 0;
+      e -= 32;
+      if (hi == 0) return 0.0;
+    }
+  }
+  const int z = __clz(hi);
+  const unsigned t1 = __funnelshift_l((unsigned)(lo >> 32), hi, z);
+  const unsigned t0 = __funnelshift_l((unsigned)lo, (unsigned)(lo >> 32), z);
+  // 53 bits, to nearest on the next one (the bits below it cannot matter by
+  // more than 2^-11 of a unit)
+  const unsigned long long q =
+      ((((unsigned long long)t1 << 32) | t0) >> 11) + (unsigned long long)((t0 >> 10) & 1u);
+  const int E = e + 95 - z + 1023;
+  const unsigned long long sign = (unsigned long long)(sg & 0x80000000u) << 32;
+  if (E <= 0 || E >= 2046) {  // outside the normal range: rare
+    const double v = ldexp((double)q, E - 1023 - 52);
+    return sg ? -v : v;
+  }
+  // a carry of the rounding runs into the exponent, as it should
+  return __longlong_as_double((long long)((((unsigned long long)(E - 1)) << 52) + q + sign));
+}
+// (H 2^32 + L) 2^e with |H|, |L| < 2^62
+__device__ __forceinline__ double fixed_to_double(long long H, long long L, int e) {
+  const unsigned long long l = (unsigned long long)L;
+  const unsigned long long lo = ((unsigned long long)H << 32) + l;
+  const int hi = (int)(H >> 32) + (int)(L >> 63) + (lo < l ? 1 : 0);
+  return fixed_to_double(hi, (unsigned)(lo >> 32), (unsigned)lo, e);
+}
+
+// Exponent of two for fixed_to_double of a product sum of rows with exponents
+// er and ec: X_A X_B = T 2^56, each X = value 2^62 / 2^(exponent - 1022)
+__device__ __forceinline__ int slice_product_exponent(int er, int ec) {
+  return er + ec - 2044 - 68;
+}
+
+// Tiles of 2 TN x TN of the lower trapezoid M x N: row ti of tiles holds
+// tile columns 0 .. min(tn, 2 ti + 2) - 1.
+template <int TN>
+__host__ __device__ inline int trapezoid_tiles(int M, int N) {
+  const int tm = (M + 2 * TN - 1) / (2 * TN), tn = (N + TN - 1) / TN;
+  const int q = tn / 2 < tm ? tn / 2 : tm;
+  return q * (q + 1) + (tm - q) * tn;
+}
+template <int TN>
+__device__ __forceinline__ void trapezoid_tile(int t, int N, int& ti, int& tj) {
+  const int tn = (N + TN - 1) / TN;
+  const int q = tn / 2;
+  if (t >= q * (q + 1)) {
+    const int s = t - q * (q + 1);
+    ti = q + s / tn;
+    tj = s % tn;
+    return;
+  }
+  int i = (int)((sqrtf(4.0f * t + 1.0f) - 1.0f) * 0.5f);
+  while (i > 0 && i * (i + 1) > t) --i;
+  while ((i + 1) * (i + 2) <= t) ++i;
+  ti = i;
+  tj = t - i * (i + 1);
+}
+
+}  // namespace ssids300

@@ -79,7 +79,7 @@ struct FrontDesc {
   int panel;     // > 0: APP in panels of this many candidate columns (see below)
 };
 
-// Panels (wide fronts, see Numeric::panel_cols): the APP block
+// Panels (FP32 factors, fronts wider than FrontDesc::panel): the APP block
 // steps draw their candidates from a panel of `panel` columns [pstart, qend)
 // and update only the panel's columns; at the panel's end the trailing
 // fully-summed columns [qend, n) take the panel's pk pivots in one
@@ -105,6 +105,11 @@ struct Stats {  // device-side reduction target (integers only -> deterministic)
   int num_neg, num_two, num_zero, num_delay;
   long long num_factor, num_flops;
 };
+
+// Device workspace from the per-device block cache (numeric.cu), whose blocks
+// go back to it once the work that uses them has finished.
+void* workspace_alloc(size_t bytes, size_t* cls, int* dev);
+void workspace_free(void* p, size_t cls, int dev);
 
 // Count of kernels launched by this library (reported by the benchmark).
 void note_launches(int k);
@@ -247,13 +252,12 @@ int tc_gemm_run(const std::vector<TcProblem>& ps, void* scratch, TcBuffers& buf,
                 float* ms_gemm = nullptr, int bn = 0);
 
 // ---------------- FP64 updates on the tensor cores (slice_gemm.cu) ----------------
-// C -= A B^T (r >= c), all FP64, from exact bf16 slice products.  A job is
-// one front's contribution block (pivots [k0, k0 + kcap)), one closed panel's
-// trailing update, or operands given by the caller; k_slice_plan completes it
-// on the device from the front's state.
+// C -= A B^T (r >= c), all FP64, from exact FP16 slice products.  A job is
+// one front's contribution block (pivots [k0, k0 + kcap)) or operands given by
+// the caller; k_slice_plan completes it on the device from the front's state.
 constexpr int kSlices = 8;         // base-256 digits of an operand
 constexpr int kSliceMaxK = 2048;   // deepest job (bounds the slices' memory)
-enum SliceKind : int { kSliceContrib = 0, kSlicePanel, kSliceGiven };
+enum SliceKind : int { kSliceContrib = 0, kSliceGiven };
 struct SliceJob {
   int front, kind, k0, kcap;  // kcap: columns the buffers hold
   int mcap, ncap;             // rows of A and of B the buffers hold
@@ -263,7 +267,7 @@ struct SliceJob {
   const double *A, *B, *D;    // D: D^{-1} for the column balance, or nullptr
   double* C;
   int lda, ldb, ldc, M, N, K;
-  int c0, dlast;              // first pivot column, end of the pivots
+  int dlast;                  // end of the pivots (k0 is the first)
 };
 size_t slice_job_bytes(int mcap, int ncap, int kcap);
 void slice_job_place(SliceJob& j, char* base);  // lays the job's buffers out at base
