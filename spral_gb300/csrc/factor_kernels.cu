@@ -40,20 +40,27 @@ __device__ __forceinline__ double dinf() { return __longlong_as_double(0x7ff0000
 
 }  // namespace
 
-// Reciprocal by Newton-Raphson iteration y <- y + y (1 - x y) from an FP32
-// seed (each step squares the relative error: 2^-23 -> 2^-46 -> 2^-92), so
-// the result is within one ulp of 1/x.  Two FP64 FMA pairs replace the long
-// dependent sequence of a correctly rounded FP64 division, which matters on
-// the serial path of the pivot decisions.  Arguments whose magnitude is
+// Reciprocal by one third-order step y (1 + e + e^2), e = 1 - x y, from an
+// FP32 seed (relative error below 2^-22, cubed by the step), so the result is
+// within one ulp of 1/x.  Three dependent FP64 instructions replace the long
+// sequence of a correctly rounded division, which matters on the serial path
+// of the pivot decisions; the seed is formed with integer instructions, a
+// conversion being an FP64 instruction too.  Arguments whose magnitude is
 // outside [2^-100, 2^100] (or zero/Inf/NaN) use ordinary division.
 __device__ __forceinline__ double recip_nr(double x) {
-  const int e = (int)((__double_as_longlong(x) >> 52) & 0x7ff);
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+  const int e = (int)((hi >> 20) & 0x7ff);
   if (e < 1023 - 100 || e > 1023 + 100) return 1.0 / x;
-  double y = (double)__frcp_rn((float)x);
-  double r = fma(-x, y, 1.0);
-  y = fma(y, r, y);
-  r = fma(-x, y, 1.0);
-  return fma(y, r, y);
+  const unsigned xb = (hi & 0x80000000u) | ((unsigned)(e - 1023 + 127) << 23) |
+                      ((hi & 0xfffffu) << 3) | (lo >> 29);
+  float yf;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(yf) : "f"(__uint_as_float(xb)));
+  const unsigned yb = __float_as_uint(yf);
+  const double y = __hiloint2double(
+      (int)((yb & 0x80000000u) | ((((yb >> 23) & 0xff) + 1023 - 127) << 20) | ((yb >> 3) & 0xfffffu)),
+      (int)(yb << 29));
+  const double r = fma(-x, y, 1.0);
+  return fma(y, fma(r, r, r), y);
 }
 
 __global__ void k_recip_probe(const double* x, double* y, int n) {
@@ -168,6 +175,27 @@ __device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long k)
 constexpr int kDiagPairs = kBlk * (kBlk + 1) / 2;
 constexpr int kDiagThreads = (kDiagPairs + 31) / 32 * 32;
 
+// 2x2 test in FP32 for FP64 entries, |a21| the largest: 1 or 0 when certain,
+// -1 when a rounding could decide.  (a11 a22 / a21^2 - 1 against 1/2, each
+// entry scaled by the exponent of a21 and cut to FP32.)
+__device__ __forceinline__ float scaled_f32(double v, int e21) {
+  const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
+  const int ev = (int)((hi >> 20) & 0x7ff), e = ev - e21 + 127;
+  if (ev == 0 || e <= 0) return 0.f;
+  return __uint_as_float((hi & 0x80000000u) | ((unsigned)min(e, 254) << 23) |
+                         ((hi & 0xfffffu) << 3) | (lo >> 29));
+}
+__device__ __forceinline__ int two_by_two_f32(double a11, double a21, double a22) {
+  const int e21 = (int)(((unsigned)__double2hiint(a21) >> 20) & 0x7ff);
+  if (e21 < 64) return -1;
+  const float f21 = scaled_f32(a21, e21);
+  float inv;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(f21));
+  const float rho = (scaled_f32(a11, e21) * inv) * (scaled_f32(a22, e21) * inv);
+  const float d = fabsf(rho - 1.0f) - 0.5f;
+  return d > 1e-4f ? 1 : d < -1e-4f ? 0 : -1;
+}
+
 // POSDEF: the Cholesky case (cpu/kernels/cholesky.cxx, LAPACK potrf): no
 // pivoting, pivot q is the block's q-th diagonal, and a pivot that is not
 // > 0 ends the factorisation with kDevNotPosdef.  The factors are kept as
@@ -246,25 +274,35 @@ __global__ void __launch_bounds__(kDiagThreads) k_app_diag(FrontDesc<T>* fds, Fr
       if (POSDEF) {
         i1 = q;  // no pivoting
         if (!((double)blk[q][q] > 0.0)) pivsiz = -1;
-      } else if (bv < small) {
+      } else if (kF64 ? ((gk & 0x7fffffffffffffffULL) | 0x3ffULL) <
+                             (unsigned long long)__double_as_longlong(small)
+                      : bv < small) {
         pivsiz = 0;
       } else if (bi != bj) {
         const int mm = map[bj], tt = map[bi];
         const double a11 = (double)blk[mm][mm], a22 = (double)blk[tt][tt];
         const double a21 = (double)blk[mm][tt];
-        const double detscale = recip_nr(fabs(a21));
-        const double detpiv = (a11 * detscale) * a22 - fabs(a21);
-        if (fabs(detpiv) >= fabs(a21) / 2) {
-          pivsiz = 2; i1 = bj; i2 = bi;
-          const double rdet = recip_nr(detpiv);
-          e11 = (a22 * detscale) * rdet;
-          e21 = (-a21 * detscale) * rdet;
-          e22 = (a11 * detscale) * rdet;
-        } else if (fabs(a11) > fabs(a22)) {
-          i1 = bj;
-        } else {
-          i1 = bi;
+        // FP64 factors: the test in FP32 where that is certain
+        const int t = kF64 ? two_by_two_f32(a11, a21, a22) : -1;
+        bool two = t == 1;
+        if (t != 0) {
+          const double detscale = recip_nr(fabs(a21));
+          // three lanes: a22, -a21, a11 times the scale
+          const double x = (lane == 0 ? a22 : lane == 1 ? -a21 : a11) * detscale;
+          const double detpiv = fma(__shfl_sync(0xffffffffu, x, 2), a22, -fabs(a21));
+          if (t < 0) two = fabs(detpiv) >= fabs(a21) / 2;
+          if (two) {
+            pivsiz = 2; i1 = bj; i2 = bi;
+            const double ee = x * recip_nr(detpiv);
+            e11 = __shfl_sync(0xffffffffu, ee, 0);
+            e21 = __shfl_sync(0xffffffffu, ee, 1);
+            e22 = __shfl_sync(0xffffffffu, ee, 2);
+          }
         }
+        if (!two)
+          i1 = (__double_as_longlong(a11) & 0x7fffffffffffffffLL) >
+                       (__double_as_longlong(a22) & 0x7fffffffffffffffLL)
+                   ? bj : bi;
       }
       if (pivsiz > 0) {
         // logical swaps q <-> i1, then q+1 <-> i2 (i2 > i1 >= q) on the
@@ -663,20 +701,62 @@ __global__ void __launch_bounds__(NW * 32)
 // CTAs moves per round
 constexpr int kPermCols = 8;
 
-// ------------------------------------------------------------------------
-// k_app_apply: rows below the block; solve, scale, threshold test
-// ------------------------------------------------------------------------
-// threads per apply CTA and rows per tile: FP32, one row per thread (64);
-// FP64, 32 rows shared by 4 warps (column blocks, see the solve below)
-template <typename T>
-__host__ __device__ constexpr int apply_threads() { return sizeof(T) == 8 ? 128 : kApplyRows; }
-template <typename T>
-__host__ __device__ constexpr int apply_rows() { return sizeof(T) == 8 ? 32 : kApplyRows; }
+// alpha lv + beta lp for FP32 factors in FP32 instructions, alpha and beta
+// given as float pairs (hi + lo): the two hi products with their exact
+// errors (FMA), their sum with its exact error (two-sum), then the error
+// and lo terms added once, so the result is within an ulp of the FP64
+// expression rounded to FP32, a 2x2 column's cancelling products included
+__device__ __forceinline__ float ld_entry_f32(float ahi, float alo, float bhi, float blo,
+                                              float lv, float lp) {
+  const float p1 = __fmul_rn(ahi, lv), e1 = __fmaf_rn(ahi, lv, -p1);
+  const float p2 = __fmul_rn(bhi, lp), e2 = __fmaf_rn(bhi, lp, -p2);
+  const float sm = __fadd_rn(p1, p2);
+  const float bb = __fsub_rn(sm, p1);
+  const float es = __fadd_rn(__fsub_rn(p1, __fsub_rn(sm, bb)), __fsub_rn(p2, bb));
+  const float corr = __fmaf_rn(alo, lv, __fmaf_rn(blo, lp, __fadd_rn(__fadd_rn(e1, e2), es)));
+  return __fadd_rn(sm, corr);
+}
 
+// Permutation CTAs of the apply launch (index cta of ncta): the block
+// permutation of rows [p, p+bs) in the eliminated columns [0, p).  A warp
+// permutes kPermCols columns per round: all loads, then all stores.
 template <typename T>
-__global__ void __launch_bounds__(apply_threads<T>()) k_app_apply(FrontDesc<T>* fds, FrontState* sts,
-                                                          const int* fronts, double u,
+__device__ __forceinline__ void app_permute(const FrontDesc<T>& fd, int p, int bs, int cta,
+                                            int ncta) {
+  if (p == 0) return;
+  constexpr int U = kPermCols;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int src = (lane < bs) ? fd.lperm[lane] : lane;
+  const int wstride = ncta * nw;
+  for (int c0 = (cta * nw + warp) * U; c0 < p; c0 += wstride * U) {
+    T v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      v[u] = (lane < bs && c0 + u < p) ? fd.L[(int64_t)(c0 + u) * fd.ld + p + src] : T(0);
+    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (lane < bs && c0 + u < p) fd.L[(int64_t)(c0 + u) * fd.ld + p + lane] = v[u];
+  }
+}
+
+// pivot kinds of a block's columns: 0 1x1, 1 first of a 2x2, 2 second, 3 zero
+__device__ __forceinline__ int pivot_kind(const double* dd, int j, int bs) {
+  if (j >= bs) return 0;
+  if (isinf(dd[2 * j])) return 2;
+  if (j + 1 < bs && isinf(dd[2 * j + 2])) return 1;
+  return dd[2 * j] == 0.0 ? 3 : 0;
+}
+
+// ------------------------------------------------------------------------
+// k_app_apply: rows below the block; solve, scale, threshold test.  FP32:
+// one row per thread.
+// ------------------------------------------------------------------------
+__global__ void __launch_bounds__(kApplyRows) k_app_apply(FrontDesc<float>* fds, FrontState* sts,
+                                                          const int* fronts, double thresh,
+                                                          float thr_lo, float thr_hi,
                                                           double small, int napply) {
+  using T = float;
   const int f = fronts[blockIdx.y];
   FrontDesc<T> fd = fds[f];  // written by the host before the launch
   pdl_wait();
@@ -686,78 +766,61 @@ __global__ void __launch_bounds__(apply_threads<T>()) k_app_apply(FrontDesc<T>* 
   if (bs == 0) return;
   const int p = st->p;
   if ((int)blockIdx.x >= napply) {
-    // block permutation of rows [p, p+bs) in the eliminated columns [0, p)
-    if (p == 0) return;
-    // a warp permutes kPermCols columns per round: all loads, then all stores
-    constexpr int U = kPermCols;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const int src = (lane < bs) ? fd.lperm[lane] : lane;
-    const int wstride = (gridDim.x - napply) * nw;
-    for (int c0 = ((blockIdx.x - napply) * nw + warp) * U; c0 < p; c0 += wstride * U) {
-      T v[U];
-#pragma unroll
-      for (int u = 0; u < U; ++u)
-        v[u] = (lane < bs && c0 + u < p) ? fd.L[(int64_t)(c0 + u) * fd.ld + p + src] : T(0);
-      __syncwarp();
-#pragma unroll
-      for (int u = 0; u < U; ++u)
-        if (lane < bs && c0 + u < p) fd.L[(int64_t)(c0 + u) * fd.ld + p + lane] = v[u];
-    }
+    app_permute<T>(fd, p, bs, blockIdx.x - napply, gridDim.x - napply);
     return;
   }
   const int r0 = p + bs;
   const int nrows = fd.m - r0;
   if (nrows <= 0) return;
-  // X = A21 L11^{-T} in the factor precision T; D^{-1} application and the
-  // a-posteriori test in FP64.  Few warps run this kernel on an SM, so its
-  // code is kept short: L11 is staged transposed (l11t[k][j] = L(j, k),
+  // X = A21 L11^{-T} in FP32; D^{-1} application and the a-posteriori test
+  // in FP64 where FP32 is not certain.  Few warps run this kernel on an SM,
+  // so its code is kept short: L11 is staged transposed (l11t[k][j] = L(j, k),
   // rows 16-byte aligned) for vector loads in the unrolled solve, and the
   // per-column epilogue is a rolled loop over X staged in shared memory,
-  // driven by the pivot kind of each column.
+  // driven by the pivot kind of each column.  FP64 instructions (conversions
+  // among them) issue for 75 cycles, so L11 is read as the FP32 factor it is,
+  // 2x2 columns are multiplied by D^{-1} in error-free FP32 products
+  // (ld_entry_f32) and the thresholds come from the host (48^3
+  // Laplacian: 10.6 -> 9.1 us a launch).
   constexpr int VW = 16 / sizeof(T);  // elements per 16-byte vector
   constexpr int LT = kBlk + VW;       // padded row of l11t
-  constexpr int NT = apply_threads<T>(), RT = apply_rows<T>();
+  constexpr int NT = kApplyRows, RT = kApplyRows;
   __shared__ __align__(16) T l11t[kBlk][LT];
   __shared__ T xs[kBlk][RT];
   __shared__ double dd[2 * kBlk + 2];
-  __shared__ float ddf[kBlk];  // FP32 copies of the 1x1 D^{-1} entries
-  __shared__ int kind[kBlk];   // 0 1x1, 1 first of a 2x2, 2 second of a 2x2, 3 zero pivot
+  __shared__ float ddh[2 * kBlk], ddl[2 * kBlk];  // D^{-1} as float pairs, hi + lo
+  __shared__ int kind[kBlk];
   __shared__ int lp[kBlk];
   {
     // all loads first (one latency), then the shared-memory stores
-    constexpr int PER = kBlk * kBlk / NT;  // 16 (FP32) or 8 (FP64)
-    double v[PER];
+    constexpr int PER = kBlk * kBlk / NT;
+    T v[PER];
 #pragma unroll
     for (int k = 0; k < PER; ++k) {
       const int i = threadIdx.x + k * NT;
       const int c = i / kBlk, r = i % kBlk;
-      v[k] = (r > c && r < bs && c < bs) ? fd.step[c * kBlk + r] : 0.0;
+      v[k] = (r > c && r < bs && c < bs) ? fd.L[(int64_t)(p + c) * fd.ld + p + r] : T(0);
     }
+    static_assert(NT == 2 * kBlk, "an entry of D^{-1} per thread");
+    const int i = threadIdx.x;
+    const double d = (i < 2 * bs) ? fd.step[kBlk * kBlk + i] : 0.0;
+    dd[i] = d;
+    if (i < 2) dd[2 * kBlk + i] = 0.0;
+    ddh[i] = (float)d;
+    ddl[i] = isinf(d) ? 0.f : (float)(d - (double)ddh[i]);
 #pragma unroll
     for (int k = 0; k < PER; ++k) {
-      const int i = threadIdx.x + k * NT;
-      l11t[i / kBlk][i % kBlk] = (T)v[k];
+      const int e = threadIdx.x + k * NT;
+      l11t[e / kBlk][e % kBlk] = v[k];
     }
   }
-  for (int i = threadIdx.x; i < 2 * kBlk + 2; i += blockDim.x)
-    dd[i] = (i < 2 * bs) ? fd.step[kBlk * kBlk + i] : 0.0;
   __syncthreads();
   if (threadIdx.x < kBlk) {
     const int j = threadIdx.x;
-    ddf[j] = (j < bs) ? (float)dd[2 * j] : 0.f;
     lp[j] = (j < bs) ? fd.lperm[j] : 0;
-    int kd = 0;
-    if (j < bs) {
-      if (isinf(dd[2 * j])) kd = 2;
-      else if (j + 1 < bs && isinf(dd[2 * j + 2])) kd = 1;
-      else if (dd[2 * j] == 0.0) kd = 3;
-    }
-    kind[j] = kd;
+    kind[j] = pivot_kind(dd, j, bs);
   }
   __syncthreads();
-  const double thresh = 1.0 / u;
-  // FP32 guard band of the threshold test (FP32 factors)
-  const float thr_lo = (float)(thresh * (1.0 - 1e-6)), thr_hi = (float)(thresh * (1.0 + 1e-6));
   // |l| > 1/u tested on bit patterns (non-negative doubles order as integers)
   const long long tkey = __double_as_longlong(thresh);
   auto over = [tkey](double l) {  // Inf fails the test, NaN does not (as fabs(l) > 1/u)
@@ -765,130 +828,208 @@ __global__ void __launch_bounds__(apply_threads<T>()) k_app_apply(FrontDesc<T>* 
     return b > tkey && b <= 0x7ff0000000000000LL;
   };
   int myfail = bs;
-  // row of the tile: FP32, thread t; FP64, lane t of each of the 4 warps,
-  // warp w owning columns [8w, 8w+8)
-  const int t = (sizeof(T) == 8) ? (threadIdx.x & 31) : threadIdx.x;
+  const int t = threadIdx.x;  // row of the tile
   for (int tile = blockIdx.x; tile * RT < nrows; tile += napply) {
     const int rr = tile * RT + t;
     const bool valid = rr < nrows;
     const int r = r0 + rr;
-    if constexpr (sizeof(T) == 8) {
-      // FP64: one warp's chain of 496 dependent FMAs per row tile waits on
-      // the FP64 pipe of its SM sub-partition (~75 cycles a warp
-      // instruction), so the columns are split over 4 warps in blocks of 8
-      // and solved block by block: warp b solves its diagonal block, then
-      // the warps right of it subtract block b.  Each x[j] still takes its
-      // terms in the order k = 0, 1, ..., j-1 (the single-warp result, bit
-      // for bit); the critical path is 4 x 28 + 3 x 64 FMAs.
-      constexpr int CB = 8;
-      const int w = threadIdx.x >> 5, c0 = CB * w;
-      T x[CB];
+    T x[kBlk];
 #pragma unroll
-      for (int i = 0; i < CB; ++i)
-        x[i] = (valid && c0 + i < bs) ? fd.L[(int64_t)(p + lp[c0 + i]) * fd.ld + r] : T(0);
-      for (int b = 0; b < kBlk / CB && CB * b < bs; ++b) {
-        if (w == b) {
+    for (int j = 0; j < kBlk; ++j)
+      x[j] = (valid && j < bs) ? fd.L[(int64_t)(p + lp[j]) * fd.ld + r] : T(0);
+    // right-looking: after x[k] is final, the updates of x[k+1..] are
+    // independent FMAs; L(j, k) for j > k comes in 16-byte vectors (the
+    // zero entries on and above the diagonal change nothing)
 #pragma unroll
-          for (int k = 0; k < CB - 1; ++k) {
-            const T xk = x[k];
+    for (int k = 0; k < kBlk - 1; ++k) {
+      if (k + 1 < bs) {
+        const T xk = x[k];
 #pragma unroll
-            for (int i = k + 1; i < CB; ++i) x[i] -= xk * l11t[c0 + k][c0 + i];
-          }
+        for (int j0 = ((k + 1) / VW) * VW; j0 < kBlk; j0 += VW) {
+          T lv[VW];
+          const float4 q = *reinterpret_cast<const float4*>(&l11t[k][j0]);
+          lv[0] = q.x; lv[1] = q.y; lv[2] = q.z; lv[3] = q.w;
 #pragma unroll
-          for (int i = 0; i < CB; ++i) xs[c0 + i][t] = x[i];
-        }
-        __syncthreads();
-        if (w > b) {
-#pragma unroll
-          for (int k = 0; k < CB; ++k) {
-            const T xk = xs[CB * b + k][t];
-#pragma unroll
-            for (int i = 0; i < CB; i += 2) {
-              const double2 q = *reinterpret_cast<const double2*>(&l11t[CB * b + k][c0 + i]);
-              x[i] -= xk * (T)q.x;
-              x[i + 1] -= xk * (T)q.y;
-            }
-          }
+          for (int v = 0; v < VW; ++v)
+            if (j0 + v > k) x[j0 + v] -= xk * lv[v];
         }
       }
-      // blocks past bs were never solved: their columns are not used
-    } else {
-      T x[kBlk];
-#pragma unroll
-      for (int j = 0; j < kBlk; ++j)
-        x[j] = (valid && j < bs) ? fd.L[(int64_t)(p + lp[j]) * fd.ld + r] : T(0);
-      // right-looking: after x[k] is final, the updates of x[k+1..] are
-      // independent FMAs; L(j, k) for j > k comes in 16-byte vectors (the
-      // zero entries on and above the diagonal change nothing)
-#pragma unroll
-      for (int k = 0; k < kBlk - 1; ++k) {
-        if (k + 1 < bs) {
-          const T xk = x[k];
-#pragma unroll
-          for (int j0 = ((k + 1) / VW) * VW; j0 < kBlk; j0 += VW) {
-            T lv[VW];
-            const float4 q = *reinterpret_cast<const float4*>(&l11t[k][j0]);
-            lv[0] = q.x; lv[1] = q.y; lv[2] = q.z; lv[3] = q.w;
-#pragma unroll
-            for (int v = 0; v < VW; ++v)
-              if (j0 + v > k) x[j0 + v] -= xk * lv[v];
-          }
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < kBlk; ++j) xs[j][t] = x[j];  // column t is this thread's
     }
+#pragma unroll
+    for (int j = 0; j < kBlk; ++j) xs[j][t] = x[j];  // column t is this thread's
     if (valid) {
       T* W = fd.W + rr;
-      // FP32: every column of the row; FP64: the warp's 8 columns
-      const int jb = (sizeof(T) == 8) ? 8 * (threadIdx.x >> 5) : 0;
-      const int je = (sizeof(T) == 8) ? min(jb + 8, bs) : bs;
 #pragma unroll 1
-      for (int j = jb; j < je; ++j) {
+      for (int j = 0; j < bs; ++j) {
         const int kd = kind[j];
         if (kd == 2) continue;  // second half of a 2x2: handled with the first
         const T xj = xs[j][t];
         if (kd == 1) {
-          const double dj = dd[2 * j], d21 = dd[2 * j + 1], d22 = dd[2 * j + 3];
-          const double x1 = (double)xj, x2 = (double)xs[j + 1][t];
-          const double l1 = dj * x1 + d21 * x2, l2 = d21 * x1 + d22 * x2;
-          fd.L[(int64_t)(p + j) * fd.ld + r] = (T)l1;
-          fd.L[(int64_t)(p + j + 1) * fd.ld + r] = (T)l2;
-          W[(int64_t)j * fd.ld] = (T)x1;
-          W[(int64_t)(j + 1) * fd.ld] = (T)x2;
-          const int cand = over(l1) ? j : (over(l2) ? j + 1 : bs);
-          myfail = min(myfail, cand);
+          const float x2 = xs[j + 1][t];
+          const float dbh = ddh[2 * j + 1], dbl = ddl[2 * j + 1];
+          const float f1 = ld_entry_f32(ddh[2 * j], ddl[2 * j], dbh, dbl, xj, x2);
+          const float f2 = ld_entry_f32(dbh, dbl, ddh[2 * j + 3], ddl[2 * j + 3], xj, x2);
+          fd.L[(int64_t)(p + j) * fd.ld + r] = f1;
+          fd.L[(int64_t)(p + j + 1) * fd.ld + r] = f2;
+          W[(int64_t)j * fd.ld] = xj;
+          W[(int64_t)(j + 1) * fd.ld] = x2;
+          if (!(fmaxf(fabsf(f1), fabsf(f2)) <= thr_lo)) {  // above the band, in it, or Inf
+            const double dj = dd[2 * j], d21 = dd[2 * j + 1], d22 = dd[2 * j + 3];
+            const double l1 = dj * (double)xj + d21 * (double)x2;
+            const double l2 = d21 * (double)xj + d22 * (double)x2;
+            const int cand = over(l1) ? j : (over(l2) ? j + 1 : bs);
+            myfail = min(myfail, cand);
+          }
         } else if (kd == 3) {
           const double v = (double)xj;
           const double l = (fabs(v) < small) ? 0.0 : dinf() * v;
           fd.L[(int64_t)(p + j) * fd.ld + r] = (T)l;
           W[(int64_t)j * fd.ld] = T(0);
           if (over(l)) myfail = min(myfail, j);
-        } else if (sizeof(T) == 4) {
-          // FP32 factors: L in FP32; the a-posteriori test |l| <= 1/u is
-          // decided in FP32 outside a relative guard band of 1e-6 around
-          // the threshold and in FP64 inside it, so every decision is the
-          // FP64 one
-          const float lf = (float)xj * ddf[j];
+        } else {
+          // L in FP32; the a-posteriori test |l| <= 1/u is decided in FP32
+          // outside a relative guard band of 1e-6 around the threshold and in
+          // FP64 inside it, so every decision is the FP64 one
+          const float lf = (float)xj * ddh[2 * j];
           fd.L[(int64_t)(p + j) * fd.ld + r] = (T)lf;
           W[(int64_t)j * fd.ld] = xj;
           const float al = fabsf(lf);
           if (!(al <= thr_lo)) {  // above the band, in it, or NaN
             if (al > thr_hi || over((double)xj * dd[2 * j])) myfail = min(myfail, j);
           }
-        } else {
-          const double l = (double)xj * dd[2 * j];
-          fd.L[(int64_t)(p + j) * fd.ld + r] = (T)l;
-          W[(int64_t)j * fd.ld] = xj;
-          if (over(l)) myfail = min(myfail, j);
         }
       }
     }
-    if constexpr (sizeof(T) == 8) __syncthreads();  // the next tile rewrites xs
   }
   // block min -> atomicMin
   for (int off = 16; off > 0; off >>= 1) myfail = min(myfail, __shfl_xor_sync(0xffffffffu, myfail, off));
   if ((threadIdx.x & 31) == 0 && myfail < bs) atomicMin(&st->npass_raw, myfail);
+}
+
+// ------------------------------------------------------------------------
+// k_app_apply_f64<RP>: the same for FP64 factors.  A warp's FP64 instruction
+// takes its SM sub-partition about 75 cycles whatever its lanes hold, so the
+// 496 multiply-adds of a row's solve are spread over the lanes: RP rows per
+// warp, 32 / RP lanes per row, lane part pp owning columns pp, pp + PARTS, ...
+// x[k] is broadcast in its row by shuffle and every lane subtracts it from
+// its own later columns: 136 FP64 instructions for 8 rows, 76 for 4 (496 for
+// the 32 rows of a warp with one row per lane).  Each x[j] takes its terms in
+// the order k = 0, 1, ..., j-1.  RP = 4 while the rows do not fill the SMs
+// with the 16 rows of a CTA each, else 8, which needs a tenth fewer
+// instructions in all.  Against one row per lane over four warps: 48^3
+// Laplacian 22.2 -> 15.9 us a launch, saddle point n = 6000 26.3 -> 10.9 us.
+// ------------------------------------------------------------------------
+constexpr int kApplyF64Threads = 128;
+constexpr int kApplySms = 2 * 152;  // CTAs of 16 rows that run at once without slowing each other
+
+template <int RP>
+__global__ void __launch_bounds__(kApplyF64Threads)
+    k_app_apply_f64(FrontDesc<double>* fds, FrontState* sts, const int* fronts, double thresh,
+                    double small, int napply) {
+  constexpr int PARTS = 32 / RP, NI = kBlk / PARTS, NT = kApplyF64Threads;
+  constexpr int RT = NT / 32 * RP;  // rows per CTA
+  const int f = fronts[blockIdx.y];
+  const FrontDesc<double> fd = fds[f];  // written by the host before the launch
+  pdl_wait();
+  pdl_trigger();
+  FrontState* st = &sts[f];
+  const int bs = st->bs;
+  if (bs == 0) return;
+  const int p = st->p;
+  if ((int)blockIdx.x >= napply) {
+    app_permute<double>(fd, p, bs, blockIdx.x - napply, gridDim.x - napply);
+    return;
+  }
+  const int r0 = p + bs;
+  const int nrows = fd.m - r0;
+  if ((int)blockIdx.x * RT >= nrows) return;
+  __shared__ double l11t[kBlk][kBlk + 1];  // l11t[k][j] = L(j, k), j > k
+  __shared__ double xs[NT / 32][kBlk][RP + 1];
+  __shared__ double dd[2 * kBlk + 2];
+  __shared__ int kind[kBlk], lp[kBlk];
+  {
+    // all loads first (one latency), then the shared-memory stores
+    constexpr int PER = kBlk * kBlk / NT;
+    double v[PER];
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+      const int i = threadIdx.x + k * NT;
+      const int c = i / kBlk, r = i % kBlk;
+      v[k] = (r > c && r < bs && c < bs) ? fd.step[c * kBlk + r] : 0.0;
+    }
+    if (threadIdx.x < 2 * kBlk + 2)
+      dd[threadIdx.x] = ((int)threadIdx.x < 2 * bs) ? fd.step[kBlk * kBlk + threadIdx.x] : 0.0;
+    if (threadIdx.x < kBlk) lp[threadIdx.x] = ((int)threadIdx.x < bs) ? fd.lperm[threadIdx.x] : 0;
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+      const int i = threadIdx.x + k * NT;
+      l11t[i / kBlk][i % kBlk] = v[k];
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x < kBlk) kind[threadIdx.x] = pivot_kind(dd, threadIdx.x, bs);
+  __syncthreads();
+  // |l| > 1/u tested on bit patterns (non-negative doubles order as integers)
+  const long long tkey = __double_as_longlong(thresh);
+  auto over = [tkey](double l) {  // Inf fails the test, NaN does not (as fabs(l) > 1/u)
+    const long long b = __double_as_longlong(l) & 0x7fffffffffffffffLL;
+    return b > tkey && b <= 0x7ff0000000000000LL;
+  };
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int row = lane % RP, pp = lane / RP;
+  double (*xw)[RP + 1] = xs[warp];
+  int myfail = bs;
+  for (int tile = blockIdx.x; tile * RT < nrows; tile += napply) {
+    const int rr = tile * RT + warp * RP + row;
+    const bool valid = rr < nrows;
+    double* Lr = fd.L + r0 + rr;
+    double* Wr = fd.W + rr;
+    double x[NI];
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      const int j = pp + PARTS * i;
+      x[i] = (valid && j < bs) ? Lr[(int64_t)(p + lp[j]) * fd.ld] : 0.0;
+    }
+#pragma unroll
+    for (int i0 = 0; i0 < NI; ++i0) {
+      if (PARTS * i0 + 1 < bs) {
+#pragma unroll
+        for (int kk = 0; kk < PARTS; ++kk) {
+          const int k = PARTS * i0 + kk;
+          const double xk = __shfl_sync(0xffffffffu, x[i0], row + RP * kk);
+          if (kk + 1 < PARTS && pp > kk) x[i0] -= xk * l11t[k][pp + PARTS * i0];
+#pragma unroll
+          for (int i = i0 + 1; i < NI; ++i) x[i] -= xk * l11t[k][pp + PARTS * i];
+        }
+      }
+    }
+    __syncwarp();  // the previous tile's xw has been read
+#pragma unroll
+    for (int i = 0; i < NI; ++i) xw[pp + PARTS * i][row] = x[i];
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      const int j = pp + PARTS * i;
+      if (!valid || j >= bs) continue;
+      const int kd = kind[j];
+      double w = x[i], l;
+      if (kd == 0) {
+        l = w * dd[2 * j];
+      } else if (kd == 3) {
+        l = (fabs(w) < small) ? 0.0 : dinf() * w;
+        w = 0.0;
+      } else if (kd == 1) {
+        l = dd[2 * j] * w + dd[2 * j + 1] * xw[j + 1][row];
+      } else {
+        l = dd[2 * j - 1] * xw[j - 1][row] + dd[2 * j + 1] * w;
+      }
+      Lr[(int64_t)(p + j) * fd.ld] = l;
+      Wr[(int64_t)j * fd.ld] = w;
+      if (over(l)) myfail = min(myfail, j);
+    }
+  }
+  for (int off = 16; off > 0; off >>= 1) myfail = min(myfail, __shfl_xor_sync(0xffffffffu, myfail, off));
+  if (lane == 0 && myfail < bs) atomicMin(&st->npass_raw, myfail);
 }
 
 __device__ __forceinline__ int adjust_npass(int np, int bs, int p, const double* D) {
@@ -2325,22 +2466,6 @@ __global__ void __launch_bounds__(kTppThreads) k_tpp_level(FrontDesc<T>* fds, Fr
 // Grid: (row blocks of 128, column chunks of kLdCols, fronts).  Each thread
 // issues the loads of all of its chunk's columns before the first store, so
 // one memory round trip covers kLdCols columns.
-// alpha lv + beta lp for FP32 factors in FP32 instructions, alpha and beta
-// given as float pairs (hi + lo): the two hi products with their exact
-// errors (FMA), their sum with its exact error (two-sum), then the error
-// and lo terms added once, so the result is within an ulp of the FP64
-// expression rounded to FP32, a 2x2 column's cancelling products included
-__device__ __forceinline__ float ld_entry_f32(float ahi, float alo, float bhi, float blo,
-                                              float lv, float lp) {
-  const float p1 = __fmul_rn(ahi, lv), e1 = __fmaf_rn(ahi, lv, -p1);
-  const float p2 = __fmul_rn(bhi, lp), e2 = __fmaf_rn(bhi, lp, -p2);
-  const float sm = __fadd_rn(p1, p2);
-  const float bb = __fsub_rn(sm, p1);
-  const float es = __fadd_rn(__fsub_rn(p1, __fsub_rn(sm, bb)), __fsub_rn(p2, bb));
-  const float corr = __fmaf_rn(alo, lv, __fmaf_rn(blo, lp, __fadd_rn(__fadd_rn(e1, e2), es)));
-  return __fadd_rn(sm, corr);
-}
-
 template <typename T>
 __global__ void __launch_bounds__(128) k_calc_ld(FrontDesc<T>* fds, const FrontState* sts,
                                                  const int* fronts) {
@@ -2507,14 +2632,28 @@ void launch_app_step(FrontDesc<T>* fd, FrontState* st, const int* fronts, int nf
   }
   note_launches(1);
   // apply (+ row permutation of the eliminated part in extra CTAs)
-  const int napply = std::max(1, cdiv(max_rows, apply_rows<T>()));
   const int pcols = step * kBlk;  // upper bound on p
-  const int nperm =
-      pcols > 0 ? std::max(1, std::min(cdiv(pcols, (apply_threads<T>() / 32) * kPermCols), 128))
-                : 0;
+  auto perm_ctas = [&](int threads) {
+    return pcols > 0 ? std::max(1, std::min(cdiv(pcols, (threads / 32) * kPermCols), 128)) : 0;
+  };
+  const double thresh = 1.0 / u;
   pmark(tm, kPhApply, s);
-  launch_pdl(k_app_apply<T>, dim3(napply + nperm, nf), apply_threads<T>(), 0, s, fd, st, fronts,
-             u, small, napply);
+  if constexpr (std::is_same<T, double>::value) {
+    const bool few = (long long)cdiv(max_rows, 16) * nf <= kApplySms;
+    const int napply = std::max(1, cdiv(max_rows, few ? 16 : 32));
+    const dim3 grid(napply + perm_ctas(kApplyF64Threads), nf);
+    if (few)
+      launch_pdl(k_app_apply_f64<4>, grid, kApplyF64Threads, 0, s, fd, st, fronts, thresh,
+                 small, napply);
+    else
+      launch_pdl(k_app_apply_f64<8>, grid, kApplyF64Threads, 0, s, fd, st, fronts, thresh,
+                 small, napply);
+  } else {
+    const int napply = std::max(1, cdiv(max_rows, kApplyRows));
+    launch_pdl(k_app_apply, dim3(napply + perm_ctas(kApplyRows), nf), kApplyRows, 0, s, fd, st,
+               fronts, thresh, (float)(thresh * (1.0 - 1e-6)), (float)(thresh * (1.0 + 1e-6)),
+               small, napply);
+  }
   note_launches(1);
   // trailing update and fixup in one launch (tile estimate assumes no failed
   // columns so far; after failures the trailing region is wider and the
