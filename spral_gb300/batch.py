@@ -179,8 +179,10 @@ class BatchFkeep:
         of each matrix (from the FP64 factors of the matrices the last
         refined solve refactored in FP64)."""
         per_node = self.fk.node_inertia()
-        out = np.zeros((self.bak.nmat, 3), dtype=np.int64)
-        np.add.at(out, self.bak.mat_of_node, per_node)
+        # one bincount per count: np.add.at takes 3.4 ms for 28,000 nodes, as
+        # long as a solve of the whole batch
+        out = np.stack([np.bincount(self.bak.mat_of_node, per_node[:, j], self.bak.nmat)
+                        for j in range(3)], axis=1).astype(np.int64)
         key = tuple(int(i) for i in self.failed)
         if key and key in self._subs and self._subs[key][1] is not None:
             out[list(key)] = self._subs[key][1].inertia()

@@ -1264,8 +1264,8 @@ __device__ __forceinline__ void mma_f16(float (&c)[4], const unsigned (&a)[4],
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
-// sum of eight levels of exact digit products (each |v| <= 2^22) as FP64 * 2^e
-__device__ __forceinline__ double levels_to_double(const float (&v)[8], int e) {
+// eight levels of exact digit products (each |v| <= 2^22) added to H 2^32 + L
+__device__ __forceinline__ void levels_add(const float (&v)[8], long long& H, long long& L) {
   // an integer |i| <= 2^22 plus 1.5 * 2^23 has i in its low mantissa bits; two
   // levels make one 32-bit integer (below 2^30 + 2^22), modulo 2^32 throughout
   int p[4];
@@ -1275,7 +1275,14 @@ __device__ __forceinline__ double levels_to_double(const float (&v)[8], int e) {
     const unsigned i1 = __float_as_uint(v[2 * l + 1] + 12582912.0f);
     p[l] = (int)(i0 * 256u + i1 - 257u * 0x4B400000u);
   }
-  return fixed_to_double((long long)p[0] * 65536 + p[1], (long long)p[2] * 65536 + p[3], e);
+  H += (long long)p[0] * 65536 + p[1];
+  L += (long long)p[2] * 65536 + p[3];
+}
+// their sum as FP64, times 2^e
+__device__ __forceinline__ double levels_to_double(const float (&v)[8], int e) {
+  long long H = 0, L = 0;
+  levels_add(v, H, L);
+  return fixed_to_double(H, L, e);
 }
 
 __global__ void __launch_bounds__(PF_THREADS, 4)
@@ -1714,10 +1721,12 @@ template <typename T>
 struct Thr {
   unsigned long long sk;
   T small, u;
+  float uf;
 };
 template <typename T>
 __device__ __forceinline__ Thr<T> make_thr(double u, double small) {
   Thr<T> t;
+  t.uf = (float)u;
   t.sk = below_key<T>(small);
   if constexpr (sizeof(T) == 4) {
     float f = (float)small;
@@ -1790,6 +1799,42 @@ __device__ void sym_swap(T* S, int ld, int m, int i, int j, int* perm, int* opos
   }
   __syncwarp();
 }
+// the larger magnitude, by integer comparison
+__device__ __forceinline__ double max_mag(double a, double b) {
+  return key_value<double>(max(mag_key(a), mag_key(b)));
+}
+// The verdict of test_pivots for FP64 entries from FP32 copies scaled by the
+// exponent of the largest of the three: 2 (2x2 accepted), 1 (1x1 accepted),
+// 0 (neither) when no FP32 rounding (relative errors of some 1e-6, the
+// determinant's being at most twice its larger product) could decide, else -1.
+__device__ __forceinline__ int pivot_verdict_f32(double a11, double a21, double a22, double maxt,
+                                                 double maxp, const Thr<double>& th) {
+  const double maxpiv = max_mag(a11, max_mag(a21, a22));
+  const int em = (int)((mag_key(maxpiv) >> 52) & 0x7ff);
+  // far above `small`, so that only a nearly vanishing determinant meets it
+  if (em < 64 || em < (int)((mag_key(th.small) >> 52) & 0x7ff) + 80) return -1;
+  if (em == 0x7ff || mag_key(max_mag(maxt, maxp)) >= 0x7ff0000000000000ULL) return -1;
+  const float b11 = scaled_f32(a11, em), b21 = scaled_f32(a21, em), b22 = scaled_f32(a22, em);
+  const float mt = scaled_f32(maxt, em), mp = scaled_f32(maxp, em), u = th.uf;
+  const float ds = __fdividef(1.0f, fmaxf(fabsf(b11), fmaxf(fabsf(b21), fabsf(b22))));
+  const float det0 = (b11 * ds) * b22, det1 = (b21 * ds) * b21, det = det0 - det1;
+  const float big = fmaxf(fabsf(det0), fabsf(det1));
+  const float margin = fabsf(det) - 0.5f * big;
+  if (!(big > 1e-9f)) return -1;
+  if (margin > 1e-4f * big) {
+    const float rd = __fdividef(ds, det);
+    const float d0 = b22 * rd, d1 = b21 * rd, d3 = b11 * rd;
+    const float x1 = fabsf(d0) * mt + fabsf(d1) * mp, x2 = fabsf(d1) * mt + fabsf(d3) * mp;
+    const float g = u * fmaxf(x1, x2);
+    if (g < 0.999f) return mag_key(max_mag(maxt, maxp)) >= th.sk ? 2 : -1;
+    if (!(g > 1.001f)) return -1;
+  } else if (!(margin < -1e-4f * big)) {
+    return -1;
+  }
+  const float need = u * fmaxf(mp, fabsf(b21)), have = fabsf(b22);
+  if (have > 1.0001f * need) return 1;
+  return have < 0.9999f * need ? 0 : -1;
+}
 // The 2x2 test of (t, p) (test_2x2, ldlt_tpp.cxx:95-126), then the 1x1
 // test of p (ldlt_tpp.cxx:216-236): true with d set when p is taken.  FP64
 // factors: FP64 arithmetic as the reference.  FP32 factors: FP32 arithmetic
@@ -1802,28 +1847,35 @@ template <typename T>
 __device__ __forceinline__ bool test_pivots(T a11, T a21, T a22, T maxt, T maxp,
                                             const Thr<T> th, int t, int p, Decision& d) {
   if constexpr (sizeof(T) == 8) {
+    // the verdict in FP32 where that is certain, else in FP64; D^{-1} of an
+    // accepted 2x2 in FP64 (reciprocals by recip_nr, its three entries in
+    // three lanes)
+    const int v = pivot_verdict_f32(a11, a21, a22, maxt, maxp, th);
+    if (v == 0) return false;
+    if (v == 1) { d.kind = kOne; d.p = p; return true; }
     const double u = th.u, small = th.small;
-    const double maxpiv = fmax(fabs(a11), fmax(fabs(a21), fabs(a22)));
-    if (!(maxpiv < small)) {
-      const double detscale = 1 / maxpiv;
-      const double det0 = (a11 * detscale) * a22, det1 = (a21 * detscale) * a21;
-      const double detpiv = det0 - det1;
-      if (!(fabs(detpiv) < fmax(small, fmax(fabs(det0 / 2), fabs(det1 / 2))))) {
-        // the three divisions side by side in lanes 0, 1, 2 (the same
-        // operations, so the same bits, in one division's latency)
-        const int lane = threadIdx.x & 31;
-        const double num = lane == 0 ? a22 * detscale : lane == 1 ? -a21 * detscale : a11 * detscale;
-        const double q = num / detpiv;
+    const double maxpiv = max_mag(a11, max_mag(a21, a22));
+    bool two = v == 2;
+    if (two || !(maxpiv < small)) {
+      const double detscale = recip_nr(maxpiv);
+      const int lane = threadIdx.x & 31;
+      const double x = (lane == 0 ? a22 : lane == 1 ? -a21 : a11) * detscale;
+      const double y = __shfl_sync(0xffffffffu, x, 2), z = __shfl_sync(0xffffffffu, x, 1);
+      const double detpiv = fma(y, a22, z * a21);
+      if (!two) {
+        const double det0 = y * a22, det1 = -z * a21;
+        two = !(fabs(detpiv) < fmax(small, fmax(fabs(det0 / 2), fabs(det1 / 2))));
+      }
+      if (two) {
+        const double q = x * recip_nr(detpiv);
         const double d0 = __shfl_sync(0xffffffffu, q, 0), d1 = __shfl_sync(0xffffffffu, q, 1);
         const double d3 = __shfl_sync(0xffffffffu, q, 2);
-        bool ok;
-        if (fmax(maxp, maxt) < small) ok = true;
-        else {
+        if (v != 2 && !(fmax(maxp, maxt) < small)) {
           const double x1 = fabs(d0) * maxt + fabs(d1) * maxp;
           const double x2 = fabs(d1) * maxt + fabs(d3) * maxp;
-          ok = (u * fmax(x1, x2) < 1.0);
+          two = (u * fmax(x1, x2) < 1.0);
         }
-        if (ok) { d.kind = kTwo; d.t = t; d.p = p; d.d0 = d0; d.d1 = d1; d.d3 = d3; return true; }
+        if (two) { d.kind = kTwo; d.t = t; d.p = p; d.d0 = d0; d.d1 = d1; d.d3 = d3; return true; }
       }
     }
     maxp = fmax(maxp, fabs(a21));
@@ -1863,8 +1915,35 @@ template <typename T>
 __device__ Decision decide(const T* S, int ld, int nel, int m, int n, bool action,
                            const Thr<T> th) {
   Decision d{kStop, 0, 0, 0.0, 0.0, 0.0};
-  if (col_small(S, ld, nel, nel, m, th.sk)) { d.kind = action ? kZeroNel : kSingular; return d; }
-  for (int p = nel + 1; p < n; ++p) {
+  int p0 = nel + 1;
+  if (p0 < n) {
+    // the first candidate: its row part is the entry (p, nel) alone, so t =
+    // nel, and one pass over the two columns gives every maximum
+    const int lane = threadIdx.x & 31, p = p0;
+    const T* cn = S + (size_t)nel * ld;
+    const T* cp = S + (size_t)p * ld;
+    unsigned long long kt = 0, kp = 0;
+    for (int r = p + 1 + lane; r < m; r += 32) {
+      kt = max(kt, mag_key(cn[r]));
+      kp = max(kp, mag_key(cp[r]));
+    }
+    kt = warp_key_max<T>(kt);
+    kp = warp_key_max<T>(kp);
+    const T a11 = cn[nel], a21 = cn[p], a22 = cp[p];
+    const unsigned long long k21 = mag_key(a21);
+    if (max(max(kt, mag_key(a11)), k21) < th.sk) { d.kind = action ? kZeroNel : kSingular; return d; }
+    if (max(max(kp, mag_key(a22)), k21) < th.sk) {
+      d.kind = action ? kZeroSwap : kSingular;
+      d.p = p;
+      return d;
+    }
+    if (test_pivots<T>(a11, a21, a22, key_value<T>(kt), key_value<T>(kp), th, nel, p, d)) return d;
+    ++p0;
+  } else if (col_small(S, ld, nel, nel, m, th.sk)) {
+    d.kind = action ? kZeroNel : kSingular;
+    return d;
+  }
+  for (int p = p0; p < n; ++p) {
     if (col_small(S, ld, p, nel, m, th.sk)) { d.kind = action ? kZeroSwap : kSingular; d.p = p; return d; }
     const int t = row_argmax(S, ld, p, nel);
     const T maxt = rc_max(S, ld, t, nel, m, p);
@@ -2151,7 +2230,7 @@ __device__ int tpp_fast(T* S, int ld, int m, int n, int nel, T* W0, T* W1, int* 
         sym_swap(S, ld, m, d.p, nel, perm, opos);
         const T app = S[(size_t)nel * ld + nel];
         if constexpr (sizeof(T) == 4) d.f0 = 1.0f / app;  // the L column's multiplier
-        else d.d0 = 1.0 / app;
+        else d.d0 = recip_nr(app);
         for (int r = nel + 1 + lane; r < m; r += 32) W0[r] = S[(size_t)nel * ld + r];
         if (lane == 0) {
           S[(size_t)nel * ld + nel] = T(1);
@@ -2268,14 +2347,14 @@ __device__ __forceinline__ void d_column(const double* D, int c, int nel, double
   const double d11 = D[2 * c];
   if (isinf(d11)) {  // second column of a 2x2
     const double a = D[2 * (c - 1)], b = D[2 * (c - 1) + 1], d = D[2 * c + 1];
-    const double det = a * d - b * b;
-    alpha = a / det; beta = -b / det; partner = c - 1;
+    const double rdet = recip_nr(a * d - b * b);
+    alpha = a * rdet; beta = -b * rdet; partner = c - 1;
   } else if (c + 1 < nel && isinf(D[2 * c + 2])) {  // first column of a 2x2
     const double b = D[2 * c + 1], d = D[2 * c + 3];
-    const double det = d11 * d - b * b;
-    alpha = d / det; beta = -b / det; partner = c + 1;
+    const double rdet = recip_nr(d11 * d - b * b);
+    alpha = d * rdet; beta = -b * rdet; partner = c + 1;
   } else {
-    alpha = (d11 != 0.0) ? 1.0 / d11 : 0.0; beta = 0.0; partner = c;
+    alpha = (d11 != 0.0) ? recip_nr(d11) : 0.0; beta = 0.0; partner = c;
   }
 }
 
@@ -2346,20 +2425,9 @@ __device__ void tpp_front_contrib(const FrontDesc<T>& fd, const T* S, int ldS, i
     }
     __syncthreads();  // the coefficients are rewritten by the next chunk
   }
+  if constexpr (sizeof(T) == 8) return;  // C -= L21 LD^T: k_small_contrib_f64
   __syncthreads();  // LD is read back by other threads of this CTA
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  if constexpr (sizeof(T) == 8) {
-    for (int c = warp; c < cm; c += nw) {
-      const T* ldc = LD + c;
-      for (int r = c + lane; r < cm; r += 32) {
-        const T* lrow = S + n + r;
-        T acc = T(0);
-        for (int k = 0; k < nel; ++k) acc += lrow[(size_t)k * ldS] * ldc[(int64_t)k * cm];
-        fd.C[(int64_t)c * fd.ldc + r] -= acc;
-      }
-    }
-    return;
-  }
   const int lr = lane & 7, lc = lane >> 3;
   const int nrt = (cm + 31) / 32, nct = (cm + 15) / 16;
   for (int t = warp; t < nrt * nct; t += nw) {
@@ -2431,9 +2499,21 @@ __global__ void __launch_bounds__(kTppThreads) k_tpp_level(FrontDesc<T>* fds, Fr
       T* W1 = W0 + ldS;
       int* sperm = reinterpret_cast<int*>(W1 + ldS);
       int* sopos = sperm + n;
-      for (int c = 0; c < n; ++c)
-        for (int r = threadIdx.x; r < m; r += blockDim.x)
-          S[(size_t)c * ldS + r] = fd.L[(int64_t)c * fd.ld + r];
+      // eight columns' loads in flight per warp (one at a time the staging
+      // is a chain of memory latencies, as long as the factorisation)
+      {
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+        for (int r = lane; r < m; r += 32)
+          for (int c0 = warp; c0 < n; c0 += 8 * nw) {
+            T v[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+              v[q] = (c0 + q * nw < n) ? fd.L[(int64_t)(c0 + q * nw) * fd.ld + r] : T(0);
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+              if (c0 + q * nw < n) S[(size_t)(c0 + q * nw) * ldS + r] = v[q];
+          }
+      }
       for (int k = threadIdx.x; k < n; k += blockDim.x) { sperm[k] = fd.perm[k]; sopos[k] = fd.opos[k]; }
       __syncthreads();
       nel = tpp_fast(S, ldS, m, n, 0, W0, W1, sperm, sopos, fd.D, action, u, small, nullptr,
@@ -2455,6 +2535,160 @@ __global__ void __launch_bounds__(kTppThreads) k_tpp_level(FrontDesc<T>* fds, Fr
     __syncthreads();  // D and the factor are complete
     if (nel > 0) tpp_front_contrib(fd, F, ldF, nel, ldsm);
     if (raw_d && nel > 0) tpp_finish_d<T>(fd.D, 0, nel);
+  }
+}
+
+// ------------------------------------------------------------------------
+// k_small_contrib_f64: C -= L21 LD^T of the small-subtree fronts of a level
+// for FP64 factors, after k_tpp_level has left L and LD.  A warp forms a
+// 16 x 16 tile of the lower triangle at a time from exact products of FP16
+// digits (slices.cuh, mma.sync m16n8k16), 32 columns at a time: a lane loads
+// the entries that its MMA fragments hold, all at once, and cuts them into
+// digits itself, so nothing passes through shared memory.  Each chunk's exact
+// sum is rounded once and subtracted.  On the FP64 pipe a warp per column of
+// C took some 70,000 cycles of an SM sub-partition for a front of 30 rows and
+// 32 columns.  Bound by the latency of the loads.
+// ------------------------------------------------------------------------
+constexpr int kSmallContribThreads = 128;
+
+// digits of four entries as MMA registers: v[s][0] holds entries 0, 1 of digit
+// s, v[s][1] entries 2, 3 (FP16 pairs)
+__device__ __forceinline__ void slice_quad(const unsigned long long (&b)[4], const int (&h)[4],
+                                           int em, unsigned (&v)[8][2]) {
+  unsigned zl[4], zh[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const unsigned long long Z = slice_digits(b[q], slice_exponent(b[q], h[q]), em);
+    zl[q] = (unsigned)Z;
+    zh[q] = (unsigned)(Z >> 32);
+  }
+#pragma unroll
+  for (int s = 0; s < 8; ++s)
+#pragma unroll
+    for (int w = 0; w < 2; ++w)
+      v[s][w] = slice_pair(s < 4 ? zh[2 * w] : zl[2 * w], s < 4 ? zh[2 * w + 1] : zl[2 * w + 1],
+                           (7 - s) & 3);
+}
+
+constexpr int kSmallBalance = 512;  // balanced columns of a front; later ones keep their scale
+
+__global__ void __launch_bounds__(kSmallContribThreads, 2)
+    k_small_contrib_f64(FrontDesc<double>* fds, const FrontState* sts, const int* fronts) {
+  const int f = fronts[blockIdx.x];
+  const FrontDesc<double> fd = fds[f];
+  const int cm = fd.m - fd.n, nel = sts[f].nelim;
+  if (cm <= 0 || nel <= 0 || sts[f].status != kDevOk) return;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t2 = (lane & 3) * 2;
+  const int nt = (cm + 15) / 16, ntile = nt * (nt + 1) / 2;
+  if ((int)blockIdx.y * (kSmallContribThreads / 32) >= ntile) return;
+  __shared__ short hs[kSmallBalance];
+  for (int k = threadIdx.x; k < min(nel, kSmallBalance); k += kSmallContribThreads)
+    hs[k] = (short)slice_balance(fd.D, k, nel);
+  __syncthreads();
+  const double* A = fd.L + fd.n;
+  const double* B = fd.LD;
+  const int64_t lda = fd.ld;
+  for (int tile = blockIdx.y * (kSmallContribThreads / 32) + warp; tile < ntile;
+       tile += gridDim.y * (kSmallContribThreads / 32)) {
+    int ti = (int)((sqrtf(8.0f * tile + 1.0f) - 1.0f) * 0.5f);
+    while (ti > 0 && ti * (ti + 1) / 2 > tile) --ti;
+    while ((ti + 1) * (ti + 2) / 2 <= tile) ++ti;
+    const int tj = tile - ti * (ti + 1) / 2;
+    const int r0 = 16 * ti + g, c0 = 16 * tj + g;  // this lane's operand rows: r0, r0 + 8, c0, c0 + 8
+    double cv[2][4];  // C, updated chunk by chunk
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        const int rr = r0 + 8 * (x >> 1), cc = 16 * tj + 8 * u + t2 + (x & 1);
+        cv[u][x] = (rr < cm && cc <= rr) ? fd.C[(int64_t)cc * fd.ldc + rr] : 0.0;
+      }
+    for (int k0 = 0; k0 < nel; k0 += 32) {
+      // fragment columns of this lane: k0 + {0, 16} + t2 + {0, 1, 8, 9}
+      unsigned long long a[2][8], b[2][8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const int k = k0 + (q >> 2) * 16 + t2 + (q & 1) + ((q >> 1) & 1) * 8;
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          a[u][q] = (k < nel && r0 + 8 * u < cm)
+                        ? (unsigned long long)__double_as_longlong(A[k * lda + r0 + 8 * u]) : 0ULL;
+          b[u][q] = (k < nel && c0 + 8 * u < cm)
+                        ? (unsigned long long)__double_as_longlong(B[(int64_t)k * cm + c0 + 8 * u]) : 0ULL;
+        }
+      }
+      int h[8], er[2] = {-(1 << 18), -(1 << 18)}, ec[2] = {-(1 << 18), -(1 << 18)};
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const int k = k0 + (q >> 2) * 16 + t2 + (q & 1) + ((q >> 1) & 1) * 8;
+        h[q] = k < min(nel, kSmallBalance) ? hs[k] : 0;
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          if ((a[u][q] << 1) != 0) er[u] = max(er[u], slice_exponent(a[u][q], h[q]));
+          if ((b[u][q] << 1) != 0) ec[u] = max(ec[u], slice_exponent(b[u][q], -h[q]));
+        }
+      }
+      // the quad's four lanes share the columns of a row
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int o = 1; o < 4; o <<= 1) {
+          er[u] = max(er[u], __shfl_xor_sync(0xffffffffu, er[u], o));
+          ec[u] = max(ec[u], __shfl_xor_sync(0xffffffffu, ec[u], o));
+        }
+      float acc[2][8][4];
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int l = 0; l < 8; ++l)
+#pragma unroll
+          for (int x = 0; x < 4; ++x) acc[u][l][x] = 0.f;
+#pragma unroll
+      for (int ks = 0; ks < 2; ++ks) {
+        if (k0 + 16 * ks >= nel) break;
+        unsigned av[2][8][2], bv[8][2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const unsigned long long aq[4] = {a[u][4 * ks], a[u][4 * ks + 1], a[u][4 * ks + 2], a[u][4 * ks + 3]};
+          const int hq[4] = {h[4 * ks], h[4 * ks + 1], h[4 * ks + 2], h[4 * ks + 3]};
+          slice_quad(aq, hq, er[u], av[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const unsigned long long bq[4] = {b[u][4 * ks], b[u][4 * ks + 1], b[u][4 * ks + 2], b[u][4 * ks + 3]};
+          const int hq[4] = {-h[4 * ks], -h[4 * ks + 1], -h[4 * ks + 2], -h[4 * ks + 3]};
+          slice_quad(bq, hq, ec[u], bv);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            // registers of A: (row g, k low), (row g + 8, k low), (g, k high), (g + 8, k high)
+            const unsigned af[4] = {av[0][i][0], av[1][i][0], av[0][i][1], av[1][i][1]};
+#pragma unroll
+            for (int j = 0; j < 8 - i; ++j) mma_f16(acc[u][i + j], af, bv[j]);
+          }
+        }
+      }
+      // columns of an accumulator: t2, t2 + 1 of the tile's half u; their
+      // exponents are held by the lanes whose row index g is that column
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+          const int e2 = __shfl_sync(0xffffffffu, ec[u], (t2 + (x & 1)) * 4);
+          const int e1 = er[x >> 1];
+          const float v[8] = {acc[u][0][x], acc[u][1][x], acc[u][2][x], acc[u][3][x],
+                              acc[u][4][x], acc[u][5][x], acc[u][6][x], acc[u][7][x]};
+          double pr = levels_to_double(v, slice_product_exponent(e1, e2));
+          if (max(e1, e2) >= kSliceNonFinite / 2) pr = dinf() - dinf();
+          cv[u][x] -= pr;
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        const int rr = r0 + 8 * (x >> 1), cc = 16 * tj + 8 * u + t2 + (x & 1);
+        if (rr < cm && cc <= rr) fd.C[(int64_t)cc * fd.ldc + rr] = cv[u][x];
+      }
   }
 }
 
@@ -2723,7 +2957,8 @@ constexpr int kTppSmallSmem = 220 * 1024;
 
 template <typename T>
 void launch_tpp_level(FrontDesc<T>* fd, FrontState* st, const int* fronts, int nf, bool action,
-                      double u, double small, int max_bytes, int threads, cudaStream_t s) {
+                      double u, double small, int max_bytes, int threads, int max_cm,
+                      cudaStream_t s) {
   if (nf <= 0) return;
   static int smem_cap = -1;  // per template instance, once per process
   if (smem_cap < 0) {
@@ -2740,12 +2975,25 @@ void launch_tpp_level(FrontDesc<T>* fd, FrontState* st, const int* fronts, int n
   int dev = 0, nsm = 0, occ = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  // a level of few fronts is bound by one front's chain of pivots, not by
+  // what the fronts of an SM share: four warps, one per sub-partition, for
+  // the trailing updates (@TPPW@)
+  if (nf <= nsm) threads = std::max(threads, 128);
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_tpp_level<T>, threads, smem) !=
       cudaSuccess)
     occ = 1;
   const int grid = std::max(1, std::min(nf, std::max(nsm, 1) * std::max(occ, 1)));
   k_tpp_level<T><<<grid, threads, smem, s>>>(fd, st, fronts, nf, action, u, small, smem);
   note_launches(1);
+  if constexpr (std::is_same<T, double>::value) {
+    // a tile per warp: CTAs (front, group of four tiles)
+    const int nt = cdiv(max_cm, 16);
+    const int gy = std::max(1, std::min(cdiv(nt * (nt + 1) / 2, 4), 1024));
+    if (max_cm > 0) {
+      k_small_contrib_f64<<<dim3(nf, gy), kSmallContribThreads, 0, s>>>(fd, st, fronts);
+      note_launches(1);
+    }
+  }
 }
 
 template <typename T>
@@ -2783,7 +3031,7 @@ void launch_stats(const FrontDesc<T>* fd, const FrontState* st, const int* front
   template void launch_tpp<T>(FrontDesc<T>*, FrontState*, const int*, int, bool, double, double, \
                               bool, cudaStream_t);                                              \
   template void launch_tpp_level<T>(FrontDesc<T>*, FrontState*, const int*, int, bool, double,  \
-                                    double, int, int, cudaStream_t);                            \
+                                    double, int, int, int, cudaStream_t);                       \
   template void launch_calc_ld<T>(FrontDesc<T>*, FrontState*, const int*, int, int, int,        \
                                   cudaStream_t);                                                 \
   template void launch_contrib_gemm<T>(FrontDesc<T>*, FrontState*, const int*, int, int,        \

@@ -1227,12 +1227,15 @@ struct Numeric : NumericBase {
       const int c = cls[k];
       const int o0 = S->tpp_off[(size_t)kTppClasses * l + c];
       const int o1 = S->tpp_off[(size_t)kTppClasses * l + c + 1];
-      int mx = 0;
-      for (int j = o0; j < o1; ++j) mx = std::max(mx, tpp_bytes(S->tpp_list[j]));
+      int mx = 0, mcm = 0;
+      for (int j = o0; j < o1; ++j) {
+        mx = std::max(mx, tpp_bytes(S->tpp_list[j]));
+        mcm = std::max(mcm, cm_of(S->tpp_list[j]));
+      }
       cudaStream_t q = k == 0 ? s : side[k - 1];
       if (k > 0) CK(cudaStreamWaitEvent(q, fork_ev, 0));
       launch_tpp_level<T>(d_fd, d_st, S->d_tpp + o0, o1 - o0, co.action, co.u, co.small,
-                          std::min(mx, tpp_class_smem_cap(c)), tpp_class_threads(c), q);
+                          std::min(mx, tpp_class_smem_cap(c)), tpp_class_threads(c), mcm, q);
       if (k > 0) {
         CK(cudaEventRecord(join_ev[k - 1], q));
         CK(cudaStreamWaitEvent(s, join_ev[k - 1], 0));

@@ -32,6 +32,33 @@ __device__ __forceinline__ int slice_balance(const double* D, int c, int dlast) 
   return (e > 0 && e < 0x7ff) ? (1023 - e) >> 1 : 0;
 }
 
+// The eight balanced digits of an entry (exponent e after the balance, row
+// exponent em) as bytes, biased by 128, the leading digit in the top byte.
+__device__ __forceinline__ unsigned long long slice_digits(unsigned long long bits, int e, int em) {
+  const unsigned hi = (unsigned)(bits >> 32), lo = (unsigned)bits;
+  const unsigned m = (hi & 0xfffffu) | ((hi & 0x7ff00000u) ? 0x100000u : 0u);
+  // |value| 2^62 / 2^(em - 1022), truncated; the mantissa's 53 bits start at
+  // bit 61 for the row's largest exponent.  (A zero's exponent may exceed em;
+  // entries of a row with Inf or NaN have no meaning.)
+  const unsigned long long M =
+      ((unsigned long long)__funnelshift_l(lo, m, 9) << 32) | (unsigned long long)(lo << 9);
+  const unsigned long long X = M >> min(max(em - e, 0), 63);
+  // balanced digits: the bytes of +-X + 0x8080808080808080, minus 128
+  const long long sg = (long long)((int)hi >> 31);
+  return (X ^ (unsigned long long)sg) + (0x8080808080808080ULL - (unsigned long long)sg);
+}
+// byte `byte` of two words as a pair of FP16 digits: 1024 + byte, minus 1152
+__device__ __forceinline__ unsigned slice_pair(unsigned x, unsigned y, int byte) {
+  const unsigned t = __byte_perm(
+      x, y, (unsigned)(byte | (byte << 4) | ((4 + byte) << 8) | ((4 + byte) << 12)));
+  unsigned w;
+  asm("{\n .reg .b32 t;\n lop3.b32 t, %1, 0x00ff00ff, 0x64006400, 0xea;\n"
+      " sub.rn.f16x2 %0, t, %2;\n}\n"
+      : "=r"(w)
+      : "r"(t), "r"(0x64806480u));
+  return w;
+}
+
 // Digits of eight consecutive columns of one row (entries b, exponents e after
 // the balance, row exponent em): slice s (0 the leading digit) goes to the 16
 // bytes at d + s * stride, as eight FP16 values.
@@ -40,35 +67,17 @@ __device__ __forceinline__ void slice_store(const unsigned long long (&b)[8], co
   unsigned zl[8], zh[8];
 #pragma unroll
   for (int q = 0; q < 8; ++q) {
-    const unsigned hi = (unsigned)(b[q] >> 32), lo = (unsigned)b[q];
-    const unsigned m = (hi & 0xfffffu) | ((hi & 0x7ff00000u) ? 0x100000u : 0u);
-    // |value| 2^62 / 2^(em - 1022), truncated; the mantissa's 53 bits start
-    // at bit 61 for the row's largest exponent.  (A zero's exponent may
-    // exceed em; entries of a row with Inf or NaN have no meaning.)
-    const unsigned long long M =
-        ((unsigned long long)__funnelshift_l(lo, m, 9) << 32) | (unsigned long long)(lo << 9);
-    const unsigned long long X = M >> min(max(em - e[q], 0), 63);
-    // balanced digits: the bytes of +-X + 0x8080808080808080, minus 128
-    const long long sg = (long long)((int)hi >> 31);
-    const unsigned long long Z =
-        (X ^ (unsigned long long)sg) + (0x8080808080808080ULL - (unsigned long long)sg);
+    const unsigned long long Z = slice_digits(b[q], e[q], em);
     zl[q] = (unsigned)Z;
     zh[q] = (unsigned)(Z >> 32);
   }
 #pragma unroll
   for (int s = 0; s < 8; ++s) {
-    const int byte = (7 - s) & 3;  // of the upper (s < 4) or lower word
     unsigned w[4];
 #pragma unroll
-    for (int p = 0; p < 4; ++p) {
-      // FP16 1024 + byte for two columns, minus 1152: exact
-      const unsigned t = __byte_perm(s < 4 ? zh[2 * p] : zl[2 * p], s < 4 ? zh[2 * p + 1] : zl[2 * p + 1],
-                                     (unsigned)(byte | (byte << 4) | ((4 + byte) << 8) | ((4 + byte) << 12)));
-      asm("{\n .reg .b32 t;\n lop3.b32 t, %1, 0x00ff00ff, 0x64006400, 0xea;\n"
-          " sub.rn.f16x2 %0, t, %2;\n}\n"
-          : "=r"(w[p])
-          : "r"(t), "r"(0x64806480u));
-    }
+    for (int p = 0; p < 4; ++p)
+      w[p] = slice_pair(s < 4 ? zh[2 * p] : zl[2 * p], s < 4 ? zh[2 * p + 1] : zl[2 * p + 1],
+                        (7 - s) & 3);
     *reinterpret_cast<uint4*>(d + s * stride) = make_uint4(w[0], w[1], w[2], w[3]);
   }
 }

@@ -183,10 +183,12 @@ void launch_tpp(FrontDesc<T>* fd, FrontState* st, const int* fronts, int nf, boo
 // column, then each front's contribution block (LD and C -= L21 LD^T);
 // max_bytes is the dynamic shared memory of the launch (fronts whose
 // staging, ((m + 1) & ~1) * (n + 2) * sizeof(T) + 8 n bytes, exceeds it
-// are factored in place); threads: 32 (one warp per front) or 256
+// are factored in place); threads: 32 (one warp per front) or 256; max_cm:
+// the largest contribution block
 template <typename T>
 void launch_tpp_level(FrontDesc<T>* fd, FrontState* st, const int* fronts, int nf, bool action,
-                      double u, double small, int max_bytes, int threads, cudaStream_t s);
+                      double u, double small, int max_bytes, int threads, int max_cm,
+                      cudaStream_t s);
 template <typename T>
 void launch_calc_ld(FrontDesc<T>* fd, FrontState* st, const int* fronts, int nf, int max_cm,
                     int max_n, cudaStream_t s);
