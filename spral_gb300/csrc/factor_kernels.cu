@@ -1646,6 +1646,11 @@ __global__ void k_app_finish(FrontDesc<T>* fds, FrontState* sts, const int* fron
 // (ldlt_tpp.cxx:166-270).  One CTA per front; FP64 arithmetic.
 // ------------------------------------------------------------------------
 constexpr int kTppThreads = 256;
+// threads of k_tpp on tall FP32 fronts: its one CTA per front scans and updates
+// lines of global memory, bound by their latency (seven fronts of some 7,000
+// rows: 3.0 ms with 256 threads, 0.95 with 1,024; FP64 is bound by the SM's
+// FP64 pipe and gains nothing)
+constexpr int kTppTallThreads = 1024;
 
 
 // ------------------------------------------------------------------------
@@ -1666,10 +1671,12 @@ constexpr int kTppThreads = 256;
 // memory.  step = 0 records that no APP pass ran.
 // ------------------------------------------------------------------------
 namespace tpps {
-enum Kind : int { kStop = 0, kZeroNel, kZeroSwap, kTwo, kOne, kSingular };
+// kTwoRaw: an accepted 2x2 whose D^{-1} is still to be formed (FP64 factors);
+// kMore: the first candidate was not taken
+enum Kind : int { kStop = 0, kZeroNel, kZeroSwap, kTwo, kOne, kSingular, kTwoRaw, kMore };
 struct Decision {
   int kind, t, p;
-  double d0, d1, d3;  // FP64 factors: D^{-1} of the pivot
+  double d0, d1, d3;  // FP64 factors: D^{-1} of the pivot (kTwoRaw: a11, a21, a22)
   float f0, f1, f3;   // FP32 factors: the L columns' multipliers
 };
 
@@ -1803,6 +1810,21 @@ __device__ void sym_swap(T* S, int ld, int m, int i, int j, int* perm, int* opos
 __device__ __forceinline__ double max_mag(double a, double b) {
   return key_value<double>(max(mag_key(a), mag_key(b)));
 }
+// The inverse of a 2x2 pivot as test_2x2 forms it, its three entries in three
+// lanes; det0 - det1 is the scaled determinant.  Warp-wide.
+__device__ __forceinline__ void two_by_two_inverse(double a11, double a21, double a22,
+                                                   double maxpiv, double& d0, double& d1,
+                                                   double& d3, double& det0, double& det1) {
+  const int lane = threadIdx.x & 31;
+  const double x = (lane == 0 ? a22 : lane == 1 ? -a21 : a11) * recip_nr(maxpiv);
+  const double y = __shfl_sync(0xffffffffu, x, 2), z = -__shfl_sync(0xffffffffu, x, 1);
+  det0 = y * a22;
+  det1 = z * a21;
+  const double q = x * recip_nr(fma(y, a22, -det1));
+  d0 = __shfl_sync(0xffffffffu, q, 0);
+  d1 = __shfl_sync(0xffffffffu, q, 1);
+  d3 = __shfl_sync(0xffffffffu, q, 2);
+}
 // The verdict of test_pivots for FP64 entries from FP32 copies scaled by the
 // exponent of the largest of the three: 2 (2x2 accepted), 1 (1x1 accepted),
 // 0 (neither) when no FP32 rounding (relative errors of some 1e-6, the
@@ -1811,8 +1833,9 @@ __device__ __forceinline__ int pivot_verdict_f32(double a11, double a21, double 
                                                  double maxp, const Thr<double>& th) {
   const double maxpiv = max_mag(a11, max_mag(a21, a22));
   const int em = (int)((mag_key(maxpiv) >> 52) & 0x7ff);
-  // far above `small`, so that only a nearly vanishing determinant meets it
-  if (em < 64 || em < (int)((mag_key(th.small) >> 52) & 0x7ff) + 80) return -1;
+  // 2^40 above `small`, so that no determinant accepted below (at least 1e-9
+  // of the largest entry) is under it
+  if (em < 64 || em < (int)((mag_key(th.small) >> 52) & 0x7ff) + 40) return -1;
   if (em == 0x7ff || mag_key(max_mag(maxt, maxp)) >= 0x7ff0000000000000ULL) return -1;
   const float b11 = scaled_f32(a11, em), b21 = scaled_f32(a21, em), b22 = scaled_f32(a22, em);
   const float mt = scaled_f32(maxt, em), mp = scaled_f32(maxp, em), u = th.uf;
@@ -1853,24 +1876,20 @@ __device__ __forceinline__ bool test_pivots(T a11, T a21, T a22, T maxt, T maxp,
     const int v = pivot_verdict_f32(a11, a21, a22, maxt, maxp, th);
     if (v == 0) return false;
     if (v == 1) { d.kind = kOne; d.p = p; return true; }
+    if (v == 2) {
+      // warp 0 forms D^{-1}: every warp of a tall front's search would
+      // queue for the FP64 pipe
+      d.kind = kTwoRaw; d.t = t; d.p = p; d.d0 = a11; d.d1 = a21; d.d3 = a22;
+      return true;
+    }
     const double u = th.u, small = th.small;
     const double maxpiv = max_mag(a11, max_mag(a21, a22));
-    bool two = v == 2;
-    if (two || !(maxpiv < small)) {
-      const double detscale = recip_nr(maxpiv);
-      const int lane = threadIdx.x & 31;
-      const double x = (lane == 0 ? a22 : lane == 1 ? -a21 : a11) * detscale;
-      const double y = __shfl_sync(0xffffffffu, x, 2), z = __shfl_sync(0xffffffffu, x, 1);
-      const double detpiv = fma(y, a22, z * a21);
-      if (!two) {
-        const double det0 = y * a22, det1 = -z * a21;
-        two = !(fabs(detpiv) < fmax(small, fmax(fabs(det0 / 2), fabs(det1 / 2))));
-      }
-      if (two) {
-        const double q = x * recip_nr(detpiv);
-        const double d0 = __shfl_sync(0xffffffffu, q, 0), d1 = __shfl_sync(0xffffffffu, q, 1);
-        const double d3 = __shfl_sync(0xffffffffu, q, 2);
-        if (v != 2 && !(fmax(maxp, maxt) < small)) {
+    if (!(maxpiv < small)) {
+      double d0, d1, d3, det0, det1;
+      two_by_two_inverse(a11, a21, a22, maxpiv, d0, d1, d3, det0, det1);
+      if (!(fabs(det0 - det1) < fmax(small, fmax(fabs(det0 / 2), fabs(det1 / 2))))) {
+        bool two = true;
+        if (!(fmax(maxp, maxt) < small)) {
           const double x1 = fabs(d0) * maxt + fabs(d1) * maxp;
           const double x2 = fabs(d1) * maxt + fabs(d3) * maxp;
           two = (u * fmax(x1, x2) < 1.0);
@@ -1910,40 +1929,50 @@ __device__ __forceinline__ bool test_pivots(T a11, T a21, T a22, T maxt, T maxp,
     return false;
   }
 }
-// the pivot search of one step of ldlt_tpp_factor, in warp 0
+// The search's first candidate p = nel + 1: its row part is the entry (p,
+// nel) alone, so t = nel, and the largest entries kt, kp of columns nel and p
+// below row p decide everything.  kMore: the search goes on.  n == nel + 1:
+// only the smallness of column nel (the caller's all_small).
 template <typename T>
-__device__ Decision decide(const T* S, int ld, int nel, int m, int n, bool action,
-                           const Thr<T> th) {
-  Decision d{kStop, 0, 0, 0.0, 0.0, 0.0};
-  int p0 = nel + 1;
-  if (p0 < n) {
-    // the first candidate: its row part is the entry (p, nel) alone, so t =
-    // nel, and one pass over the two columns gives every maximum
-    const int lane = threadIdx.x & 31, p = p0;
-    const T* cn = S + (size_t)nel * ld;
-    const T* cp = S + (size_t)p * ld;
-    unsigned long long kt = 0, kp = 0;
-    for (int r = p + 1 + lane; r < m; r += 32) {
-      kt = max(kt, mag_key(cn[r]));
-      kp = max(kp, mag_key(cp[r]));
-    }
-    kt = warp_key_max<T>(kt);
-    kp = warp_key_max<T>(kp);
-    const T a11 = cn[nel], a21 = cn[p], a22 = cp[p];
-    const unsigned long long k21 = mag_key(a21);
-    if (max(max(kt, mag_key(a11)), k21) < th.sk) { d.kind = action ? kZeroNel : kSingular; return d; }
-    if (max(max(kp, mag_key(a22)), k21) < th.sk) {
-      d.kind = action ? kZeroSwap : kSingular;
-      d.p = p;
-      return d;
-    }
-    if (test_pivots<T>(a11, a21, a22, key_value<T>(kt), key_value<T>(kp), th, nel, p, d)) return d;
-    ++p0;
-  } else if (col_small(S, ld, nel, nel, m, th.sk)) {
-    d.kind = action ? kZeroNel : kSingular;
+__device__ __forceinline__ Decision first_candidate(const T* S, int ld, int nel,
+                                                    unsigned long long kt, unsigned long long kp,
+                                                    bool action, const Thr<T>& th) {
+  Decision d{kMore, 0, 0, 0.0, 0.0, 0.0};
+  const int p = nel + 1;
+  const T a11 = S[(size_t)nel * ld + nel], a21 = S[(size_t)nel * ld + p], a22 = S[(size_t)p * ld + p];
+  const unsigned long long k21 = mag_key(a21);
+  if (max(max(kt, mag_key(a11)), k21) < th.sk) { d.kind = action ? kZeroNel : kSingular; return d; }
+  if (max(max(kp, mag_key(a22)), k21) < th.sk) {
+    d.kind = action ? kZeroSwap : kSingular;
+    d.p = p;
     return d;
   }
-  for (int p = p0; p < n; ++p) {
+  (void)test_pivots<T>(a11, a21, a22, key_value<T>(kt), key_value<T>(kp), th, nel, p, d);
+  return d;
+}
+// the same by one warp, the two maxima in one pass
+template <typename T>
+__device__ Decision first_candidate_warp(const T* S, int ld, int nel, int m, int n, bool action,
+                                         const Thr<T>& th) {
+  if (nel + 1 >= n) {
+    Decision d{kMore, 0, 0, 0.0, 0.0, 0.0};
+    if (col_small(S, ld, nel, nel, m, th.sk)) d.kind = action ? kZeroNel : kSingular;
+    return d;
+  }
+  const T* cn = S + (size_t)nel * ld;
+  unsigned long long kt = 0, kp = 0;
+  for (int r = nel + 2 + (int)(threadIdx.x & 31); r < m; r += 32) {
+    kt = max(kt, mag_key(cn[r]));
+    kp = max(kp, mag_key(cn[ld + r]));
+  }
+  return first_candidate(S, ld, nel, warp_key_max<T>(kt), warp_key_max<T>(kp), action, th);
+}
+// the other candidates and the last resort, in one warp
+template <typename T>
+__device__ Decision decide_rest(const T* S, int ld, int nel, int m, int n, bool action,
+                                const Thr<T> th) {
+  Decision d{kStop, 0, 0, 0.0, 0.0, 0.0};
+  for (int p = nel + 2; p < n; ++p) {
     if (col_small(S, ld, p, nel, m, th.sk)) { d.kind = action ? kZeroSwap : kSingular; d.p = p; return d; }
     const int t = row_argmax(S, ld, p, nel);
     const T maxt = rc_max(S, ld, t, nel, m, p);
@@ -1961,12 +1990,10 @@ __device__ Decision decide(const T* S, int ld, int nel, int m, int n, bool actio
   }
   return d;
 }
-// ---- the same pivot search with every warp of the CTA (tall fronts) ----
+// ---- the rest of the search with every warp of the CTA ----
 // Per line (row part [nel, idx) then column part [idx, m) of line idx):
 // all |v| < small, the first largest |v| of the row part, and the two
-// largest |v| off the diagonal with their positions; reduced over the CTA
-// in warp order (shuffles, then shared memory), so the result is the same
-// for every thread and every launch shape.
+// largest |v| off the diagonal with their positions.
 // Magnitudes are kept as keys (mag_key); an empty record holds key 0 at
 // position 0x7fffffff, which any entry beats.
 struct LineInfo {
@@ -1996,33 +2023,6 @@ __device__ __forceinline__ LineInfo line_shfl(const LineInfo& a, int o) {
   b.v1 = __shfl_xor_sync(0xffffffffu, a.v1, o); b.i1 = __shfl_xor_sync(0xffffffffu, a.i1, o);
   b.v2 = __shfl_xor_sync(0xffffffffu, a.v2, o); b.i2 = __shfl_xor_sync(0xffffffffu, a.i2, o);
   return b;
-}
-template <typename T>
-__device__ LineInfo line_info(const T* S, int ld, int idx, int nel, int m,
-                              unsigned long long sk, LineInfo* sh) {
-  LineInfo a{1, 0, 0x7fffffff, 0, 0x7fffffff, 0, 0x7fffffff};
-  for (int c = nel + (int)threadIdx.x; c < idx; c += blockDim.x) {
-    const unsigned long long v = mag_key(S[(size_t)c * ld + idx]);
-    a.all_small = a.all_small && (v < sk);
-    if (better(v, c, a.rv, a.ri)) { a.rv = v; a.ri = c; }
-    top2_add(a, v, c);
-  }
-  for (int r = idx + (int)threadIdx.x; r < m; r += blockDim.x) {
-    const unsigned long long v = mag_key(S[(size_t)idx * ld + r]);
-    a.all_small = a.all_small && (v < sk);
-    if (r != idx) top2_add(a, v, r);
-  }
-  for (int o = 1; o < 32; o <<= 1) {
-    const LineInfo b = line_shfl(a, o);
-    line_merge(a, b);
-  }
-  const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  __syncthreads();  // sh may still be read from the previous reduction
-  if ((threadIdx.x & 31) == 0) sh[warp] = a;
-  __syncthreads();
-  LineInfo r = sh[0];
-  for (int w = 1; w < nw; ++w) line_merge(r, sh[w]);
-  return r;
 }
 // the line information of lines [l0, l1) (one warp per line) into
 // out[idx - nel], then a barrier
@@ -2069,53 +2069,58 @@ __device__ bool try_candidate(const T* S, int ld, int p, const LineInfo& lp, con
   return test_pivots<T>(a11, a21, a22, maxt, maxp, th, t, p, d);
 }
 
-// the pivot search of one step of ldlt_tpp_factor with all threads (each
-// gets the same Decision).  The first candidate is tested from two line
-// scans; when it fails and `batch` (>= n - nel line records of global
-// scratch) is given, the information of every remaining line is gathered
-// in one pass, one warp per line, and the other candidates are tested from
-// it: a search that runs through many candidates (failed columns, as in KKT
-// systems) reads each line once instead of twice per candidate.  The
-// records equal line_info's, so the decision is the same either way.
+// The candidates after the first and the last resort with all threads (each
+// gets the same Decision).  The information of every line is gathered in one
+// pass, one warp per line (>= n - nel records of global scratch); then each
+// thread examines a candidate of its own, and the first one that it does not
+// reject for certain is decided as in the serial search.  So a search that
+// runs through many candidates (failed columns, as in KKT systems) reads each
+// line once and takes a few rounds instead of a chain of candidates (saddle
+// points, FP64 n = 6000: 18.1 -> 16.0 ms).
 template <typename T>
 __device__ Decision decide_cta(const T* S, int ld, int nel, int m, int n, bool action,
-                               const Thr<T> th, LineInfo* sh, LineInfo* batch) {
+                               const Thr<T> th, LineInfo* batch, int* s_first) {
   Decision d{kStop, 0, 0, 0.0, 0.0, 0.0};
-  if (line_info(S, ld, nel, nel, m, th.sk, sh).all_small) {
-    d.kind = action ? kZeroNel : kSingular;
-    return d;
-  }
-  int p = nel + 1;
-  if (p < n) {
-    const LineInfo lp = line_info(S, ld, p, nel, m, th.sk, sh);
-    const LineInfo lt = line_info(S, ld, lp.ri, nel, m, th.sk, sh);
-    if (try_candidate(S, ld, p, lp, lt, action, th, d)) return d;
-    ++p;
-  }
-  if (batch != nullptr && p < n) {
-    line_info_batch(S, ld, nel, n, nel, m, th.sk, batch);
-    for (; p < n; ++p) {
-      const LineInfo lp = batch[p - nel];
-      if (try_candidate(S, ld, p, lp, batch[(lp.all_small ? p : lp.ri) - nel], action, th, d))
-        return d;
+  line_info_batch(S, ld, nel, n, nel, m, th.sk, batch);
+  for (int p0 = nel + 2; p0 < n;) {
+    const int i = p0 + (int)threadIdx.x;
+    bool hit = false;
+    if (i < n) {
+      const LineInfo lp = batch[i - nel];
+      hit = lp.all_small;
+      if (!hit) {
+        const int t = lp.ri;
+        const LineInfo lt = batch[t - nel];
+        const T maxp = key_value<T>((lp.i1 == t) ? lp.v2 : lp.v1);
+        const T maxt = key_value<T>((lt.i1 == i) ? lt.v2 : lt.v1);
+        const T a11 = S[(size_t)t * ld + t], a21 = S[(size_t)t * ld + i];
+        const T a22 = S[(size_t)i * ld + i];
+        if constexpr (sizeof(T) == 8) {
+          hit = pivot_verdict_f32(a11, a21, a22, maxt, maxp, th) != 0;
+        } else {
+          Decision q{kStop, 0, 0, 0.0, 0.0, 0.0};
+          hit = test_pivots<T>(a11, a21, a22, maxt, maxp, th, t, i, q);
+        }
+      }
     }
-    const LineInfo ln = batch[0];
-    const T maxp = key_value<T>(ln.v1);
-    if (sizeof(T) == 8 ? fabs((double)S[(size_t)nel * ld + nel]) >= (double)th.u * (double)maxp
-                       : fabsf((float)S[(size_t)nel * ld + nel]) >= (float)th.u * (float)maxp) {
-      d.kind = kOne;
-      d.p = nel;
+    if (threadIdx.x == 0) *s_first = 0x7fffffff;
+    __syncthreads();
+    const unsigned who = __ballot_sync(0xffffffffu, hit);
+    if (who && (threadIdx.x & 31) == 0)
+      atomicMin(s_first, p0 + (int)threadIdx.x + __ffs((int)who) - 1);
+    __syncthreads();
+    const int p = *s_first;
+    __syncthreads();  // s_first is reset by the next round
+    if (p == 0x7fffffff) {
+      p0 += blockDim.x;
+      continue;
     }
-    return d;
+    const LineInfo lp = batch[p - nel];
+    if (try_candidate(S, ld, p, lp, batch[(lp.all_small ? p : lp.ri) - nel], action, th, d))
+      return d;
+    p0 = p + 1;
   }
-  for (; p < n; ++p) {
-    const LineInfo lp = line_info(S, ld, p, nel, m, th.sk, sh);
-    if (lp.all_small) { d.kind = action ? kZeroSwap : kSingular; d.p = p; return d; }
-    const LineInfo lt = line_info(S, ld, lp.ri, nel, m, th.sk, sh);
-    if (try_candidate(S, ld, p, lp, lt, action, th, d)) return d;
-  }
-  const LineInfo ln = line_info(S, ld, nel, nel, m, th.sk, sh);
-  const T maxp = key_value<T>(ln.v1);
+  const T maxp = key_value<T>(batch[0].v1);
   if (sizeof(T) == 8 ? fabs((double)S[(size_t)nel * ld + nel]) >= (double)th.u * (double)maxp
                      : fabsf((float)S[(size_t)nel * ld + nel]) >= (float)th.u * (float)maxp) {
     d.kind = kOne;
@@ -2125,7 +2130,8 @@ __device__ Decision decide_cta(const T* S, int ld, int nel, int m, int n, bool a
 }
 }  // namespace tpps
 
-// rows of a front above which the TPP pivot search uses every warp
+// rows of a front above which the TPP pivot search's first candidate is
+// examined by every warp
 constexpr int kTppWideRows = 1024;
 
 // line records of the batched pivot search: the front's workspace W (ld x 32
@@ -2191,16 +2197,58 @@ __device__ int tpp_fast(T* S, int ld, int m, int n, int nel, T* W0, T* W1, int* 
                         bool finish = true) {
   using namespace tpps;
   __shared__ Decision s_dec;
-  __shared__ LineInfo s_line[kTppThreads / 32];
+  __shared__ unsigned long long s_key[kTppTallThreads / 32][2];
+  __shared__ int s_first;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   const int nel0 = nel;
   const Thr<T> th = make_thr<T>(u, small);
   while (nel < n) {
-    Decision dw;
-    const bool wide = m - nel > kTppWideRows;
-    if (wide) dw = decide_cta(S, ld, nel, m, n, action, th, s_line, batch);
+    // the first candidate: by every warp on a tall front, else by warp 0
+    Decision dw{kMore, 0, 0, 0.0, 0.0, 0.0};
+    const bool wide = m - nel > kTppWideRows && batch != nullptr && nel + 1 < n;
+    if (wide) {
+      const T* cn = S + (size_t)nel * ld;
+      unsigned long long kt = 0, kp = 0;
+      for (int r = nel + 2 + (int)threadIdx.x; r < m; r += blockDim.x) {
+        kt = max(kt, mag_key(cn[r]));
+        kp = max(kp, mag_key(cn[ld + r]));
+      }
+      kt = warp_key_max<T>(kt);
+      kp = warp_key_max<T>(kp);
+      if (lane == 0) { s_key[warp][0] = kt; s_key[warp][1] = kp; }
+      __syncthreads();
+      kt = warp_key_max<T>(lane < nw ? s_key[lane][0] : 0ULL);
+      kp = warp_key_max<T>(lane < nw ? s_key[lane][1] : 0ULL);
+      dw = first_candidate(S, ld, nel, kt, kp, action, th);
+    } else if (batch != nullptr && nw > 1) {
+      if (warp == 0) {
+        dw = first_candidate_warp(S, ld, nel, m, n, action, th);
+        if (lane == 0) s_first = dw.kind;
+      }
+      __syncthreads();
+      if (s_first == kMore) dw.kind = kMore;
+      else if (warp != 0) dw.kind = kStop;  // decided: warp 0 goes on
+    }
+    const bool all = batch != nullptr && nw > 1;
+    if (all && dw.kind == kMore) {
+      __syncthreads();  // s_first is rewritten
+      dw = decide_cta(S, ld, nel, m, n, action, th, batch, &s_first);
+    }
     if (warp == 0) {
-      Decision d = wide ? dw : decide(S, ld, nel, m, n, action, th);
+      Decision d = dw;
+      if (!all) {
+        d = first_candidate_warp(S, ld, nel, m, n, action, th);
+        if (d.kind == kMore) d = decide_rest(S, ld, nel, m, n, action, th);
+      }
+      if constexpr (sizeof(T) == 8) {
+        if (d.kind == kTwoRaw) {
+          double det0, det1;
+          const double a11 = d.d0, a21 = d.d1, a22 = d.d3;
+          two_by_two_inverse(a11, a21, a22, max_mag(a11, max_mag(a21, a22)), d.d0, d.d1, d.d3, det0,
+                             det1);
+          d.kind = kTwo;
+        }
+      }
       if (d.kind == kZeroSwap) sym_swap(S, ld, m, d.p, nel, perm, opos);
       if (d.kind == kZeroNel || d.kind == kZeroSwap) {
         for (int r = nel + lane; r < m; r += 32) S[(size_t)nel * ld + r] = T(0);
@@ -2308,7 +2356,7 @@ __device__ int tpp_fast(T* S, int ld, int m, int n, int nel, T* W0, T* W1, int* 
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kTppThreads) k_tpp(FrontDesc<T>* fds, FrontState* sts,
+__global__ void __launch_bounds__(kTppTallThreads) k_tpp(FrontDesc<T>* fds, FrontState* sts,
                                                      const int* fronts, bool action, double u,
                                                      double small, bool all_fronts) {
   const int f = fronts[blockIdx.x];
@@ -2516,7 +2564,7 @@ __global__ void __launch_bounds__(kTppThreads) k_tpp_level(FrontDesc<T>* fds, Fr
       }
       for (int k = threadIdx.x; k < n; k += blockDim.x) { sperm[k] = fd.perm[k]; sopos[k] = fd.opos[k]; }
       __syncthreads();
-      nel = tpp_fast(S, ldS, m, n, 0, W0, W1, sperm, sopos, fd.D, action, u, small, nullptr,
+      nel = tpp_fast(S, ldS, m, n, 0, W0, W1, sperm, sopos, fd.D, action, u, small, tpp_batch(fd),
                      !raw_d);
       __syncthreads();
       if (nel >= 0) {
@@ -2941,10 +2989,11 @@ void launch_panel_close(FrontDesc<T>* fd, FrontState* st, const int* fronts, int
 }
 
 template <typename T>
-void launch_tpp(FrontDesc<T>* fd, FrontState* st, const int* fronts, int nf, bool action,
-                double u, double small, bool all_fronts, cudaStream_t s) {
+void launch_tpp(FrontDesc<T>* fd, FrontState* st, const int* fronts, int nf, int max_m,
+                bool action, double u, double small, bool all_fronts, cudaStream_t s) {
   if (nf <= 0) return;
-  { k_tpp<T><<<nf, kTppThreads, 0, s>>>(fd, st, fronts, action, u, small, all_fronts); note_launches(1); }
+  const int threads = sizeof(T) == 4 && max_m > kTppWideRows ? kTppTallThreads : kTppThreads;
+  { k_tpp<T><<<nf, threads, 0, s>>>(fd, st, fronts, action, u, small, all_fronts); note_launches(1); }
 }
 
 // Largest dynamic shared memory of k_tpp_small: the fronts of small leaf
@@ -2977,7 +3026,7 @@ void launch_tpp_level(FrontDesc<T>* fd, FrontState* st, const int* fronts, int n
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   // a level of few fronts is bound by one front's chain of pivots, not by
   // what the fronts of an SM share: four warps, one per sub-partition, for
-  // the trailing updates (@TPPW@)
+  // the trailing updates (64 x 64 grid: 1.32 -> 1.24 ms)
   if (nf <= nsm) threads = std::max(threads, 128);
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_tpp_level<T>, threads, smem) !=
       cudaSuccess)
@@ -3028,8 +3077,8 @@ void launch_stats(const FrontDesc<T>* fd, const FrontState* st, const int* front
   template void launch_panel_end<T>(FrontDesc<T>*, FrontState*, const int*, int, int, int,      \
                                     cudaStream_t);                                              \
   template void launch_panel_close<T>(FrontDesc<T>*, FrontState*, const int*, int, cudaStream_t); \
-  template void launch_tpp<T>(FrontDesc<T>*, FrontState*, const int*, int, bool, double, double, \
-                              bool, cudaStream_t);                                              \
+  template void launch_tpp<T>(FrontDesc<T>*, FrontState*, const int*, int, int, bool, double,    \
+                              double, bool, cudaStream_t);                                      \
   template void launch_tpp_level<T>(FrontDesc<T>*, FrontState*, const int*, int, bool, double,  \
                                     double, int, int, int, cudaStream_t);                       \
   template void launch_calc_ld<T>(FrontDesc<T>*, FrontState*, const int*, int, int, int,        \

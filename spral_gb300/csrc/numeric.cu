@@ -312,12 +312,21 @@ struct DevBuf {
 
 // Size classes of the small leaf subtrees' fronts for the level-set kernel
 // (launch_tpp_level): rows <= 32 one warp per front, <= 96 two warps, more
-// 256 threads; a class launch stages fronts up to its cap in shared memory
-// and factors larger ones in place.
-constexpr int kTppClasses = 3;
-inline int tpp_class(int rows) { return rows <= 32 ? 0 : rows <= 96 ? 1 : 2; }
-inline int tpp_class_threads(int c) { return c == 0 ? 32 : c == 1 ? 64 : 256; }
-inline int tpp_class_smem_cap(int c) { return c == 2 ? (100 << 10) : (64 << 10); }
+// 256 threads; within those, by the shared memory that stages an FP64 front.
+// A launch reserves its largest front's staging for every CTA, so one class
+// of 96 rows left 4 CTAs per SM to fronts that need a third of it (a level of
+// 16,336 fronts: 2.6 -> 1.9 ms).  A class launch stages fronts up to its cap in
+// shared memory and factors larger ones in place.
+constexpr int kTppClasses = 6;
+constexpr int kTppSide = 3;  // side streams the classes of a level share
+inline int tpp_class(int rows, int cols) {
+  const int kb = ((rows + 1) & ~1) * (cols + 2) * 8 >> 10;
+  if (rows <= 32) return 0;
+  if (rows <= 96) return kb < 20 ? 1 : kb < 32 ? 2 : 3;
+  return kb < 50 ? 4 : 5;
+}
+inline int tpp_class_threads(int c) { return c == 0 ? 32 : c <= 3 ? 64 : 256; }
+inline int tpp_class_smem_cap(int c) { return c >= 4 ? (100 << 10) : (64 << 10); }
 
 template <typename T>
 static T* upload(const std::vector<T>& v) {
@@ -626,7 +635,7 @@ static Symbolic* build_symbolic(int device, int n, int sa, int en, const int* sp
       S->tpp_off[(size_t)kTppClasses * l + c] = (int)S->tpp_list.size();
       std::vector<int> cls;
       for (int f = S->lvl_start[l]; f < S->lvl_start[l + 1]; ++f)
-        if (S->tpp_only[f] && tpp_class(S->nrow[S->node_of[f]]) == c) cls.push_back(f);
+        if (S->tpp_only[f] && tpp_class(S->nrow[S->node_of[f]], S->ncol[S->node_of[f]]) == c) cls.push_back(f);
       std::stable_sort(cls.begin(), cls.end(), [&](int a, int b) {
         return S->nrow[S->node_of[a]] > S->nrow[S->node_of[b]];
       });
@@ -1217,11 +1226,12 @@ struct Numeric : NumericBase {
   void launch_tpp_levels(int l, cudaStream_t s) {
     const auto& co = S->copts;
     int cls[kTppClasses], nc = 0;
-    for (int c = 0; c < kTppClasses; ++c)
+    for (int c = kTppClasses - 1; c >= 0; --c)
       if (S->tpp_off[(size_t)kTppClasses * l + c + 1] > S->tpp_off[(size_t)kTppClasses * l + c])
         cls[nc++] = c;
     // the classes' fronts are independent: the first class on s, the others
-    // on the side streams, joined back into s
+    // on the side streams, joined back into s; the largest fronts, whose
+    // chains of pivots are the longest, start first
     if (nc > 1) CK(cudaEventRecord(fork_ev, s));
     for (int k = 0; k < nc; ++k) {
       const int c = cls[k];
@@ -1232,14 +1242,14 @@ struct Numeric : NumericBase {
         mx = std::max(mx, tpp_bytes(S->tpp_list[j]));
         mcm = std::max(mcm, cm_of(S->tpp_list[j]));
       }
-      cudaStream_t q = k == 0 ? s : side[k - 1];
-      if (k > 0) CK(cudaStreamWaitEvent(q, fork_ev, 0));
+      cudaStream_t q = k == 0 ? s : side[(k - 1) % kTppSide];
+      if (k > 0 && k <= kTppSide) CK(cudaStreamWaitEvent(q, fork_ev, 0));
       launch_tpp_level<T>(d_fd, d_st, S->d_tpp + o0, o1 - o0, co.action, co.u, co.small,
                           std::min(mx, tpp_class_smem_cap(c)), tpp_class_threads(c), mcm, q);
-      if (k > 0) {
-        CK(cudaEventRecord(join_ev[k - 1], q));
-        CK(cudaStreamWaitEvent(s, join_ev[k - 1], 0));
-      }
+    }
+    for (int k = 0; k < std::min(nc - 1, kTppSide); ++k) {
+      CK(cudaEventRecord(join_ev[k], side[k]));
+      CK(cudaStreamWaitEvent(s, join_ev[k], 0));
     }
   }
 
@@ -1523,7 +1533,7 @@ struct Numeric : NumericBase {
         }
         launch_app_finish<T>(d_fd, d_st, fr, nf, s);
         const bool tpp_all = (co.pivot_method == 3) || (co.failed_pivot_method == 1);
-        launch_tpp<T>(d_fd, d_st, fr, napp, co.action, co.u, co.small, tpp_all, s);
+        launch_tpp<T>(d_fd, d_st, fr, napp, max_m, co.action, co.u, co.small, tpp_all, s);
         if (napp < nf) launch_tpp_levels(l, s);
         launch_calc_ld<T>(d_fd, d_st, fr, napp, max_app_cm, max_app_n, s);
         launch_contrib_gemm<T>(d_fd, d_st, fr, napp, max_app_cm, s);
@@ -1650,8 +1660,8 @@ struct Numeric : NumericBase {
   // side streams and events that let the size-class launches of one level's
   // small-subtree fronts run concurrently (fork from and join back to the
   // handle's stream; captured into the factorisation graph as branches)
-  cudaStream_t side[kTppClasses - 1] = {};
-  cudaEvent_t fork_ev = nullptr, join_ev[kTppClasses - 1] = {};
+  cudaStream_t side[kTppSide] = {};
+  cudaEvent_t fork_ev = nullptr, join_ev[kTppSide] = {};
 
   explicit Numeric(Symbolic* s) : S(s) {
     CK(cudaSetDevice(S->device));
@@ -1916,7 +1926,7 @@ struct Numeric : NumericBase {
       launch_app_finish<T>(d_fd, d_st, fr, nf, s);
       pmark(tm(), kPhTpp, s);
       const bool tpp_all = (co.pivot_method == 3) || (co.failed_pivot_method == 1);
-      launch_tpp<T>(d_fd, d_st, fr, napp, co.action, co.u, co.small, tpp_all, s);
+      launch_tpp<T>(d_fd, d_st, fr, napp, max_m, co.action, co.u, co.small, tpp_all, s);
       if (napp < nf) launch_tpp_levels(l, s);
       pmark(tm(), kPhCalcLd, s);
       launch_calc_ld<T>(d_fd, d_st, fr, napp, max_app_cm, max_app_n, s);

@@ -177,8 +177,8 @@ template <typename T>
 void launch_panel_close(FrontDesc<T>* fd, FrontState* st, const int* fronts, int nf,
                         cudaStream_t s);
 template <typename T>
-void launch_tpp(FrontDesc<T>* fd, FrontState* st, const int* fronts, int nf, bool action,
-                double u, double small, bool root_only_or_all, cudaStream_t s);
+void launch_tpp(FrontDesc<T>* fd, FrontState* st, const int* fronts, int nf, int max_m,
+                bool action, double u, double small, bool root_only_or_all, cudaStream_t s);
 // fronts of small leaf subtrees, one persistent launch: TPP from the first
 // column, then each front's contribution block (LD and C -= L21 LD^T);
 // max_bytes is the dynamic shared memory of the launch (fronts whose
