@@ -1246,45 +1246,6 @@ constexpr int PF_A_SLICE = PF_M * kBlk * 2, PF_B_SLICE = PF_N * kBlk * 2;  // by
 constexpr int kEmptyRow = -(1 << 18);  // exponent of a row of zeros
 constexpr size_t kPanelF64Smem = (size_t)8 * (PF_A_SLICE + PF_B_SLICE);
 
-__device__ __forceinline__ void ldsm_x4(unsigned (&v)[4], const char* p) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
-               : "r"((unsigned)__cvta_generic_to_shared(p)));
-}
-__device__ __forceinline__ void ldsm_x2(unsigned (&v)[2], const char* p) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];"
-               : "=r"(v[0]), "=r"(v[1])
-               : "r"((unsigned)__cvta_generic_to_shared(p)));
-}
-__device__ __forceinline__ void mma_f16(float (&c)[4], const unsigned (&a)[4],
-                                         const unsigned (&b)[2]) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-      "{%0,%1,%2,%3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
-}
-// eight levels of exact digit products (each |v| <= 2^22) added to H 2^32 + L
-__device__ __forceinline__ void levels_add(const float (&v)[8], long long& H, long long& L) {
-  // an integer |i| <= 2^22 plus 1.5 * 2^23 has i in its low mantissa bits; two
-  // levels make one 32-bit integer (below 2^30 + 2^22), modulo 2^32 throughout
-  int p[4];
-#pragma unroll
-  for (int l = 0; l < 4; ++l) {
-    const unsigned i0 = __float_as_uint(v[2 * l] + 12582912.0f);
-    const unsigned i1 = __float_as_uint(v[2 * l + 1] + 12582912.0f);
-    p[l] = (int)(i0 * 256u + i1 - 257u * 0x4B400000u);
-  }
-  H += (long long)p[0] * 65536 + p[1];
-  L += (long long)p[2] * 65536 + p[3];
-}
-// their sum as FP64, times 2^e
-__device__ __forceinline__ double levels_to_double(const float (&v)[8], int e) {
-  long long H = 0, L = 0;
-  levels_add(v, H, L);
-  return fixed_to_double(H, L, e);
-}
-
 __global__ void __launch_bounds__(PF_THREADS, 4)
     k_app_panel_f64(FrontDesc<double>* fds, FrontState* sts, const int* fronts, int ptiles) {
   extern __shared__ __align__(16) char pf_smem[];
@@ -2598,25 +2559,6 @@ __global__ void __launch_bounds__(kTppThreads) k_tpp_level(FrontDesc<T>* fds, Fr
 // 32 columns.  Bound by the latency of the loads.
 // ------------------------------------------------------------------------
 constexpr int kSmallContribThreads = 128;
-
-// digits of four entries as MMA registers: v[s][0] holds entries 0, 1 of digit
-// s, v[s][1] entries 2, 3 (FP16 pairs)
-__device__ __forceinline__ void slice_quad(const unsigned long long (&b)[4], const int (&h)[4],
-                                           int em, unsigned (&v)[8][2]) {
-  unsigned zl[4], zh[4];
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const unsigned long long Z = slice_digits(b[q], slice_exponent(b[q], h[q]), em);
-    zl[q] = (unsigned)Z;
-    zh[q] = (unsigned)(Z >> 32);
-  }
-#pragma unroll
-  for (int s = 0; s < 8; ++s)
-#pragma unroll
-    for (int w = 0; w < 2; ++w)
-      v[s][w] = slice_pair(s < 4 ? zh[2 * w] : zl[2 * w], s < 4 ? zh[2 * w + 1] : zl[2 * w + 1],
-                           (7 - s) & 3);
-}
 
 constexpr int kSmallBalance = 512;  // balanced columns of a front; later ones keep their scale
 

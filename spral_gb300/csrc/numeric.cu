@@ -942,6 +942,13 @@ struct Numeric : NumericBase {
   DevBuf<int2> binv_blocks;
   int wave_nfwd = 0, wave_nbwd = 0;  // items of the forward pass, then of the backward pass
   int wave_nsmall = 0;  // small fronts (one item each per pass)
+  // inverses of the diagonal half blocks of FP64 fronts (all but the small
+  // items'), formed before the first pass with more than two right-hand sides
+  // after a factorisation
+  DevBuf<double> wave_hinv;
+  DevBuf<int2> hinv_blocks;
+  std::vector<int2> hblocks;
+  bool hinv_ready = false, hinv_off = false;  // off: no memory for them
   size_t wave_nflags = 0;
   // optional trace of the wavefront passes (SPRAL_GB300_WAVE_TRACE = path
   // prefix): per item four stamps (taken, last wait over, finished, SM),
@@ -949,7 +956,7 @@ struct Numeric : NumericBase {
   // graphs
   std::string wave_trace;
   DevBuf<unsigned long long> wave_trace_buf;
-  WaveLevel wave_pass(bool fwd) {
+  WaveLevel wave_pass(bool fwd, int q) {
     WaveLevel w;
     w.items = wave_items.p + (fwd ? 0 : wave_nfwd);
     w.nitems = fwd ? wave_nfwd : wave_nbwd;
@@ -957,7 +964,12 @@ struct Numeric : NumericBase {
     w.trace = nullptr;
     // many small-front items: more CTAs in flight; otherwise the widest
     // fronts' chains set the time and keep their registers
-    w.ctas_per_sm = 2 * wave_nsmall > wave_nfwd ? 3 : 2;
+    // (FP64 tensor-core items spill in the registers of three: they keep two
+    // unless they are a few among many small ones.  A 6000-row saddle point,
+    // 4 columns: forward and backward 1.60 ms with two, 1.82 ms with three)
+    w.hinv = q > 2 && hinv_ready ? wave_hinv.p : nullptr;
+    const bool tc = w.hinv && 64 * (long long)hblocks.size() > wave_nsmall;
+    w.ctas_per_sm = 2 * wave_nsmall > wave_nfwd && !tc ? 3 : 2;
     w.front_group = S->d_front_group;
     w.active = S->d_front_group ? group_active.p : nullptr;
     if (!wave_trace.empty()) {
@@ -1020,7 +1032,7 @@ struct Numeric : NumericBase {
   // columns whatever the block, the three slice launches 31 us (one block of
   // 32 .. 1024 rows; 2048 rows: 44 us against 143 us, and 227 us against
   // 4125 us for 1024 columns).
-  bool use_slices = false;
+  bool use_slices = false, use_tc_solve = false;
   int slice_min_cm = 16, slice_min_k = 32;
   DevBuf<char> slice_tab, slice_scratch;
   static constexpr size_t kSliceScratch = size_t(256) << 20;
@@ -1707,7 +1719,7 @@ struct Numeric : NumericBase {
     }
     if (std::is_same<T, double>::value) {
       const char* env = getenv("SPRAL_GB300_TENSOR_CORES");
-      use_slices = !(env && env[0] == '0');
+      use_slices = use_tc_solve = !(env && env[0] == '0');
     }
     if (std::is_same<T, float>::value) {
       const char* env = getenv("SPRAL_GB300_TENSOR_CORES");
@@ -2040,6 +2052,16 @@ struct Numeric : NumericBase {
         CK(cudaMemcpyAsync(binv_blocks.p, bblocks.data(), bblocks.size() * sizeof(int2),
                            cudaMemcpyHostToDevice, stream));
     }
+    hblocks.clear();
+    hinv_ready = false;
+    std::vector<int64_t> hinv_first(nn, -1);
+    if (std::is_same<T, double>::value && use_wave && use_tc_solve) {
+      for (int f = 0; f < nn; ++f) {
+        if (nblk_of(f) < 1 || small_of(f)) continue;
+        hinv_first[f] = (int64_t)hblocks.size();
+        for (int b = 0; b < nblk_of(f); ++b) hblocks.push_back(make_int2(f, b));
+      }
+    }
     wave_nflags = flag_off[nn];
     wave_flags.ensure(std::max<size_t>(wave_nflags, 1));
     wave_ints.ensure(3);
@@ -2103,6 +2125,7 @@ struct Numeric : NumericBase {
       q.flag = wave_flags.p + flag_off[f];
       q.l21p = wave_l21p.p + l21_off[f];
       q.binv = binv ? wave_binv.p + binv_off[f] : nullptr;
+      q.hoff = hinv_first[f];
       q.nblk = nblk_of(f);
       q.ngat = ngat_of(f);
       q.nch = nch_of(f);
@@ -2148,6 +2171,7 @@ struct Numeric : NumericBase {
     mix((uint64_t)(uintptr_t)wave_items.p); mix((uint64_t)(uintptr_t)wave_flags.p);
     mix((uint64_t)(uintptr_t)wave_ints.p); mix((uint64_t)(uintptr_t)wave_l21p.p);
     mix((uint64_t)(uintptr_t)wave_binv.p); mix((uint64_t)binv);
+    mix((uint64_t)hblocks.empty());
     mix((uint64_t)wave_nfwd); mix((uint64_t)wave_nbwd);
     mix((uint64_t)(uintptr_t)S->d_front_group); mix((uint64_t)(uintptr_t)group_active.p);
     if (h != solve_sig) drop_graphs();
@@ -2169,7 +2193,7 @@ struct Numeric : NumericBase {
         CK(cudaMemsetAsync(wave_flags.p, 0, std::max<size_t>(wave_nflags, 1) * sizeof(int), s));
         CK(cudaMemsetAsync(wave_ints.p + 1, 0, sizeof(int), s));
         pmark(tm(), kPhFwdUpdate, s);
-        launch_fwd_tree<T>(d_sn, d_children, S->d_pairs, wave_pass(true), q, xp, ldx, job == 5,
+        launch_fwd_tree<T>(d_sn, d_children, S->d_pairs, wave_pass(true, q), q, xp, ldx, job == 5,
                            wstatus, s);
       } else {
         for (int l = 0; l < S->nlev; ++l) {
@@ -2188,7 +2212,7 @@ struct Numeric : NumericBase {
         CK(cudaMemsetAsync(wave_flags.p, 0, std::max<size_t>(wave_nflags, 1) * sizeof(int), s));
         CK(cudaMemsetAsync(wave_ints.p + 2, 0, sizeof(int), s));
         pmark(tm(), kPhBwdUpdate, s);
-        launch_bwd_tree<T>(d_sn, wave_pass(false), xp, ldx, q, diag_mode, wstatus, s);
+        launch_bwd_tree<T>(d_sn, wave_pass(false, q), xp, ldx, q, diag_mode, wstatus, s);
       } else {
         for (int l = S->nlev - 1; l >= 0; --l) {
           const int f0 = S->lvl_start[l], nf = S->lvl_start[l + 1] - f0;
@@ -2199,8 +2223,35 @@ struct Numeric : NumericBase {
     }
   }
 
+  // the diagonal half blocks' inverses of this factorisation; without memory
+  // for them the passes keep the FP64 multiply-adds
+  void form_half_inverses(cudaStream_t s) {
+    if constexpr (std::is_same<T, double>::value) {
+      if (hinv_ready || hinv_off || hblocks.empty()) return;
+      const double* before = wave_hinv.p;
+      try {
+        wave_hinv.ensure(hblocks.size() * 2 * 32 * 32);
+        hinv_blocks.ensure(hblocks.size());
+      } catch (CudaFail const& e) {
+        if (e.err != cudaErrorMemoryAllocation) throw;
+        cudaGetLastError();
+        if (!wave_hinv.p) wave_hinv.cap = 0;
+        if (!hinv_blocks.p) hinv_blocks.cap = 0;
+        hinv_off = true;
+      }
+      // captured passes hold the table's address, or none
+      if (hinv_off || wave_hinv.p != before) drop_graphs();
+      if (hinv_off) return;
+      CK(cudaMemcpyAsync(hinv_blocks.p, hblocks.data(), hblocks.size() * sizeof(int2),
+                         cudaMemcpyHostToDevice, s));
+      launch_half_inv(d_sn, hinv_blocks.p, (int)hblocks.size(), wave_hinv.p, s);
+      hinv_ready = true;
+    }
+  }
+
   // the same pass through a captured graph (captured on first use)
   void run_solve(int job, int q, double* xp, int ldx, cudaStream_t s) {
+    if (q > 2) form_half_inverses(s);
     if (!wave_trace.empty()) {
       enqueue_solve(job, q, xp, ldx, s);
       dump_wave_trace(s);

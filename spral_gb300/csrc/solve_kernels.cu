@@ -34,6 +34,7 @@
 #include <mutex>
 #include <type_traits>
 
+#include "slices.cuh"
 #include "ssids_gpu.cuh"
 
 namespace ssids300 {
@@ -178,6 +179,41 @@ __device__ __forceinline__ void solve_in_regs(int jb, const T* Lb, T (&x)[R][2])
   }
 }
 
+// ---- FP64 solves of the general items on the tensor cores ----
+// With FP64 factors a 64 x 64 tile of L times 16 right-hand sides is 65,536
+// multiply-adds, 18 us of an SM's FP64 pipe, and a block's substitution takes
+// about as long again on the chain of the pass.  For more than two right-hand
+// sides the tiles of every front that is not one small item are cut into FP16
+// digits (slices.cuh) and multiplied exactly with mma.sync: warp (rt, kh) =
+// (warp % 4, warp / 4) takes 16 rows of a tile and 32 of its 64 columns, whose
+// digits stay in its registers (cut before the item waits for the values);
+// the right-hand sides' digits pass through shared memory.  Each half's sum
+// is rounded once and added to an FP64 accumulator.  The diagonal block is
+// solved as two halves of 32 rows with their inverses (k_half_inv, once per
+// factorisation) and the product between them; those operands' digits are put
+// into shared memory as fragments before the waits too.  One or two columns
+// keep the multiply-adds: the padding to eight columns would cost more.
+// Bound by the chain of pivot blocks at the top of the tree (eight columns:
+// 10 us a block for flag, digits, products of one tile and of the diagonal
+// block; 19 us before) and by the FP64 pipe in the small items below it.  57^3 Laplacian, 16 columns: forward 7.2 -> 3.6 ms, backward 8.5
+// -> 4.0 ms a pass (wide fronts only, from 4 pivot blocks: 4.3 and 5.0; from
+// 2: 3.8 and 4.3).  Six matrices each of five kinds, 16 columns: errors 0.50
+// to 0.95 of the multiply-adds', which round every product.
+template <typename T, int NR>
+constexpr bool solve_mma() { return sizeof(T) == 8 && NR >= 4; }
+template <int NR>
+constexpr int mma_cols() { return (NR + 7) / 8 * 8; }  // right-hand sides, padded
+// shared memory of an item: the diagonal block's fragments (3 operands x 2
+// row tiles x 2 k steps x 8 digits x 512 bytes), row exponents, right-hand
+// side exponents, the block's values, the sums (also the values' digits)
+constexpr int kMmaFragBytes = 3 * 2 * 2 * 8 * 512;
+constexpr int kMmaHeadBytes = kMmaFragBytes + 3 * 32 * 4 + 16 * 4 + 64;
+constexpr int MV = SB + 1;  // stride of the block's values
+template <int NR>
+constexpr size_t mma_smem_bytes() {
+  return kMmaHeadBytes + sizeof(double) * ((size_t)(NR * MV + 1) / 2 * 2 + 2 * mma_cols<NR>() * SB);
+}
+
 // dynamic shared memory of the solve kernels: the staged block, the
 // block's solved values yb[r * NR + q], then the partial sums of the
 // update passes red[(qq * NR + q) * PR + t] (256 NR values for any pass width)
@@ -189,7 +225,8 @@ constexpr size_t solve_smem_bytes() {
 // vector (kWaveSmall items: at most SB + kWaveSmallRows rows)
 template <typename T, int NR>
 constexpr size_t wave_smem_bytes() {
-  return solve_smem_bytes<T, NR>() + sizeof(T) * (size_t)(SB + kWaveSmallRows) * NR;
+  return std::max(solve_smem_bytes<T, NR>() + sizeof(T) * (size_t)(SB + kWaveSmallRows) * NR,
+                  solve_mma<T, NR>() ? mma_smem_bytes<NR>() : 0);
 }
 
 // Solve of diagonal block [j0, j0+jb) inside a block step, after the CTA
@@ -752,6 +789,426 @@ __device__ __forceinline__ void bwd_gather_rows(const SolveNode<T>& sn, const do
   }
 }
 
+struct TileDigits {
+  unsigned d[2][2][8][2];  // [k step][row g or g + 8][digit][register]
+  int e[2];                // row exponents
+};
+// tile entry (r, k) at p[r * rs + k * ks], zero past nr rows or nk columns
+// of the 16 rows from r0 and 32 columns from k0
+__device__ __forceinline__ void tile_digits(const double* p, int64_t rs, int64_t ks, int nr, int nk,
+                                            int r0, int k0, TileDigits& t) {
+  r0 += (threadIdx.x & 31) >> 2;
+  k0 += (threadIdx.x & 3) * 2;
+  unsigned long long v[2][2][4];
+#pragma unroll
+  for (int s = 0; s < 2; ++s)
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int r = r0 + 8 * u, k = k0 + 16 * s + (q & 1) + (q >> 1) * 8;
+        v[s][u][q] = (r < nr && k < nk)
+                         ? (unsigned long long)__double_as_longlong(p[r * rs + k * ks]) : 0ULL;
+      }
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    int e = -(1 << 18);
+#pragma unroll
+    for (int s = 0; s < 2; ++s)
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if ((v[s][u][q] << 1) != 0ULL) e = max(e, slice_exponent(v[s][u][q], 0));
+    e = max(e, __shfl_xor_sync(0xffffffffu, e, 1));
+    e = max(e, __shfl_xor_sync(0xffffffffu, e, 2));
+    t.e[u] = e;
+    const int h[4] = {0, 0, 0, 0};
+#pragma unroll
+    for (int s = 0; s < 2; ++s) slice_quad(v[s][u], h, e, t.d[s][u]);
+  }
+}
+// digits of 64 values of every right-hand side, value k of right-hand side q
+// at p[q * m + k] (another CTA's: read from L2): into yd, exponents into ey.
+// The caller's barriers separate it from the products.
+template <int NR>
+__device__ __forceinline__ void rhs_digits(const double* p, int64_t m, int nk, int nrhs, char* yd,
+                                           int* ey) {
+  constexpr int NP = mma_cols<NR>();
+  static_assert(NP * 8 <= kSolveThreads, "a thread per right-hand side and 8 values");
+  if ((int)threadIdx.x >= NP * 8) return;  // whole warps
+  const int q = threadIdx.x >> 3, o = threadIdx.x & 7;
+  unsigned long long v[8];
+  int e[8], em = -(1 << 18);
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+    v[i] = (q < nrhs && o * 8 + i < nk)
+               ? (unsigned long long)__double_as_longlong(__ldcg(p + q * m + o * 8 + i)) : 0ULL;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    e[i] = slice_exponent(v[i], 0);
+    if ((v[i] << 1) != 0ULL) em = max(em, e[i]);
+  }
+#pragma unroll
+  for (int x = 1; x < 8; x <<= 1) em = max(em, __shfl_xor_sync(0xffffffffu, em, x));
+  if (o == 0) ey[q] = em;
+  slice_store(v, e, em, yd + o * (NP * 16) + q * 16, 8 * NP * 16);
+}
+// acc += tile x right-hand sides: acc[nt][x] is row g + 8 (x / 2) of the warp's
+// 16, right-hand side 8 nt + 2 (lane % 4) + x % 2
+template <int NR>
+__device__ __forceinline__ void tile_product(const TileDigits& t, const char* yd, const int* ey,
+                                             double (&acc)[mma_cols<NR>() / 8][4]) {
+  constexpr int NP = mma_cols<NR>();
+  const int lane = threadIdx.x & 31, kh = threadIdx.x >> 7;
+#pragma unroll
+  for (int nt = 0; nt < NP / 8; ++nt) {
+    float f[8][4];
+#pragma unroll
+    for (int l = 0; l < 8; ++l)
+#pragma unroll
+      for (int x = 0; x < 4; ++x) f[l][x] = 0.f;
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      const char* yp = yd + (kh * 4 + s * 2 + ((lane >> 3) & 1)) * (NP * 16) + (nt * 8 + (lane & 7)) * 16;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        unsigned b[2];
+        ldsm_x2(b, yp + j * (8 * NP * 16));
+#pragma unroll
+        for (int i = 0; i < 8 - j; ++i) {
+          const unsigned a[4] = {t.d[s][0][i][0], t.d[s][1][i][0], t.d[s][0][i][1], t.d[s][1][i][1]};
+          mma_f16(f[i + j], a, b);
+        }
+      }
+    }
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      const float v[8] = {f[0][x], f[1][x], f[2][x], f[3][x], f[4][x], f[5][x], f[6][x], f[7][x]};
+      const int ec = ey[nt * 8 + (lane & 3) * 2 + (x & 1)];
+      double p = levels_to_double(v, slice_product_exponent(t.e[x >> 1], ec));
+      if (max(t.e[x >> 1], ec) >= kSliceNonFinite / 2) p = __longlong_as_double(0x7ff8000000000000LL);
+      acc[nt][x] += p;
+    }
+  }
+}
+// this warp's share of a tile
+__device__ __forceinline__ void tile_digits(const double* p, int64_t rs, int64_t ks, int nr, int nk,
+                                            TileDigits& t) {
+  const int warp = threadIdx.x >> 5;
+  tile_digits(p, rs, ks, nr, nk, (warp & 3) * 16, (warp >> 2) * 32, t);
+}
+// the two column halves' sums into red[half][q][row]
+template <int NR>
+__device__ __forceinline__ void tile_sums(const double (&acc)[mma_cols<NR>() / 8][4], double* red) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int nt = 0; nt < mma_cols<NR>() / 8; ++nt)
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      const int q = nt * 8 + (lane & 3) * 2 + (x & 1);
+      if (q < NR)
+        red[((warp >> 2) * NR + q) * SB + (warp & 3) * 16 + (lane >> 2) + 8 * (x >> 1)] = acc[nt][x];
+    }
+}
+
+template <int NR>
+struct MmaSpace {  // an item's shared memory (kMmaHeadBytes)
+  char* frag;
+  int* fexp;
+  int* ey;
+  double* vb;   // vb[q * MV + row]
+  double* red;
+  char* yd;     // in the sums' space
+  __device__ explicit MmaSpace(void* base) {
+    frag = static_cast<char*>(base);
+    fexp = reinterpret_cast<int*>(frag + kMmaFragBytes);
+    ey = fexp + 96;
+    vb = reinterpret_cast<double*>(frag + kMmaHeadBytes);
+    red = vb + (NR * MV + 1) / 2 * 2;
+    yd = reinterpret_cast<char*>(red);
+  }
+};
+static_assert(kMmaHeadBytes % 16 == 0, "the digits of the values are 16-byte aligned");
+
+// The fragments of the three 32 x 32 operands of a diagonal block's solve
+// (rows and columns [c0, c0 + jb) of L; X: the inverses of its halves):
+// forward X_0, L_10, X_1, backward their transposes from the last.
+template <bool TRANS>
+__device__ __forceinline__ void half_operands(const SolveNode<double>& sn, const double* X, int c0,
+                                              int jb, char* frag, int* fexp) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (warp >= 6) return;
+  const int mat = warp >> 1, rt = warp & 1;
+  TileDigits t;
+  if (mat != 1) {
+    const double* p = X + (((mat == 2) != TRANS) ? 32 * 32 : 0);
+    tile_digits(p, TRANS ? 1 : 32, TRANS ? 32 : 1, 32, 32, rt * 16, 0, t);
+  } else {
+    const double* p = sn.L + (int64_t)c0 * sn.ld + c0 + 32;
+    const int n0 = min(jb, 32), n1 = jb - 32;
+    tile_digits(p, TRANS ? sn.ld : 1, TRANS ? 1 : sn.ld, TRANS ? n0 : n1, TRANS ? n1 : n0, rt * 16,
+                0, t);
+  }
+#pragma unroll
+  for (int s = 0; s < 2; ++s)
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      *reinterpret_cast<uint4*>(frag + ((warp * 2 + s) * 8 + i) * 512 + lane * 16) =
+          make_uint4(t.d[s][0][i][0], t.d[s][1][i][0], t.d[s][0][i][1], t.d[s][1][i][1]);
+  if ((lane & 3) == 0) {
+    fexp[warp * 16 + (lane >> 2)] = t.e[0];
+    fexp[warp * 16 + 8 + (lane >> 2)] = t.e[1];
+  }
+}
+// digits of half h of the block's values
+template <int NR>
+__device__ __forceinline__ void half_digits(const MmaSpace<NR>& sp, int h) {
+  constexpr int NP = mma_cols<NR>();
+  if ((int)threadIdx.x >= NP * 4) return;  // whole warps
+  const int q = threadIdx.x >> 2, o = threadIdx.x & 3;
+  unsigned long long v[8];
+  int e[8], em = -(1 << 18);
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+    v[i] = q < NR ? (unsigned long long)__double_as_longlong(sp.vb[q * MV + h * 32 + o * 8 + i])
+                  : 0ULL;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    e[i] = slice_exponent(v[i], 0);
+    if ((v[i] << 1) != 0ULL) em = max(em, e[i]);
+  }
+  em = max(em, __shfl_xor_sync(0xffffffffu, em, 1));
+  em = max(em, __shfl_xor_sync(0xffffffffu, em, 2));
+  if (o == 0) sp.ey[q] = em;
+  slice_store(v, e, em, sp.yd + o * (NP * 16) + q * 16, 4 * NP * 16);
+}
+// half h of the values = operand mat times the digits (sub: minus it)
+template <int NR>
+__device__ __forceinline__ void half_product(const MmaSpace<NR>& sp, int mat, int h, bool sub) {
+  constexpr int NP = mma_cols<NR>();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rt = warp & 1, nt = warp >> 1;
+  if (nt >= NP / 8) return;
+  float f[8][4];
+#pragma unroll
+  for (int l = 0; l < 8; ++l)
+#pragma unroll
+    for (int x = 0; x < 4; ++x) f[l][x] = 0.f;
+#pragma unroll
+  for (int s = 0; s < 2; ++s) {
+    unsigned b[8][2];
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      ldsm_x2(b[j], sp.yd + j * (4 * NP * 16) + (s * 2 + ((lane >> 3) & 1)) * (NP * 16) +
+                        (nt * 8 + (lane & 7)) * 16);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const uint4 w = *reinterpret_cast<const uint4*>(
+          sp.frag + (((mat * 2 + rt) * 2 + s) * 8 + i) * 512 + lane * 16);
+      const unsigned a[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+      for (int j = 0; j < 8 - i; ++j) mma_f16(f[i + j], a, b[j]);
+    }
+  }
+#pragma unroll
+  for (int x = 0; x < 4; ++x) {
+    const int row = rt * 16 + (lane >> 2) + 8 * (x >> 1), q = nt * 8 + (lane & 3) * 2 + (x & 1);
+    if (q >= NR) continue;
+    const float v[8] = {f[0][x], f[1][x], f[2][x], f[3][x], f[4][x], f[5][x], f[6][x], f[7][x]};
+    const int er = sp.fexp[mat * 32 + row], ec = sp.ey[q];
+    double p = levels_to_double(v, slice_product_exponent(er, ec));
+    if (max(er, ec) >= kSliceNonFinite / 2) p = __longlong_as_double(0x7ff8000000000000LL);
+    double& t = sp.vb[q * MV + h * 32 + row];
+    t = sub ? t - p : p;
+  }
+}
+// the diagonal block's solve, from half `first` (0 forward, 1 backward) on
+template <int NR>
+__device__ __forceinline__ void half_solves(const MmaSpace<NR>& sp, int first) {
+#pragma unroll 1
+  for (int st = 0; st < 3; ++st) {
+    __syncthreads();
+    half_digits<NR>(sp, st == 2 ? 1 - first : first);
+    __syncthreads();
+    half_product<NR>(sp, st, st == 0 ? first : 1 - first, st == 1);
+  }
+  __syncthreads();
+}
+
+// Inverses of the two 32 x 32 unit lower halves on the diagonal of pivot
+// block blocks[i] = (front, block) of the FP64 factors, row-major, into
+// X[hoff + block]; a warp per half, lane c column c by substitution (496
+// FP64 multiply-adds: 20 us, once per factorisation).
+__global__ void __launch_bounds__(64) k_half_inv(const SolveNode<double>* sns, const int2* blocks,
+                                                 double* X) {
+  __shared__ double Ls[2][32][33];
+  const int2 w = blocks[blockIdx.x];
+  const SolveNode<double>& sn = sns[w.x];
+  const int h = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int c0 = w.y * SB + 32 * h, jb = sn.nelim - c0;  // rows left (may be <= 0)
+  for (int c = 0; c < 32; ++c)
+    Ls[h][lane][c] =
+        (lane > c && lane < jb) ? sn.L[(int64_t)(c0 + c) * sn.ld + c0 + lane] : 0.0;
+  __syncwarp();
+  double x[32];
+#pragma unroll
+  for (int i = 0; i < 32; ++i) {
+    double acc = i == lane ? 1.0 : 0.0;
+#pragma unroll
+    for (int k = 0; k < i; ++k) acc -= Ls[h][i][k] * x[k];
+    x[i] = acc;
+  }
+  double* out = X + ((size_t)(sn.hoff + w.y) * 2 + h) * 32 * 32;
+#pragma unroll
+  for (int i = 0; i < 32; ++i) out[i * 32 + lane] = x[i];
+}
+
+// fwd_block on the tensor cores
+template <int NR>
+__device__ bool fwd_block_mma(const SolveNode<double>& sn, int code, int nrhs, double* x, int ldx,
+                              bool scale_sqrt, int* status, void* base, int* s_fail,
+                              const WaveLevel& wl, int it) {
+  constexpr int E = SB * NR / kSolveThreads;
+  const MmaSpace<NR> sp(base);
+  const int tid = threadIdx.x, row = tid % SB, q0 = tid / SB;  // value (row, q0 + 4 k)
+  const int m = sn.m, nelim = sn.nelim;
+  const bool piv = code < kWaveContrib;
+  const int r0 = piv ? code * SB : nelim + (code - kWaveContrib) * SB;
+  const int rows = min(SB, (piv ? nelim : m) - r0);
+  const int ncb = piv ? code : sn.nblk;
+  double own[E];  // the block's gathered values, final before any wait below
+#pragma unroll
+  for (int k = 0; k < E; ++k) {
+    const int q = q0 + 4 * k;
+    own[k] = (row < rows && q < nrhs) ? __ldcg(&sn.xloc[(int64_t)q * m + r0 + row]) : 0.0;
+  }
+  if (piv)
+    half_operands<false>(sn, wl.hinv + (size_t)(sn.hoff + code) * 2 * 32 * 32, r0, rows, sp.frag,
+                         sp.fexp);
+  double acc[mma_cols<NR>() / 8][4] = {};
+  for (int j = 0; j < ncb; ++j) {
+    const int c0 = j * SB, jb = min(SB, nelim - c0);
+    TileDigits td;
+    tile_digits(sn.L + (int64_t)c0 * sn.ld + r0, 1, sn.ld, rows, jb, td);
+    if (!wave_wait(&sn.flag[j], status, s_fail)) return false;
+    rhs_digits<NR>(sn.xloc + c0, m, jb, nrhs, sp.yd, sp.ey);
+    __syncthreads();
+    tile_product<NR>(td, sp.yd, sp.ey, acc);
+    __syncthreads();
+  }
+  wave_stamp(wl, it, 1);
+  tile_sums<NR>(acc, sp.red);
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < E; ++k) {
+    const int q = q0 + 4 * k;
+    own[k] -= sp.red[q * SB + row] + sp.red[(NR + q) * SB + row];
+    if (piv) sp.vb[q * MV + row] = own[k];
+    else if (row < rows && q < nrhs) sn.xloc[(int64_t)q * m + r0 + row] = own[k];
+  }
+  if (!piv) return true;
+  half_solves<NR>(sp, 0);
+#pragma unroll
+  for (int k = 0; k < E; ++k) {
+    const int q = q0 + 4 * k;
+    if (row < rows && q < nrhs) {
+      double v = sp.vb[q * MV + row];
+      sn.xloc[(int64_t)q * m + r0 + row] = v;
+      if (scale_sqrt) v *= sqrt(sn.D[2 * (r0 + row)]);
+      x[(int64_t)q * ldx + sn.perm[r0 + row]] = v;
+    }
+  }
+  __syncthreads();
+  if (tid == 0) st_release(&sn.flag[code], 1);
+  return true;
+}
+
+// bwd_l21_item on the tensor cores
+template <int NR>
+__device__ void bwd_l21_mma(const SolveNode<double>& sn, int t, int nrhs, void* base) {
+  const MmaSpace<NR> sp(base);
+  const int m = sn.m, b = t / sn.nch, c = t - b * sn.nch;
+  const int c0 = b * SB, jb = min(SB, sn.nelim - c0);
+  const int R0 = sn.nelim + c * kWaveL21Rows, nr = min(kWaveL21Rows, m - R0);
+  double acc[mma_cols<NR>() / 8][4] = {};
+  for (int k0 = 0; k0 < nr; k0 += SB) {
+    const int nk = min(SB, nr - k0);
+    TileDigits td;
+    tile_digits(sn.L + (int64_t)c0 * sn.ld + R0 + k0, sn.ld, 1, jb, nk, td);
+    rhs_digits<NR>(sn.xloc + R0 + k0, m, nk, nrhs, sp.yd, sp.ey);
+    __syncthreads();
+    tile_product<NR>(td, sp.yd, sp.ey, acc);
+    __syncthreads();
+  }
+  tile_sums<NR>(acc, sp.red);
+  __syncthreads();
+  double* out = sn.l21p + (size_t)t * SB * kSolveRhs;
+  for (int e = threadIdx.x; e < SB * NR; e += kSolveThreads) {
+    const int q = e % NR, col = e / NR;
+    out[col * kSolveRhs + q] = sp.red[q * SB + col] + sp.red[(NR + q) * SB + col];
+  }
+}
+
+// bwd_block on the tensor cores (such fronts' contribution rows, if any, come
+// as partial items)
+template <int NR>
+__device__ bool bwd_block_mma(const SolveNode<double>& sn, int b, int nrhs, double* x, int ldx,
+                              int* status, void* base, int* s_fail, const WaveLevel& wl, int it) {
+  constexpr int E = SB * NR / kSolveThreads;
+  const MmaSpace<NR> sp(base);
+  const int tid = threadIdx.x, col = tid % SB, q0 = tid / SB;
+  const int m = sn.m, nelim = sn.nelim;
+  const int c0 = b * SB, jb = min(SB, nelim - c0);
+  double own[E];
+#pragma unroll
+  for (int k = 0; k < E; ++k) {
+    const int q = q0 + 4 * k;
+    own[k] = (col < jb && q < nrhs) ? __ldcg(&sn.xloc[(int64_t)q * m + c0 + col]) : 0.0;
+  }
+  half_operands<true>(sn, wl.hinv + (size_t)(sn.hoff + b) * 2 * 32 * 32, c0, jb, sp.frag, sp.fexp);
+  if (sn.nch > 0 && !wave_wait_count(wave_l21done(sn, b), sn.nch, status, s_fail)) return false;
+  const double* pp = sn.l21p + (size_t)b * sn.nch * SB * kSolveRhs;
+  for (int e = tid; e < SB * NR; e += kSolveThreads) {
+    const int q = e % NR, c = e / NR;
+    double v = 0.0;
+    if (q < nrhs)
+      for (int k = 0; k < sn.nch; ++k) v += __ldcg(pp + ((size_t)k * SB + c) * kSolveRhs + q);
+    sp.vb[q * MV + c] = v;
+  }
+  double acc[mma_cols<NR>() / 8][4] = {};
+  for (int j = sn.nblk - 1; j > b; --j) {
+    const int R0 = j * SB, nr = min(SB, nelim - R0);
+    TileDigits td;
+    tile_digits(sn.L + (int64_t)c0 * sn.ld + R0, sn.ld, 1, jb, nr, td);
+    if (!wave_wait(&sn.flag[j], status, s_fail)) return false;
+    rhs_digits<NR>(sn.xloc + R0, m, nr, nrhs, sp.yd, sp.ey);
+    __syncthreads();
+    tile_product<NR>(td, sp.yd, sp.ey, acc);
+    __syncthreads();
+  }
+  wave_stamp(wl, it, 1);
+  tile_sums<NR>(acc, sp.red);
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < E; ++k) {
+    const int q = q0 + 4 * k;
+    double& v = sp.vb[q * MV + col];
+    v = own[k] - (v + sp.red[q * SB + col] + sp.red[(NR + q) * SB + col]);
+  }
+  half_solves<NR>(sp, 1);
+#pragma unroll
+  for (int k = 0; k < E; ++k) {
+    const int q = q0 + 4 * k;
+    if (col < jb && q < nrhs) {
+      const double v = sp.vb[q * MV + col];
+      sn.xloc[(int64_t)q * m + c0 + col] = v;
+      x[(int64_t)q * ldx + sn.perm[c0 + col]] = v;
+    }
+  }
+  __syncthreads();
+  if (tid == 0) st_release(&sn.flag[b], 1);
+  return true;
+}
+
 // Forward block item.  A pivot block b takes x_b -= sum_{j < b} L(b, j) y_j,
 // block by block as the flags of blocks j arrive (thread (r, cq): row r,
 // columns [16 cq, 16 cq + 16) of each 64-column block), adds the four column
@@ -1213,9 +1670,19 @@ __global__ void __launch_bounds__(kSolveThreads, CPS)
       }
     } else {
       ok = wave_wait_count(wave_gathered(sn), sn.ngat, status, &s_fail);
-      if (ok)
-        ok = fwd_block<T, NR>(sn, code, nrhs, x, ldx, scale_sqrt, status, Lb, yb, red, &s_fail,
-                              wl, it);
+      if (ok) {
+        bool done = false;
+        if constexpr (solve_mma<T, NR>()) {
+          if (wl.hinv && sn.hoff >= 0) {
+            ok = fwd_block_mma<NR>(sn, code, nrhs, x, ldx, scale_sqrt, status, solve_smem, &s_fail,
+                                   wl, it);
+            done = true;
+          }
+        }
+        if (!done)
+          ok = fwd_block<T, NR>(sn, code, nrhs, x, ldx, scale_sqrt, status, Lb, yb, red, &s_fail,
+                                wl, it);
+      }
       if (ok) wave_signal(wave_finished(sn), nullptr);
     }
     wave_stamp(wl, it, 2);
@@ -1237,6 +1704,7 @@ __device__ void bwd_l21_item(const SolveNode<T>& sn, int t, int nrhs, T* xs, T* 
   const int c0 = b * SB, jb = min(SB, nelim - c0);
   const int R0 = nelim + c * kWaveL21Rows, nr = min(kWaveL21Rows, m - R0);
   const int tid = threadIdx.x, col = tid % SB, rq = tid / SB;
+  T* out = sn.l21p + (size_t)(b * sn.nch + c) * SB * kSolveRhs;
   for (int e = tid; e < kWaveL21Rows * NR; e += kSolveThreads) {
     const int rr = e % kWaveL21Rows, q = e / kWaveL21Rows;
     xs[rr * NR + q] = (rr < nr && q < nrhs) ? __ldcg(&sn.xloc[(int64_t)q * m + R0 + rr]) : T(0);
@@ -1263,7 +1731,6 @@ __device__ void bwd_l21_item(const SolveNode<T>& sn, int t, int nrhs, T* xs, T* 
 #pragma unroll
   for (int q = 0; q < NR; ++q) red[(rq * NR + q) * SB + col] = acc[q];
   __syncthreads();
-  T* out = sn.l21p + (size_t)(b * sn.nch + c) * SB * kSolveRhs;
   for (int e = tid; e < SB * NR; e += kSolveThreads) {
     const int cc = e % SB, q = e / SB;
     out[cc * kSolveRhs + q] = red[q * SB + cc] + red[(NR + q) * SB + cc] +
@@ -1703,7 +2170,16 @@ __global__ void __launch_bounds__(kSolveThreads, CPS)
       ok = wave_wait_count(wave_gathered(sn), sn.ngat, status, &s_fail);
       if (ok) wave_stamp(wl, it, 1);
       const int t = code - kWaveL21;
-      if (ok) bwd_l21_item<T, NR>(sn, t, nrhs, Lb, red);
+      if (ok) {
+        bool done = false;
+        if constexpr (solve_mma<T, NR>()) {
+          if (wl.hinv && sn.hoff >= 0) {
+            bwd_l21_mma<NR>(sn, t, nrhs, solve_smem);
+            done = true;
+          }
+        }
+        if (!done) bwd_l21_item<T, NR>(sn, t, nrhs, Lb, red);
+      }
       if (ok) wave_signal(wave_l21done(sn, t / sn.nch), wave_finished(sn));
     } else if (code >= kWaveGather) {
       // the rows below the pivots are solved at the ancestors, which are
@@ -1719,7 +2195,17 @@ __global__ void __launch_bounds__(kSolveThreads, CPS)
       wave_signal(wave_gathered(sn), wave_finished(sn));
     } else {
       ok = wave_wait_count(wave_gathered(sn), sn.ngat, status, &s_fail);
-      if (ok) ok = bwd_block<T, NR>(sn, code, nrhs, x, ldx, status, Lb, yb, red, &s_fail, wl, it);
+      if (ok) {
+        bool done = false;
+        if constexpr (solve_mma<T, NR>()) {
+          if (wl.hinv && sn.hoff >= 0) {
+            ok = bwd_block_mma<NR>(sn, code, nrhs, x, ldx, status, solve_smem, &s_fail, wl, it);
+            done = true;
+          }
+        }
+        if (!done)
+          ok = bwd_block<T, NR>(sn, code, nrhs, x, ldx, status, Lb, yb, red, &s_fail, wl, it);
+      }
       if (ok) wave_signal(wave_finished(sn), nullptr);
     }
     wave_stamp(wl, it, 2);
@@ -1912,6 +2398,13 @@ void launch_diag_inv(const SolveNode<T>* sn, const int2* blocks, int nblocks, cu
     k_diag_inv<<<nblocks, SB, 0, s>>>(sn, blocks);
     note_launches(1);
   }
+}
+
+void launch_half_inv(const SolveNode<double>* sn, const int2* blocks, int nblocks, double* X,
+                     cudaStream_t s) {
+  if (nblocks <= 0) return;
+  k_half_inv<<<nblocks, 64, 0, s>>>(sn, blocks, X);
+  note_launches(1);
 }
 
 template <typename T>

@@ -323,6 +323,7 @@ struct SolveNode {
   int nch;           // L21^T partial items per pivot block (0: none)
   int nitf, nitb;    // items of the forward and of the backward pass
   int parent;        // front index of the parent, -1 at a root
+  int64_t hoff;      // first pivot block in WaveLevel::hinv, -1: none
 };
 
 // Wavefront solves: one persistent launch per pass over the whole tree.
@@ -373,6 +374,10 @@ struct WaveLevel {
   // for
   const int* front_group;
   const unsigned char* active;
+  // FP64 factors, more than two right-hand sides: inverses of the two 32 x 32
+  // unit lower halves on the diagonal of the pivot blocks of the fronts that
+  // are not one small item (SolveNode::hoff), [block][half][32][32]; or nullptr
+  const double* hinv;
 };
 
 constexpr int kSolveBlk = 64;   // diagonal block of the blocked triangular solves
@@ -401,6 +406,8 @@ void launch_bwd_tree(const SolveNode<T>* sn, const WaveLevel& wl, double* x, int
                      int diag_mode, int* status, cudaStream_t s);
 // the inverses of the 64 x 64 unit lower diagonal blocks blocks[i] =
 // (front, block) into each front's SolveNode::binv
+void launch_half_inv(const SolveNode<double>* sn, const int2* blocks, int nblocks, double* X,
+                     cudaStream_t s);
 template <typename T>
 void launch_diag_inv(const SolveNode<T>* sn, const int2* blocks, int nblocks, cudaStream_t s);
 // failure-detection probe of the wavefront solves' bounded flag wait

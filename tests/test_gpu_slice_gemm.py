@@ -123,6 +123,47 @@ def test_gpu_fp64_factors_match_simt_and_oracle(kind, monkeypatch):
         assert inf.num_two > 0 and inf.num_delay > 0
 
 
+@pytest.mark.parametrize("nrhs", [3, 4, 8, 9, 16, 21])
+@pytest.mark.parametrize("kind", ["lap3d", "kkt"])
+def test_gpu_fp64_block_solves_match_columns(kind, nrhs):
+    """Three and more right-hand sides at once (tensor-core products in the
+    fronts that are not one small item) against one column at a time (FP64
+    multiply-adds): columns 200 orders of magnitude apart, a zero column and
+    one with a NaN that must stay in its column."""
+    if kind == "kkt":
+        p, r, v = M.kkt(3000, 1500, seed=7)
+        ak = ssids.analyse(p, r, ssids.order_amd(p, r))
+    else:
+        k = 22  # separators of 484, 242, ... columns
+        p, r, v = M.laplacian_3d(k, shift=-0.3)
+        ak = ssids.analyse(p, r, M.nd_order_grid(k, k, k))
+    n = len(p) - 1
+    fk, inf = ssids.factor(ak, v, ssids.Options(precision=ssids.PRECISION_FP64))
+    assert inf.flag == 0
+    b = np.random.default_rng(9).standard_normal((n, nrhs))
+    b[:, 0] *= 1e100
+    b[:, 1] *= 1e-100
+    b[:, 2] = 0.0
+    for job in (0, 1, 3):
+        x = fk.solve(b, job=job)
+        assert np.array_equal(fk.solve(b, job=job), x)
+        assert np.all(x[:, 2] == 0.0)
+        for q in range(nrhs):
+            if q != 2:
+                # rounding differences times a condition number of about 1e3
+                assert _rel(x[:, q], fk.solve(b[:, q], job=job)) < 1e-11
+    x = fk.solve(b)
+    # direct solves: the bound of the reference fixtures (0 / 0 for the zero column)
+    nz = np.arange(nrhs) != 2
+    assert M.scaled_bwd_error(p, r, v, x[:, nz], b[:, nz]).max() <= 5e-14
+    bad = b.copy()
+    bad[n // 2, nrhs - 1] = np.nan
+    y = fk.solve(bad)
+    assert np.isnan(y[:, nrhs - 1]).any()
+    assert np.array_equal(y[:, :nrhs - 1], x[:, :nrhs - 1])
+    fk.free()
+
+
 @pytest.mark.parametrize("m,n", [(33, 33), (64, 40), (65, 64), (97, 65), (129, 96), (160, 33),
                                  (200, 128), (257, 160), (700, 600)])
 def test_gpu_dense_front_reconstructs(m, n):
