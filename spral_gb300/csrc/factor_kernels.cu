@@ -1044,9 +1044,8 @@ __device__ __forceinline__ int adjust_npass(int np, int bs, int p, const double*
 // Fixup of a block step (one of nfix CTAs, index fix): CTA 0 stores npass
 // (Column::adjust, ldlt_app.cxx:112-130); for failed columns the
 // restore-and-update of restore_if_required + update, computed as
-// X_f L_ff^T (rows below, blockDim.x rows per tile) and L_ff D_f L_ff^T
-// (diagonal block, CTA 0).  Failed columns are rare, so this path keeps few
-// registers rather than being fast.
+// X_f L_ff^T (rows below, 32 rows per tile) and L_ff D_f L_ff^T (diagonal
+// block, CTA 0).  FP64 sums for both types; no failed column: a few loads.
 // ------------------------------------------------------------------------
 template <typename T>
 __device__ void app_fixup_cta(const FrontDesc<T>& fd, FrontState* st, int p, int bs, int np,
@@ -1062,14 +1061,23 @@ __device__ void app_fixup_cta(const FrontDesc<T>& fd, FrontState* st, int p, int
   }
   __syncthreads();
   const int r0 = p + bs, nrows = fd.m - r0;
-  // rows below: A(r, p+np+i) = sum_{k<=i} X(r, np+k) * L(np+i, np+k)
-  for (int tile = fix; tile * (int)blockDim.x < nrows; tile += nfix) {
-    const int rr = tile * blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  // rows below: A(r, p+np+i) = sum_{k<=i} X(r, np+k) * L(np+i, np+k), tiles
+  // of 32 rows by all CTAs but the first (a lone CTA does both): the tile's X
+  // in ldf, a lane per row, the columns shared out to the warps.  A thread
+  // per row with every column was 528 FP64 multiply-adds and as many dependent
+  // loads in one thread: 110 us a launch with 32 failed columns
+  const int t0 = nfix > 1 ? fix - 1 : 0, nt = nfix > 1 ? nfix - 1 : 1;
+  for (int tile = t0; tile >= 0 && tile * 32 < nrows; tile += nt) {
+    const int rr = tile * 32 + lane;
+    __syncthreads();  // the previous tile has been read
+    for (int k = warp; k < nf; k += nw)
+      ldf[k][lane] = rr < nrows ? (double)fd.W[(int64_t)(np + k) * fd.ld + rr] : 0.0;
+    __syncthreads();
     if (rr < nrows) {
-      const T* W = fd.W + rr;
-      for (int i = 0; i < nf; ++i) {
+      for (int i = warp; i < nf; i += nw) {
         double s = 0.0;
-        for (int k = 0; k <= i; ++k) s += (double)W[(int64_t)(np + k) * fd.ld] * l11[np + i][np + k];
+        for (int k = 0; k <= i; ++k) s += ldf[k][lane] * l11[np + i][np + k];
         fd.L[(int64_t)(p + np + i) * fd.ld + r0 + rr] = (T)s;
       }
     }
@@ -1077,29 +1085,23 @@ __device__ void app_fixup_cta(const FrontDesc<T>& fd, FrontState* st, int p, int
   if (fix == 0) {
     // diagonal failed block S = L_ff D_f L_ff^T
     const double* d = fd.step + kBlk * kBlk;
-    // LD = L_ff * D_f  (D_f = inverse of stored inverse)
-    for (int i = threadIdx.x; i < nf * nf; i += blockDim.x) {
-      int r = i % nf, c = i / nf;
-      ldf[r][c] = 0.0;
-    }
     __syncthreads();
-    if ((int)threadIdx.x < nf) {
-      int r = threadIdx.x;
-      for (int c = 0; c < nf;) {
-        int cc = np + c;
-        if (c + 1 == nf || isfinite(d[2 * (cc + 1)])) {
-          double d11 = d[2 * cc];
-          if (d11 != 0.0) d11 = 1.0 / d11;
-          ldf[r][c] = d11 * l11[np + r][cc];
-          c += 1;
-        } else {
-          double d11 = d[2 * cc], d21 = d[2 * cc + 1], d22 = d[2 * cc + 3];
-          double det = d11 * d22 - d21 * d21;
-          d11 /= det; d21 /= det; d22 /= det;
+    // LD = L_ff * D_f  (D_f = inverse of stored inverse): a lane per column
+    // or pair of columns, the rows shared out to the warps
+    const int c = lane, cc = np + c;
+    if (c < nf && (c == 0 || isfinite(d[2 * cc]))) {
+      if (c + 1 == nf || isfinite(d[2 * (cc + 1)])) {
+        double d11 = d[2 * cc];
+        if (d11 != 0.0) d11 = 1.0 / d11;
+        for (int r = warp; r < nf; r += nw) ldf[r][c] = d11 * l11[np + r][cc];
+      } else {
+        double d11 = d[2 * cc], d21 = d[2 * cc + 1], d22 = d[2 * cc + 3];
+        double det = d11 * d22 - d21 * d21;
+        d11 /= det; d21 /= det; d22 /= det;
+        for (int r = warp; r < nf; r += nw) {
           double a1 = l11[np + r][cc], a2 = l11[np + r][cc + 1];
           ldf[r][c] = d22 * a1 - d21 * a2;
           ldf[r][c + 1] = -d21 * a1 + d11 * a2;
-          c += 2;
         }
       }
     }
@@ -1108,7 +1110,7 @@ __device__ void app_fixup_cta(const FrontDesc<T>& fd, FrontState* st, int p, int
       int r = i % nf, c = i / nf;
       if (r < c) continue;
       double s = 0.0;
-      for (int k = 0; k < nf; ++k) s += l11[np + r][np + k] * ldf[c][k];
+      for (int k = 0; k <= r; ++k) s += l11[np + r][np + k] * ldf[c][k];
       fd.L[(int64_t)(p + np + c) * fd.ld + p + np + r] = (T)s;
     }
   }
@@ -2882,7 +2884,11 @@ void launch_app_step(FrontDesc<T>* fd, FrontState* st, const int* fronts, int nf
   // trailing update and fixup in one launch (tile estimate assumes no failed
   // columns so far; after failures the trailing region is wider and the
   // kernel's tile loop covers it, so the launch is never skipped)
-  const int nfix = std::max(1, cdiv(max_rows, 256));
+  // fixup CTAs: one per 64 rows up to a CTA per SM in all (without failed
+  // columns they only add to the launch), one per 256 for levels of many
+  // fronts and for positive definite ones, which have no failed columns
+  int nfix = std::max(1, cdiv(max_rows, 256));
+  if (!posdef) nfix = std::max(nfix, std::min(1 + cdiv(max_rows, 64), kApplySms / 2 / nf));
   pmark(tm, kPhPanel, s);
   if constexpr (std::is_same<T, double>::value) {
     panel_f64_init();
