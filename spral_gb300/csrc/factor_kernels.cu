@@ -1240,8 +1240,8 @@ __global__ void __launch_bounds__(256) k_app_panel(FrontDesc<T>* fds, FrontState
 // FP64 subtraction per entry is left.  mma.sync rather than tcgen05: the
 // depth is a single block (32 columns), so a tile's operands are used once
 // and its sums leave the registers directly, without a pass through TMEM.
-// Bound by latency on one front (a tile is one round), by the digit
-// arithmetic when tiles fill the GPU.  48^3 Laplacian: 58 -> 17 us a launch.
+// Bound by latency on a small front (a tile is one round), by the mma.sync
+// rate when the tiles fill the GPU.  48^3 Laplacian: 124 -> 26 us a launch.
 // ------------------------------------------------------------------------
 constexpr int PF_M = 64, PF_N = 32, PF_THREADS = 128;
 constexpr int PF_A_SLICE = PF_M * kBlk * 2, PF_B_SLICE = PF_N * kBlk * 2;  // bytes per digit
@@ -1323,7 +1323,8 @@ __global__ void __launch_bounds__(PF_THREADS, 4)
     const int g = lane >> 2, c2 = (lane & 3) * 2;  // row and column pair of a fragment
     const int ks = K > 16 ? 2 : 1;
     // one column group of 8 at a time: 32 accumulators, so that four CTAs
-    // share an SM (two at a time and two CTAs: 31 us against 22 us a launch)
+    // share an SM (two at a time and two CTAs: 31 us against 24 us at
+    // 3,400 rows)
 #pragma unroll 1
     for (int nt = 0; nt < PF_N / 8; ++nt) {
       float acc[8][4];

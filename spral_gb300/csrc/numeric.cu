@@ -1028,10 +1028,10 @@ struct Numeric : NumericBase {
   DevBuf<int> panel_list;   // fronts ending a panel (eager mode)
   // FP64 factors: contribution blocks from exact FP16 slice products on the
   // tensor cores (slice_gemm.cu).  From slice_min_k pivots on they beat the
-  // SIMT kernel at every block size: a 64 x 64 SIMT tile takes 39 us for 32
-  // columns whatever the block, the three slice launches 31 us (one block of
-  // 32 .. 1024 rows; 2048 rows: 44 us against 143 us, and 227 us against
-  // 4125 us for 1024 columns).
+  // SIMT kernel at every block size: a 64 x 64 SIMT tile takes 41 us for 32
+  // columns whatever the block, the three slice launches 23 us (one block of
+  // up to 1024 rows; 2048 rows: 32 us against 143 us, and 242 us against
+  // 4128 us for 1024 columns).
   bool use_slices = false, use_tc_solve = false;
   int slice_min_cm = 16, slice_min_k = 32;
   DevBuf<char> slice_tab, slice_scratch;

