@@ -884,7 +884,7 @@ __global__ void __launch_bounds__(kApplyRows) k_app_apply(FrontDesc<float>* fds,
           const double v = (double)xj;
           const double l = (fabs(v) < small) ? 0.0 : dinf() * v;
           fd.L[(int64_t)(p + j) * fd.ld + r] = (T)l;
-          W[(int64_t)j * fd.ld] = T(0);
+          W[(int64_t)j * fd.ld] = xj;  // a failed column is restored from it
           if (over(l)) myfail = min(myfail, j);
         } else {
           // L in FP32; the a-posteriori test |l| <= 1/u is decided in FP32
@@ -1016,8 +1016,7 @@ __global__ void __launch_bounds__(kApplyF64Threads)
       if (kd == 0) {
         l = w * dd[2 * j];
       } else if (kd == 3) {
-        l = (fabs(w) < small) ? 0.0 : dinf() * w;
-        w = 0.0;
+        l = (fabs(w) < small) ? 0.0 : dinf() * w;  // W: a failed column is restored from it
       } else if (kd == 1) {
         l = dd[2 * j] * w + dd[2 * j + 1] * xw[j + 1][row];
       } else {
