@@ -43,6 +43,23 @@ namespace {
 
 constexpr int SB = kSolveBlk;
 
+// The child whose delayed columns hold entry k of a front's delay block: the
+// offsets doff rise in child order, so it is the last child with doff <= k
+// (children after it start past its columns).  Binary search: a front of a
+// saddle point can have hundreds of children.
+template <typename T>
+__device__ __forceinline__ const SolveNode<T>& delay_child(const SolveNode<T>& sn,
+                                                           const SolveNode<T>* sns,
+                                                           const int* children, int k) {
+  int lo = sn.child_beg, hi = sn.child_end;  // doff(lo) <= k < doff(hi)
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (sns[children[mid]].doff <= k) lo = mid;
+    else hi = mid;
+  }
+  return sns[children[lo]];
+}
+
 // Value of assembly-order position pos of a node's local vector for
 // right-hand side q: b for the node's own pivots, the delayed entry of the
 // child that delayed it, and the contribution rows that the children map to
@@ -64,13 +81,8 @@ __device__ __forceinline__ T gather_value(const SolveNode<T>& sn, const SolveNod
     P = pos;
   } else if (pos < sn.ncol + sn.ndelay_in) {
     const int k = pos - sn.ncol;
-    for (int ci = sn.child_beg; ci < sn.child_end; ++ci) {
-      const SolveNode<T>& cn = sns[children[ci]];
-      const int nd = cn.n - cn.nelim;
-      if (k >= cn.doff && k < cn.doff + nd)
-        return ld(&cn.xloc[(int64_t)q * cn.m + cn.nelim + (k - cn.doff)]);
-    }
-    return v;
+    const SolveNode<T>& cn = delay_child(sn, sns, children, k);
+    return ld(&cn.xloc[(int64_t)q * cn.m + cn.nelim + (k - cn.doff)]);
   } else {
     P = pos - sn.ndelay_in;
   }
@@ -691,6 +703,26 @@ template <typename T>
 __device__ __forceinline__ int* wave_finished(const SolveNode<T>& sn) {
   return sn.flag + 2 * sn.nblk + 1;
 }
+// Wait until every child of a front has finished all its items, a thread per
+// child (their acquires ordered before the other threads' loads by the
+// barrier).  One after the other cost a poll and a barrier per child: saddle
+// point n = 15,000 (root with hundreds of children), forward pass 1.42 ->
+// 0.61 ms.
+template <typename T>
+__device__ bool wave_wait_children(const SolveNode<T>& sn, const SolveNode<T>* sns,
+                                   const int* children, int* status) {
+  bool ok = true;
+  for (int ci = sn.child_beg + threadIdx.x; ci < sn.child_end && ok; ci += blockDim.x) {
+    const SolveNode<T>& cn = sns[children[ci]];
+    const int* ctr = wave_finished(cn);
+    for (long long it = 0; ld_acquire(ctr) < cn.nitf; ++it) {
+      if (it >= kWaveSpinLimit || *(volatile int*)status != 0) { ok = false; break; }
+      __nanosleep(20);
+    }
+  }
+  if (!ok) atomicExch(status, 1);
+  return __syncthreads_and(ok);
+}
 
 // Forward gather of rows [r0, r1) of a front's local vector, one row per
 // thread with every right-hand side (the row's index lookups once, its
@@ -714,17 +746,11 @@ __device__ __forceinline__ void fwd_gather_rows(const SolveNode<T>& sn, const So
       P = pos;
     } else if (pos < sn.ncol + sn.ndelay_in) {
       const int k = pos - sn.ncol;
-      for (int ci = sn.child_beg; ci < sn.child_end; ++ci) {
-        const SolveNode<T>& cn = sns[children[ci]];
-        const int nd = cn.n - cn.nelim;
-        if (k >= cn.doff && k < cn.doff + nd) {
-          const T* src = cn.xloc + cn.nelim + (k - cn.doff);
+      const SolveNode<T>& cn = delay_child(sn, sns, children, k);
+      const T* src = cn.xloc + cn.nelim + (k - cn.doff);
 #pragma unroll
-          for (int q = 0; q < NR; ++q)
-            if (q < nrhs) v[q] = __ldcg(src + (int64_t)q * cn.m);
-          break;
-        }
-      }
+      for (int q = 0; q < NR; ++q)
+        if (q < nrhs) v[q] = __ldcg(src + (int64_t)q * cn.m);
     } else {
       P = pos - sn.ndelay_in;
     }
@@ -1460,12 +1486,7 @@ __device__ bool fwd_small(const SolveNode<T>& sn, const SolveNode<T>* sns, const
   }
   // the children's contribution rows (and delayed entries) are final once
   // every item of theirs has finished
-  bool ok = true;
-  for (int ci = sn.child_beg; ci < sn.child_end && ok; ++ci) {
-    const SolveNode<T>& cn = sns[children[ci]];
-    ok = wave_wait_count(wave_finished(cn), cn.nitf, status, s_fail);
-  }
-  if (!ok) {
+  if (!wave_wait_children(sn, sns, children, status)) {
     if (nelim > 0 && !sn.binv) cp_async_wait_all();
     return false;
   }
@@ -1479,17 +1500,11 @@ __device__ bool fwd_small(const SolveNode<T>& sn, const SolveNode<T>* sns, const
     for (int q = 0; q < NR; ++q) v[q] = xs[i * NR + q];
     if (dl[j] >= 0) {
       const int k = dl[j];
-      for (int ci = sn.child_beg; ci < sn.child_end; ++ci) {
-        const SolveNode<T>& cn = sns[children[ci]];
-        const int nd = cn.n - cn.nelim;
-        if (k >= cn.doff && k < cn.doff + nd) {
-          const T* src = cn.xloc + cn.nelim + (k - cn.doff);
+      const SolveNode<T>& cn = delay_child(sn, sns, children, k);
+      const T* src = cn.xloc + cn.nelim + (k - cn.doff);
 #pragma unroll
-          for (int q = 0; q < NR; ++q)
-            if (q < nrhs) v[q] = __ldcg(src + (int64_t)q * cn.m);
-          break;
-        }
-      }
+      for (int q = 0; q < NR; ++q)
+        if (q < nrhs) v[q] = __ldcg(src + (int64_t)q * cn.m);
     }
     if (src0[j]) {
 #pragma unroll
@@ -1656,11 +1671,7 @@ __global__ void __launch_bounds__(kSolveThreads, CPS)
     } else if (code >= kWaveGather) {
       // the children's contribution rows (and delayed entries) are final
       // once every item of theirs has finished
-      for (int ci = sn.child_beg; ci < sn.child_end && ok; ++ci) {
-        const SolveNode<T>& cn = sns[children[ci]];
-        ok = wave_wait_count(wave_finished(cn), cn.nitf, status, &s_fail);
-      }
-      if (!ok) continue;
+      if (!wave_wait_children(sn, sns, children, status)) continue;
       wave_stamp(wl, it, 1);
       {
         const int g0 = (code - kWaveGather) * kWaveGatherRows;
