@@ -204,13 +204,16 @@ __device__ __forceinline__ void solve_in_regs(int jb, const T* Lb, T (&x)[R][2])
 // solved as two halves of 32 rows with their inverses (k_half_inv, once per
 // factorisation) and the product between them; those operands' digits are put
 // into shared memory as fragments before the waits too.  One or two columns
-// keep the multiply-adds: the padding to eight columns would cost more.
+// keep the multiply-adds: the digit work of a tile, padded to eight columns,
+// stays the same while theirs falls (at four columns the two passes of a
+// 6000-row saddle point gain 1.97 -> 1.60 ms only).
 // Bound by the chain of pivot blocks at the top of the tree (eight columns:
 // 10 us a block for flag, digits, products of one tile and of the diagonal
-// block; 19 us before) and by the FP64 pipe in the small items below it.  57^3 Laplacian, 16 columns: forward 7.2 -> 3.6 ms, backward 8.5
-// -> 4.0 ms a pass (wide fronts only, from 4 pivot blocks: 4.3 and 5.0; from
-// 2: 3.8 and 4.3).  Six matrices each of five kinds, 16 columns: errors 0.50
-// to 0.95 of the multiply-adds', which round every product.
+// block; 19 us before) and by the FP64 pipe in the small items below it.
+// 57^3 Laplacian, 16 columns: forward 7.2 -> 3.6 ms, backward 8.5 -> 4.0 ms a
+// pass (fronts of 4 and more pivot blocks only: 4.3 and 5.0; of 2 and more:
+// 3.8 and 4.3).  Six matrices each of five kinds, 16 columns: errors 0.47 to
+// 0.86 of those of the multiply-adds, which round every product.
 template <typename T, int NR>
 constexpr bool solve_mma() { return sizeof(T) == 8 && NR >= 4; }
 template <int NR>
@@ -2401,7 +2404,7 @@ inline int wave_grid(int nitems, int cps) {
   return std::max(1, std::min(nitems, cps * nsm));
 }
 
-// FP32 factors only (FP64 factors keep the substitution in the passes)
+// FP32 factors only (FP64 factors: launch_half_inv, or the substitution)
 template <typename T>
 void launch_diag_inv(const SolveNode<T>* sn, const int2* blocks, int nblocks, cudaStream_t s) {
   if (nblocks <= 0) return;
