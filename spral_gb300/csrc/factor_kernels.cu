@@ -2193,10 +2193,17 @@ __device__ int tpp_fast(T* S, int ld, int m, int n, int nel, T* W0, T* W1, int* 
       else if (warp != 0) dw.kind = kStop;  // decided: warp 0 goes on
     }
     const bool all = batch != nullptr && nw > 1;
-    if (all && dw.kind == kMore) {
+    const bool more = all && dw.kind == kMore;
+    if (more) {
       __syncthreads();  // s_first is rewritten
       dw = decide_cta(S, ld, nel, m, n, action, th, batch, &s_first);
     }
+    // every warp read the pivot entries from S itself: all have their verdict
+    // (the same one) before warp 0 swaps and overwrites entries.  Without this
+    // barrier a late warp could reach another verdict and leave the others at
+    // a barrier of a different round.  A first candidate that warp 0 took alone
+    // was shared through s_first.
+    if (all && (wide || more)) __syncthreads();
     if (warp == 0) {
       Decision d = dw;
       if (!all) {
