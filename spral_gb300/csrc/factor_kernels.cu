@@ -867,19 +867,24 @@ __global__ void __launch_bounds__(kApplyRows) k_app_apply(FrontDesc<float>* fds,
         if (kd == 1) {
           const float x2 = xs[j + 1][t];
           const float dbh = ddh[2 * j + 1], dbl = ddl[2 * j + 1];
-          const float f1 = ld_entry_f32(ddh[2 * j], ddl[2 * j], dbh, dbl, xj, x2);
-          const float f2 = ld_entry_f32(dbh, dbl, ddh[2 * j + 3], ddl[2 * j + 3], xj, x2);
+          float f1 = ld_entry_f32(ddh[2 * j], ddl[2 * j], dbh, dbl, xj, x2);
+          float f2 = ld_entry_f32(dbh, dbl, ddh[2 * j + 3], ddl[2 * j + 3], xj, x2);
+          // above the band, in it, or NaN: a product outside the FP32 range
+          // makes its column NaN, whatever the FP64 value is (each is
+          // compared by itself, a maximum drops a NaN)
+          if (!(fabsf(f1) <= thr_lo && fabsf(f2) <= thr_lo)) {
+            const double dj = dd[2 * j], d21 = dd[2 * j + 1], d22 = dd[2 * j + 3];
+            const double l1 = dj * (double)xj + d21 * (double)x2;
+            const double l2 = d21 * (double)xj + d22 * (double)x2;
+            f1 = (float)l1;
+            f2 = (float)l2;
+            const int cand = over(l1) ? j : (over(l2) ? j + 1 : bs);
+            myfail = min(myfail, cand);
+          }
           fd.L[(int64_t)(p + j) * fd.ld + r] = f1;
           fd.L[(int64_t)(p + j + 1) * fd.ld + r] = f2;
           W[(int64_t)j * fd.ld] = xj;
           W[(int64_t)(j + 1) * fd.ld] = x2;
-          if (!(fmaxf(fabsf(f1), fabsf(f2)) <= thr_lo)) {  // above the band, in it, or Inf
-            const double dj = dd[2 * j], d21 = dd[2 * j + 1], d22 = dd[2 * j + 3];
-            const double l1 = dj * (double)xj + d21 * (double)x2;
-            const double l2 = d21 * (double)xj + d22 * (double)x2;
-            const int cand = over(l1) ? j : (over(l2) ? j + 1 : bs);
-            myfail = min(myfail, cand);
-          }
         } else if (kd == 3) {
           const double v = (double)xj;
           const double l = (fabs(v) < small) ? 0.0 : dinf() * v;
