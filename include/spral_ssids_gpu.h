@@ -185,7 +185,8 @@ int spral_ssids_gpu_debug_front(const void* numeric, int node, int* info, double
 
 /* Full solve plus FP64 refinement with b and x in device memory (n x nrhs,
  * leading dimension ld, pivot order).  iters / bwd_err receive the largest
- * refinement count and the final scaled backward error. */
+ * refinement count and the final scaled backward error (infinite where a
+ * solution has a NaN or Inf). */
 int spral_ssids_gpu_solve_refined_dev(void* numeric, int nrhs, const double* b_dev, double* x_dev,
                                       int ld, int* iters, double* bwd_err);
 

@@ -38,9 +38,8 @@ __global__ void k_zero_fronts(FrontDesc<T>* fds, const int* fronts) {
 // patterns, and an FP64 maximum issues some 30 times slower than an integer
 // one on GB300.
 typedef unsigned long long u64;
-__device__ __forceinline__ u64 mag_bits(double v) {  // a NaN counts as 0, as in fmax
-  const u64 k = (u64)__double_as_longlong(v) & 0x7fffffffffffffffULL;
-  return k > 0x7ff0000000000000ULL ? 0ULL : k;
+__device__ __forceinline__ u64 mag_bits(double v) {  // a NaN is above every number
+  return (u64)__double_as_longlong(v) & 0x7fffffffffffffffULL;
 }
 __device__ __forceinline__ u64 warp_max(u64 k) {
   const unsigned hi = (unsigned)(k >> 32), lo = (unsigned)k;
@@ -169,23 +168,27 @@ __global__ void __launch_bounds__(256) k_resid_norms(const int64_t* aptr, const 
 }
 
 // out[q] = the largest scaled backward error of right-hand side q over the
-// groups (one group when rows are not grouped)
+// groups (one group when rows are not grouped), out[nrhs + q] = 0, or the
+// groups' bwd_ratio flags where a NaN or Inf leaves a group without an error
 __global__ void k_bwd_finish(const double* work, int nrhs, int ngroups, double* out) {
   __shared__ double red[256];
   for (int q = 0; q < nrhs; ++q) {
     double m = 0.0;
+    int bad = 0;
     for (int g = threadIdx.x; g < ngroups; g += blockDim.x) {
       const double* w = work + (int64_t)g * kResStride;
-      const double den = w[0] * w[1 + 3 * q] + w[2 + 3 * q];
-      m = fmax(m, den > 0 ? w[3 + 3 * q] / den : 0.0);
+      m = fmax(m, bwd_ratio(w[0], w[1 + 3 * q], w[2 + 3 * q], w[3 + 3 * q], bad));
     }
     red[threadIdx.x] = m;
-    __syncthreads();
+    bad = (__syncthreads_or(bad & 1) ? 1 : 0) | (__syncthreads_or(bad & 2) ? 2 : 0);
     for (int h = blockDim.x / 2; h > 0; h >>= 1) {
       if ((int)threadIdx.x < h) red[threadIdx.x] = fmax(red[threadIdx.x], red[threadIdx.x + h]);
       __syncthreads();
     }
-    if (threadIdx.x == 0) out[q] = red[0];
+    if (threadIdx.x == 0) {
+      out[q] = red[0];
+      out[nrhs + q] = bad;
+    }
     __syncthreads();
   }
 }
@@ -216,14 +219,14 @@ template void launch_zero_fronts<float>(FrontDesc<float>*, const int*, int, int,
 
 // r = b - A x and the scaled backward error of each right-hand side, the
 // largest over the row groups when row_group is given (work must hold
-// nrhs + max(ngroups, 1) * (1 + 3*kSolveRhs) doubles; the result per rhs is
-// written to work[0 .. nrhs)).  nnz: entries of the full CSR.
+// 2 nrhs + max(ngroups, 1) * kResStride doubles; the result per rhs, see k_bwd_finish, is written to
+// work[0 .. 2 nrhs), the groups' maxima follow).  nnz: entries of the full CSR.
 void launch_resid_bwd_err(const int64_t* aptr, const int* acol, const int64_t* asrc,
                           const double* aval, int n, int64_t nnz, const double* x,
                           const double* b, double* r, int nrhs, int ld, double* work,
                           const int* row_group, int ngroups,
                           cudaStream_t s) {
-  double* acc = work + nrhs;
+  double* acc = work + 2 * nrhs;
   const int ng = row_group ? std::max(ngroups, 1) : 1;
   cudaMemsetAsync(acc, 0, (size_t)ng * kResStride * sizeof(double), s);
   const bool small = nnz <= (int64_t)kResShort * n;

@@ -2328,7 +2328,7 @@ struct Numeric : NumericBase {
       bbuf.ensure((size_t)n * q + 1);
       xbuf.ensure((size_t)n * q + 1);
       rbuf.ensure((size_t)n * q + 1);
-      nbuf.ensure(q + (size_t)std::max(S->ngroups, 1) * (1 + 3 * kSolveRhs) + 8);
+      nbuf.ensure(2 * q + (size_t)std::max(S->ngroups, 1) * kResStride + 8);
       for (int r = 0; r < q; ++r)
         CK(cudaMemcpyAsync(bbuf.p + (size_t)r * n, xh + (size_t)(r0 + r) * ldx,
                            n * sizeof(double), cudaMemcpyHostToDevice, s));
@@ -2389,11 +2389,11 @@ struct Numeric : NumericBase {
   // and refined with those factors.  The FP64 factorisation's statistics
   // (inertia, delays) replace the FP32 ones.  Returns the FP64 handle to
   // solve with, or nullptr when no fallback is needed (FP64 handles, or the
-  // target was met).
+  // target was met, or a NaN or Inf in A or b leaves nothing to gain).
   NumericBase* fp64_fallback() {
     if (!std::is_same<T, float>::value) return nullptr;
     if (S->gopts.no_fp64_fallback) return nullptr;
-    if (!(last_bwd_err > S->gopts.refine_tol)) return nullptr;
+    if (!missed) return nullptr;
     if (!fb) {
       fb.reset(new Numeric<double>(S));
       fb->posdef = posdef;
@@ -2414,15 +2414,20 @@ struct Numeric : NumericBase {
     return fb_ok ? fb.get() : nullptr;
   }
 
+  // whether the last refinement left a right-hand side that better factors
+  // could bring to the target (not one with a NaN or Inf in A or b)
+  bool missed = false;
+
   // refinement of x (device, n x q, ld) against b; returns steps taken
   int refine_dev(int q, double* x, const double* b, int ld) {
     const int n = S->n;
     cudaStream_t s = stream;
     rbuf.ensure((size_t)ld * q + 1);
-    nbuf.ensure(q + (size_t)std::max(S->ngroups, 1) * (1 + 3 * kSolveRhs) + 8);
-    std::vector<double> h(q);
+    nbuf.ensure(2 * q + (size_t)std::max(S->ngroups, 1) * kResStride + 8);
+    std::vector<double> h(2 * q);
     int it = 0;
     const int maxit = S->gopts.max_refine;
+    double prev = 0.0;  // the last step's error
     last_refine_q = q;
     group_prev.clear();
     for (;; ++it) {
@@ -2430,17 +2435,24 @@ struct Numeric : NumericBase {
       launch_resid_bwd_err(S->d_aptr, S->d_acol, S->d_asrc, cur_aval, n, S->nnz_full, x, b,
                            rbuf.p, q, ld, nbuf.p, S->d_row_group, S->ngroups, s);
       pmark(tm(), kPhHost, s);
-      CK(cudaMemcpyAsync(h.data(), nbuf.p, q * sizeof(double), cudaMemcpyDeviceToHost, s));
+      CK(cudaMemcpyAsync(h.data(), nbuf.p, h.size() * sizeof(double), cudaMemcpyDeviceToHost, s));
       CK(cudaStreamSynchronize(s));
       if (profile) ptimer.flush();
+      // right-hand sides (or row groups) with a NaN or Inf have missed the
+      // target and no step mends them: the others are refined as without them
       double worst = 0;
-      for (int r = 0; r < q; ++r) worst = std::max(worst, h[r]);
+      bool bad_x = false, bad = false;
+      for (int r = 0; r < q; ++r) {
+        worst = std::max(worst, h[r]);
+        bad_x = bad_x || ((int)h[q + r] & 1);
+        bad = bad || h[q + r] != 0.0;
+      }
       // stop at the target, after max_refine steps, or when a step did not
       // halve the backward error (the factors' precision cannot reach it).
       // Row groups whose caller handles the misses itself (no FP64
       // fallback): stalled only once no group above the target halved its
       // own error, so the other groups finish their refinement.
-      bool stalled = it > 0 && !(worst < 0.5 * last_bwd_err);
+      bool stalled = it > 0 && !(worst < 0.5 * prev);
       bool masked = false;
       // row groups judged one by one: FP32 factors whose caller handles
       // the misses (no FP64 fallback here), and FP64 factors
@@ -2448,7 +2460,7 @@ struct Numeric : NumericBase {
       if (S->d_row_group && by_group && worst > S->gopts.refine_tol) {
         last_refine_q = q;
         std::vector<double> ge(S->ngroups);
-        group_bwd_errors(ge.data(), S->ngroups);
+        group_errors(ge.data(), false);
         if (S->gopts.no_fp64_fallback && it > 0 && group_prev.size() == ge.size()) {
           stalled = true;
           for (size_t g = 0; g < ge.size() && stalled; ++g)
@@ -2466,7 +2478,9 @@ struct Numeric : NumericBase {
         }
         group_prev.swap(ge);
       }
-      last_bwd_err = worst;
+      prev = worst;
+      last_bwd_err = bad ? INFINITY : worst;
+      missed = worst > S->gopts.refine_tol || bad_x;
       if (!(worst > S->gopts.refine_tol) || it >= maxit || stalled) break;
       solve_dev(0, q, rbuf.p, ld, nullptr);
       pmark(tm(), kPhAxpy, s);
@@ -2485,20 +2499,24 @@ struct Numeric : NumericBase {
 
   int last_refine_q = 0;  // right-hand sides of the last refinement's residuals in nbuf
   std::vector<double> group_prev;  // per row group, the previous refinement step's error
-  int group_bwd_errors(double* out, int ngroups) override {
-    if (!S->d_row_group || last_refine_q <= 0 || ngroups != S->ngroups) return -1;
-    std::vector<double> w((size_t)ngroups * kResStride);
-    CK(cudaMemcpy(w.data(), nbuf.p + last_refine_q, w.size() * sizeof(double),
+  // per row group, the largest error of the last residuals; with_bad: infinite
+  // where a NaN or Inf leaves a right-hand side without one, else without those
+  void group_errors(double* out, bool with_bad) {
+    std::vector<double> w((size_t)S->ngroups * kResStride);
+    CK(cudaMemcpy(w.data(), nbuf.p + 2 * last_refine_q, w.size() * sizeof(double),
                   cudaMemcpyDeviceToHost));
-    for (int g = 0; g < ngroups; ++g) {
+    for (int g = 0; g < S->ngroups; ++g) {
       const double* wg = w.data() + (size_t)g * kResStride;
       double e = 0.0;
-      for (int r = 0; r < last_refine_q; ++r) {
-        const double den = wg[0] * wg[1 + 3 * r] + wg[2 + 3 * r];
-        e = std::max(e, den > 0 ? wg[3 + 3 * r] / den : 0.0);
-      }
-      out[g] = e;
+      int bad = 0;
+      for (int r = 0; r < last_refine_q; ++r)
+        e = std::max(e, bwd_ratio(wg[0], wg[1 + 3 * r], wg[2 + 3 * r], wg[3 + 3 * r], bad));
+      out[g] = with_bad && bad ? INFINITY : e;
     }
+  }
+  int group_bwd_errors(double* out, int ngroups) override {
+    if (!S->d_row_group || last_refine_q <= 0 || ngroups != S->ngroups) return -1;
+    group_errors(out, true);
     return 0;
   }
 

@@ -385,6 +385,16 @@ constexpr int kSolveRhs = 16;   // right-hand sides per pass
 // doubles per row group in the refinement's residual workspace: ||A||, then
 // (||x||, ||b||, ||r||) per right-hand side of a pass
 constexpr int kResStride = 1 + 3 * kSolveRhs;
+// Scaled backward error ||r|| / (||A|| ||x|| + ||b||) from those maxima, and
+// in bad (or-ed): 1 a NaN or Inf in x or r, 2 in A or b; such a right-hand
+// side has no error (0), it is never met.
+__host__ __device__ inline double bwd_ratio(double a, double x, double b, double r, int& bad) {
+  const double top = 1.7976931348623157e308;
+  if (!(a <= top && b <= top)) { bad |= 2; return 0.0; }
+  if (!(x <= top && r <= top)) { bad |= 1; return 0.0; }
+  const double den = a * x + b;
+  return den > 0 ? r / den : 0.0;
+}
 
 template <typename T>
 void launch_fwd_gather(const SolveNode<T>* sn, const int* nodes, int nn, const int* children,
