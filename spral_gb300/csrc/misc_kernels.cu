@@ -51,34 +51,50 @@ __device__ __forceinline__ void atomic_max_pos(double* a, u64 bits) {
   atomicMax(reinterpret_cast<u64*>(a), bits);
 }
 
-// r = b - A x and the maxima of the scaled backward error in one pass.
-// G lanes share a row (its non-zeros strided over the lanes); each non-zero
-// is applied to kResQC right-hand sides at once (chunk blockIdx.y), so the
-// row's index and value loads are shared by the chunk.  Every lane of a warp
-// runs the same number of row iterations, so the lane reductions use
-// full-warp shuffles.  work: [0] ||A||_inf, then per rhs (||x||, ||b||,
-// ||r||) at 1 + 3q (maxima, order-independent).
+// r = b - A x and the maxima of the scaled backward error in one pass.  Each
+// non-zero is applied to kResQC right-hand sides at once (chunk blockIdx.y),
+// so the row's index and value loads are shared by the chunk.  work: [0]
+// ||A||_inf, then per rhs (||x||, ||b||, ||r||) at 1 + 3q (maxima,
+// order-independent).
 //
 // Bound by FP64 issue (about 75 cycles a warp instruction): a non-zero costs
 // one multiply-add per right-hand side and, in the first chunk, one addition
-// for the row sum.  One lane per row needs the fewest (short rows: no partial
-// sums to add over lanes); four lanes per row where rows average more than
-// kResShort non-zeros and a warp would wait for its longest.  320 stacked 2D
-// Laplacians (n = 0.93M, one right-hand side): 751 -> 123 us, 48^3 Laplacian
-// with 8 right-hand sides 127 -> 62 us, with the maxima in integers.
+// for the row sum.  One lane per row needs the fewest (no partial sums to add
+// over lanes), but a warp waits for its longest row: a row of more than
+// kResShort non-zeros is read by four lanes.  Each row goes by its own length,
+// so its residual has the same bits whatever rows and matrices are beside it.
+// A warp takes RPW rows: 32, or 8 where rows average more than kResShort
+// non-zeros and most are read by four lanes (the order of a row's sum does not
+// depend on it).  320 stacked 2D Laplacians (n = 0.93M, one right-hand side):
+// 751 -> 123 us, 48^3 Laplacian with 8 right-hand sides 127 -> 62 us, with the
+// maxima in integers.
 constexpr int kResQC = 4;
 constexpr int kResShort = 12;
+// the non-zeros k0, k0 + step, ... < k1 of a row
+__device__ __forceinline__ void resid_row(const int* acol, const int64_t* asrc, const double* aval,
+                                          const double* x, int ld, int q0, int nq, bool norm,
+                                          int64_t k0, int64_t k1, int step, double (&s)[kResQC],
+                                          double& ra) {
+  for (int64_t k = k0; k < k1; k += step) {
+    const double a = aval[asrc[k]];
+    const int64_t c = acol[k];
+    if (norm) ra += fabs(a);
+#pragma unroll
+    for (int q = 0; q < kResQC; ++q)
+      if (q < nq) s[q] = fma(a, x[(int64_t)(q0 + q) * ld + c], s[q]);
+  }
+}
 // With row groups (row_group != nullptr: the group of each row, e.g. the
 // matrix of a batch it belongs to) the maxima are kept per group, at
 // work[g * kResStride ...], so the backward error can be judged per group.
-template <int G>
+template <int RPW>
 __global__ void __launch_bounds__(256) k_resid_norms(const int64_t* aptr, const int* acol,
                                                      const int64_t* asrc, const double* aval,
                                                      int n, const double* x, const double* b,
                                                      double* r, int nrhs, int ld, double* work,
                                                      const int* row_group) {
-  constexpr int QC = kResQC, RPW = 32 / G, NV = 1 + 3 * QC;
-  const int lane = threadIdx.x & 31, sub = lane & (G - 1);
+  constexpr int QC = kResQC, NV = 1 + 3 * QC;
+  const int lane = threadIdx.x & 31;
   const int q0 = blockIdx.y * QC;
   const int nq = min(QC, nrhs - q0);
   const bool norm = blockIdx.y == 0;  // this chunk forms ||A||
@@ -88,34 +104,47 @@ __global__ void __launch_bounds__(256) k_resid_norms(const int64_t* aptr, const 
 #pragma unroll
   for (int v = 0; v < NV; ++v) m[v] = 0;
   for (int64_t base = warp * RPW; base < n; base += nwarp * RPW) {
-    const int64_t i = base + lane / G;
-    const bool ok = i < n;
+    const int64_t i = base + lane;  // this lane's row
+    const bool ok = lane < RPW && i < n;
+    const int64_t k0 = ok ? aptr[i] : 0, k1 = ok ? aptr[i + 1] : 0;
+    const bool wide = k1 - k0 > kResShort;
     double s[QC], ra = 0.0;
 #pragma unroll
     for (int q = 0; q < QC; ++q) s[q] = 0.0;
-    if (ok) {
-      const int64_t k1 = aptr[i + 1];
-      for (int64_t k = aptr[i] + sub; k < k1; k += G) {
-        const double a = aval[asrc[k]];
-        const int64_t c = acol[k];
-        if (norm) ra += fabs(a);
+    if (!wide) resid_row(acol, asrc, aval, x, ld, q0, nq, norm, k0, k1, 1, s, ra);
+    const unsigned wides = __ballot_sync(0xffffffffu, wide);
+    if (wides) {
+#pragma unroll 1
+      for (int j = 0; j < RPW / 8; ++j) {  // eight rows, four lanes each
+        if (!((wides >> (8 * j)) & 0xffu)) continue;
+        const int w = 8 * j + (lane >> 2);  // the row's own lane
+        const int64_t j0 = __shfl_sync(0xffffffffu, k0, w), j1 = __shfl_sync(0xffffffffu, k1, w);
+        double t[QC], ta = 0.0;
 #pragma unroll
-        for (int q = 0; q < QC; ++q)
-          if (q < nq) s[q] = fma(a, x[(int64_t)(q0 + q) * ld + c], s[q]);
+        for (int q = 0; q < QC; ++q) t[q] = 0.0;
+        if ((wides >> w) & 1u)
+          resid_row(acol, asrc, aval, x, ld, q0, nq, norm, j0 + (lane & 3), j1, 4, t, ta);
+        const bool back = wide && (lane >> 3) == j;
+        const int from = 4 * (lane & 7);
+#pragma unroll
+        for (int q = -1; q < QC; ++q) {
+          if (q < 0 ? !norm : q >= nq) continue;
+          double v = q < 0 ? ta : t[q < 0 ? 0 : q];
+          v += __shfl_xor_sync(0xffffffffu, v, 2);
+          v += __shfl_xor_sync(0xffffffffu, v, 1);
+          v = __shfl_sync(0xffffffffu, v, from);
+          if (back) {
+            if (q < 0) ra = v;
+            else s[q < 0 ? 0 : q] = v;
+          }
+        }
       }
-    }
-#pragma unroll
-    for (int off = G / 2; off > 0; off >>= 1) {
-      if (norm) ra += __shfl_xor_sync(0xffffffffu, ra, off);
-#pragma unroll
-      for (int q = 0; q < QC; ++q)
-        if (q < nq) s[q] += __shfl_xor_sync(0xffffffffu, s[q], off);
     }
     if (row_group) {
 #pragma unroll
       for (int v = 0; v < NV; ++v) m[v] = 0;
     }
-    if (ok && sub == 0) {
+    if (ok) {
       m[0] = max(m[0], mag_bits(ra));
 #pragma unroll
       for (int q = 0; q < QC; ++q) {
@@ -142,7 +171,7 @@ __global__ void __launch_bounds__(256) k_resid_norms(const int64_t* aptr, const 
         const u64 k = warp_max(m[v]);
         if (lane == 0) atomic_max_pos(&w[v == 0 ? 0 : 3 * q0 + v], k);
       }
-    } else if (ok && sub == 0) {
+    } else if (ok) {
       double* w = work + (int64_t)g * kResStride;
 #pragma unroll
       for (int v = 0; v < NV; ++v)
@@ -234,10 +263,10 @@ void launch_resid_bwd_err(const int64_t* aptr, const int* acol, const int64_t* a
   const int bx = std::max(1, std::min((n + rows_per_block - 1) / rows_per_block, 4 * 152));
   const dim3 grid(bx, (nrhs + kResQC - 1) / kResQC);
   if (small)
-    k_resid_norms<1><<<grid, 256, 0, s>>>(aptr, acol, asrc, aval, n, x, b, r, nrhs, ld, acc,
-                                          row_group);
+    k_resid_norms<32><<<grid, 256, 0, s>>>(aptr, acol, asrc, aval, n, x, b, r, nrhs, ld, acc,
+                                           row_group);
   else
-    k_resid_norms<4><<<grid, 256, 0, s>>>(aptr, acol, asrc, aval, n, x, b, r, nrhs, ld, acc,
+    k_resid_norms<8><<<grid, 256, 0, s>>>(aptr, acol, asrc, aval, n, x, b, r, nrhs, ld, acc,
                                           row_group);
   note_launches(1);
   { k_bwd_finish<<<1, 256, 0, s>>>(acc, nrhs, ng, work); note_launches(1); }
