@@ -297,11 +297,17 @@ struct DevBuf {
     if (n <= cap) return;
     // kernels already queued may still use the old block: give it to the
     // driver (cudaFree waits for them) rather than to the cache
-    if (p) release_now(p, dev);
-    p = nullptr;
-    size_t nc = std::max(n, cap + cap / 2);
+    const size_t nc = std::max(n, cap + cap / 2);
+    release();
     p = static_cast<T*>(cache_alloc(std::max<size_t>(nc, 1) * sizeof(T), &bytes, &dev));
     cap = bytes / sizeof(T);
+  }
+  // an allocation that fails leaves the buffer empty (no old size beside a
+  // null pointer), so that a later call allocates it again
+  void release() {
+    if (p) release_now(p, dev);
+    p = nullptr;
+    cap = 0;
   }
   // the owner has finished all work that uses the block (Numeric's
   // destructor synchronises its stream first)
@@ -1207,7 +1213,6 @@ struct Numeric : NumericBase {
     } catch (CudaFail const& e) {
       if (e.err != cudaErrorMemoryAllocation) throw;
       cudaGetLastError();
-      slice_scratch.cap = 0;
       return false;
     }
     return true;
@@ -2235,8 +2240,6 @@ struct Numeric : NumericBase {
       } catch (CudaFail const& e) {
         if (e.err != cudaErrorMemoryAllocation) throw;
         cudaGetLastError();
-        if (!wave_hinv.p) wave_hinv.cap = 0;
-        if (!hinv_blocks.p) hinv_blocks.cap = 0;
         hinv_off = true;
       }
       // captured passes hold the table's address, or none
