@@ -701,6 +701,20 @@ struct NumericBase {
   std::vector<int> contrib_rlist, contrib_perm;
   int contrib_n = 0, contrib_ndelay = 0, contrib_lddelay = 0;
   DevBuf<double> hsolve;  // device copy of host right-hand sides (host-buffer solves)
+  virtual bool give_up_memory() = 0;
+  // f(); where memory for it is lacking, once more without what the handle
+  // can do without (f can be repeated)
+  template <typename F>
+  void with_memory(F&& f) {
+    try {
+      f();
+      return;
+    } catch (CudaFail const& e) {
+      cudaGetLastError();
+      if (e.err != cudaErrorMemoryAllocation || !give_up_memory()) throw;
+    }
+    f();
+  }
   // FP64 refactorisations taken by the FP32-factor path's refined solves
   int fallbacks = 0;
 };
@@ -1208,8 +1222,10 @@ struct Numeric : NumericBase {
   // The slices' memory for the fronts of a level whose sizes are known; a
   // device too full for it keeps the SIMT kernel (false, for this handle).
   bool slice_reserve(int f0, int f1) {
+    const SliceBatch b = slice_contrib(f0, f1);
     try {
-      slice_scratch.ensure(slice_contrib(f0, f1).scratch + 1);
+      slice_scratch.ensure(b.scratch);
+      slice_tab.ensure(b.table);
     } catch (CudaFail const& e) {
       if (e.err != cudaErrorMemoryAllocation) throw;
       cudaGetLastError();
@@ -1217,11 +1233,26 @@ struct Numeric : NumericBase {
     }
     return true;
   }
-  // eager mode: tables uploaded now, then the launches
+  // Gives back what only makes the handle faster (the slices' memory and the
+  // half inverses of the solves) when an allocation it needs has failed; the
+  // handle goes on with the multiply-adds.  False when there is nothing to give.
+  bool give_up_memory() override {
+    if (!slice_scratch.p && !wave_hinv.p) return false;
+    CK(cudaStreamSynchronize(stream));
+    drop_fgraph();
+    drop_graphs();
+    use_slices = false;
+    hinv_off = true;
+    hinv_ready = false;
+    slice_scratch.release();
+    slice_tab.release();
+    wave_hinv.release();
+    hinv_blocks.release();
+    return true;
+  }
+  // eager mode: tables uploaded now, then the launches (memory: slice_reserve)
   void slice_run(SliceBatch b, cudaStream_t s) {
     if (b.jobs.empty()) return;
-    slice_scratch.ensure(b.scratch);
-    slice_tab.ensure(b.table);
     const std::vector<char> img = slice_place(b);
     CK(cudaMemcpyAsync(slice_tab.p, img.data(), img.size(), cudaMemcpyHostToDevice, s));
     slice_enqueue(b, slice_tab.p, s);
@@ -1479,7 +1510,7 @@ struct Numeric : NumericBase {
         soff.push_back(tab);
         tab += b.table;
       }
-      slice_scratch.ensure(scr + 1);
+      slice_scratch.ensure(scr);
       void* b = nullptr;
       CK(cudaMalloc(&b, std::max<size_t>(tab, 1)));
       fgraph_blobs.push_back(b);
@@ -1767,6 +1798,12 @@ struct Numeric : NumericBase {
   int factor(const double* aval, bool on_device, const double* scaling,
              cudaStream_t user_stream) override {
     if (user_stream) CK(cudaStreamSynchronize(user_stream));
+    int r = 0;
+    with_memory([&] { r = factor_once(aval, on_device, scaling); });
+    return r;
+  }
+
+  int factor_once(const double* aval, bool on_device, const double* scaling) {
     solve_ready = false;
     fb_stale = true;
     last_scaled = scaling != nullptr;
@@ -2298,7 +2335,7 @@ struct Numeric : NumericBase {
   }
 
   int solve_dev(int job, int nrhs, double* x, int ldx, cudaStream_t us) override {
-    prepare_solve();
+    with_memory([&] { prepare_solve(); });
     cudaStream_t s = stream;
     if (us) CK(cudaStreamSynchronize(us));
     for (int r0 = 0; r0 < nrhs; r0 += kSolveRhs) {
@@ -2328,10 +2365,10 @@ struct Numeric : NumericBase {
     int itmax = 0;
     for (int r0 = 0; r0 < nrhs; r0 += kSolveRhs) {
       const int q = std::min(kSolveRhs, nrhs - r0);
-      bbuf.ensure((size_t)n * q + 1);
-      xbuf.ensure((size_t)n * q + 1);
-      rbuf.ensure((size_t)n * q + 1);
-      nbuf.ensure(2 * q + (size_t)std::max(S->ngroups, 1) * kResStride + 8);
+      with_memory([&] {
+        bbuf.ensure((size_t)n * q + 1);
+        xbuf.ensure((size_t)n * q + 1);
+      });
       for (int r = 0; r < q; ++r)
         CK(cudaMemcpyAsync(bbuf.p + (size_t)r * n, xh + (size_t)(r0 + r) * ldx,
                            n * sizeof(double), cudaMemcpyHostToDevice, s));
@@ -2425,8 +2462,10 @@ struct Numeric : NumericBase {
   int refine_dev(int q, double* x, const double* b, int ld) {
     const int n = S->n;
     cudaStream_t s = stream;
-    rbuf.ensure((size_t)ld * q + 1);
-    nbuf.ensure(2 * q + (size_t)std::max(S->ngroups, 1) * kResStride + 8);
+    with_memory([&] {
+      rbuf.ensure((size_t)ld * q + 1);
+      nbuf.ensure(2 * q + (size_t)std::max(S->ngroups, 1) * kResStride + 8);
+    });
     std::vector<double> h(2 * q);
     int it = 0;
     const int maxit = S->gopts.max_refine;
@@ -2781,7 +2820,7 @@ static int host_solve(const void* numeric, int job, int nrhs, double* x, int ldx
     CK(cudaSetDevice(S->device));
     // a per-handle device buffer and the handle's stream: no allocation and
     // no device-wide synchronisation per call
-    N->hsolve.ensure(std::max<size_t>((size_t)n * nrhs, 1));
+    N->with_memory([&] { N->hsolve.ensure(std::max<size_t>((size_t)n * nrhs, 1)); });
     double* dx = N->hsolve.p;
     cudaStream_t s = N->get_stream();
     for (int r = 0; r < nrhs; ++r)

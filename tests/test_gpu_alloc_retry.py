@@ -65,3 +65,48 @@ def test_gpu_handle_works_after_a_failed_allocation(fail_after, precision):
         fail_after(-1)
         _check(fk, p, r, v, b)
     fk.free()
+
+
+def test_gpu_slices_are_given_up_for_memory_the_factorisation_needs(fail_after):
+    """FP64 factors: from the first digit slices of the tensor-core updates on,
+    an allocation that fails costs those and not the factorisation, and later
+    factorisations and solves (captured graphs too) go on without."""
+    p, r, v, ak, b = _problem()
+    lib = _native.lib()
+    flags = []
+    for k in range(40):
+        lib.spral_ssids_gpu_release_cache()
+        fail_after(k)
+        try:
+            fk, inf = ssids.factor(ak, v)
+        except RuntimeError:
+            flags.append(None)
+            continue
+        finally:
+            fail_after(-1)
+        flags.append(inf.flag)
+        if inf.flag == 0:
+            _check(fk, p, r, v, b)
+            for _ in range(2):
+                assert fk.refactor(v) == 0
+                _check(fk, p, r, v, b)
+        fk.free()
+    assert flags.count(ssids.SSIDS_ERROR_ALLOCATION) > 0 and flags[-1] == 0
+    assert all(f == 0 for f in flags[flags.index(0):])
+
+
+def test_gpu_solve_gives_up_slices_for_its_own_memory(fail_after):
+    p, r, v, ak, b = _problem()
+    lib = _native.lib()
+    for refined in (False, True):
+        for k in range(12):
+            fk, inf = ssids.factor(ak, v)
+            assert inf.flag == 0
+            lib.spral_ssids_gpu_release_cache()
+            fail_after(k)
+            x = fk.solve_refined(b) if refined else fk.solve(b)
+            fail_after(-1)
+            assert M.scaled_bwd_error(p, r, v, x, b).max() <= 5e-14
+            assert fk.refactor(v) == 0
+            _check(fk, p, r, v, b)
+            fk.free()
