@@ -2834,6 +2834,8 @@ static int host_solve(const void* numeric, int job, int nrhs, double* x, int ldx
     return 0;
   } catch (CudaFail const& e) {
     return map_cuda_error(e, nullptr);
+  } catch (std::bad_alloc const&) {
+    return -50;
   }
 }
 
@@ -2865,6 +2867,8 @@ int spral_ssids_gpu_solve_dev(void* numeric, int job, int nrhs, double* x_dev, i
     return N->solve_dev(job, nrhs, x_dev, ldx, (cudaStream_t)stream);
   } catch (CudaFail const& e) {
     return map_cuda_error(e, nullptr);
+  } catch (std::bad_alloc const&) {
+    return -50;
   }
 }
 
@@ -2874,6 +2878,8 @@ int spral_ssids_gpu_solve_refined(void* numeric, int nrhs, double* x, int ldx, i
     return N->solve_refined(nrhs, x, ldx, iters);
   } catch (CudaFail const& e) {
     return map_cuda_error(e, nullptr);
+  } catch (std::bad_alloc const&) {
+    return -50;
   }
 }
 
@@ -3110,6 +3116,8 @@ int spral_ssids_gpu_solve_refined_dev(void* numeric, int nrhs, const double* b_d
     return N->solve_refined_dev(nrhs, b_dev, x_dev, ld, iters, bwd_err);
   } catch (ssids300::CudaFail const& e) {
     return map_cuda_error(e, nullptr);
+  } catch (std::bad_alloc const&) {
+    return -50;
   }
 }
 

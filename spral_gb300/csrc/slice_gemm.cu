@@ -43,6 +43,7 @@
 #include <algorithm>
 #include <climits>
 #include <cstring>
+#include <new>
 #include <vector>
 
 #include "spral_ssids_gpu.h"
@@ -509,7 +510,7 @@ int launch_slice_gemm(void* table, const std::vector<SliceJob>& jobs, size_t fir
 // ---------------------------------------------------------------------------
 extern "C" int spral_ssids_gpu_slice_gemm_f64(int M, int N, int K, const double* A, int lda,
                                               const double* B, int ldb, double* C, int ldc,
-                                              int reps, void* stream) {
+                                              int reps, void* stream) try {
   using namespace ssids300;
   if (M < 0 || N < 0 || K < 0 || N > M || lda < M || ldb < N || ldc < M || reps < 1) return -1;
   if (M == 0 || N == 0 || K == 0) return 0;
@@ -557,4 +558,6 @@ extern "C" int spral_ssids_gpu_slice_gemm_f64(int M, int N, int K, const double*
   if (rc == 0 && hs != 0) rc = -52;
   cudaFree(base);
   return rc;
+} catch (std::bad_alloc const&) {
+  return -50;
 }
