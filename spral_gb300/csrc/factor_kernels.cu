@@ -1249,7 +1249,6 @@ __global__ void __launch_bounds__(256) k_app_panel(FrontDesc<T>* fds, FrontState
 // ------------------------------------------------------------------------
 constexpr int PF_M = 64, PF_N = 32, PF_THREADS = 128;
 constexpr int PF_A_SLICE = PF_M * kBlk * 2, PF_B_SLICE = PF_N * kBlk * 2;  // bytes per digit
-constexpr int kEmptyRow = -(1 << 18);  // exponent of a row of zeros
 constexpr size_t kPanelF64Smem = (size_t)8 * (PF_A_SLICE + PF_B_SLICE);
 
 __global__ void __launch_bounds__(PF_THREADS, 4)
@@ -1303,7 +1302,7 @@ __global__ void __launch_bounds__(PF_THREADS, 4)
                   ? (unsigned long long)__double_as_longlong(B[(kb + q) * ld + col0 + rb]) : 0ULL;
     }
     __syncthreads();  // hs; the previous tile's digits have been read
-    int e0[8], e1[8], eb[8], ma = kEmptyRow, mb = kEmptyRow;
+    int e0[8], e1[8], eb[8], ma = kEmptyExponent, mb = kEmptyExponent;
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
       e0[q] = slice_exponent(a0[q], ka + q < K ? hs[ka + q] : 0);
@@ -2621,7 +2620,7 @@ __global__ void __launch_bounds__(kSmallContribThreads, 2)
                         ? (unsigned long long)__double_as_longlong(B[(int64_t)k * cm + c0 + 8 * u]) : 0ULL;
         }
       }
-      int h[8], er[2] = {-(1 << 18), -(1 << 18)}, ec[2] = {-(1 << 18), -(1 << 18)};
+      int h[8], er[2] = {kEmptyExponent, kEmptyExponent}, ec[2] = {kEmptyExponent, kEmptyExponent};
 #pragma unroll
       for (int q = 0; q < 8; ++q) {
         const int k = k0 + (q >> 2) * 16 + t2 + (q & 1) + ((q >> 1) & 1) * 8;

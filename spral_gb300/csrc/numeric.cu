@@ -966,8 +966,14 @@ struct Numeric : NumericBase {
   // items'), formed before the first pass with more than two right-hand sides
   // after a factorisation
   DevBuf<double> wave_hinv;
+  // X, then the rows' balance exponents, then the blocks' growth flags
+  int* hinv_exps() { return reinterpret_cast<int*>(wave_hinv.p + hblocks.size() * 2 * 32 * 32); }
+  unsigned char* hinv_grown() {
+    return reinterpret_cast<unsigned char*>(hinv_exps() + hinv_rows);
+  }
   DevBuf<int2> hinv_blocks;
-  std::vector<int2> hblocks;
+  std::vector<int2> hblocks, hchunks;  // pivot blocks; chunks of 64 rows
+  size_t hinv_rows = 0;
   bool hinv_ready = false, hinv_off = false;  // off: no memory for them
   size_t wave_nflags = 0;
   // optional trace of the wavefront passes (SPRAL_GB300_WAVE_TRACE = path
@@ -988,6 +994,8 @@ struct Numeric : NumericBase {
     // unless they are a few among many small ones.  A 6000-row saddle point,
     // 4 columns: forward and backward 1.60 ms with two, 1.82 ms with three)
     w.hinv = q > 2 && hinv_ready ? wave_hinv.p : nullptr;
+    w.hexp = w.hinv ? hinv_exps() : nullptr;
+    w.grown = w.hinv ? hinv_grown() : nullptr;
     const bool tc = w.hinv && 64 * (long long)hblocks.size() > wave_nsmall;
     w.ctas_per_sm = 2 * wave_nsmall > wave_nfwd && !tc ? 3 : 2;
     w.front_group = S->d_front_group;
@@ -2095,13 +2103,18 @@ struct Numeric : NumericBase {
                            cudaMemcpyHostToDevice, stream));
     }
     hblocks.clear();
+    hchunks.clear();
+    hinv_rows = 0;
     hinv_ready = false;
-    std::vector<int64_t> hinv_first(nn, -1);
+    std::vector<int64_t> hinv_first(nn, -1), hinv_row0(nn, 0);
     if (std::is_same<T, double>::value && use_wave && use_tc_solve) {
       for (int f = 0; f < nn; ++f) {
         if (nblk_of(f) < 1 || small_of(f)) continue;
         hinv_first[f] = (int64_t)hblocks.size();
         for (int b = 0; b < nblk_of(f); ++b) hblocks.push_back(make_int2(f, b));
+        hinv_row0[f] = (int64_t)hinv_rows;
+        hinv_rows += m_[f];
+        for (int c = 0; c * kSolveBlk < m_[f]; ++c) hchunks.push_back(make_int2(f, c));
       }
     }
     wave_nflags = flag_off[nn];
@@ -2168,6 +2181,7 @@ struct Numeric : NumericBase {
       q.l21p = wave_l21p.p + l21_off[f];
       q.binv = binv ? wave_binv.p + binv_off[f] : nullptr;
       q.hoff = hinv_first[f];
+      q.eoff = hinv_row0[f];
       q.nblk = nblk_of(f);
       q.ngat = ngat_of(f);
       q.nch = nch_of(f);
@@ -2213,7 +2227,7 @@ struct Numeric : NumericBase {
     mix((uint64_t)(uintptr_t)wave_items.p); mix((uint64_t)(uintptr_t)wave_flags.p);
     mix((uint64_t)(uintptr_t)wave_ints.p); mix((uint64_t)(uintptr_t)wave_l21p.p);
     mix((uint64_t)(uintptr_t)wave_binv.p); mix((uint64_t)binv);
-    mix((uint64_t)hblocks.empty());
+    mix((uint64_t)hblocks.size()); mix((uint64_t)hinv_rows);
     mix((uint64_t)wave_nfwd); mix((uint64_t)wave_nbwd);
     mix((uint64_t)(uintptr_t)S->d_front_group); mix((uint64_t)(uintptr_t)group_active.p);
     if (h != solve_sig) drop_graphs();
@@ -2272,8 +2286,9 @@ struct Numeric : NumericBase {
       if (hinv_ready || hinv_off || hblocks.empty()) return;
       const double* before = wave_hinv.p;
       try {
-        wave_hinv.ensure(hblocks.size() * 2 * 32 * 32);
-        hinv_blocks.ensure(hblocks.size());
+        wave_hinv.ensure(hblocks.size() * 2 * 32 * 32 +
+                         (hinv_rows * sizeof(int) + hblocks.size()) / sizeof(double) + 1);
+        hinv_blocks.ensure(hblocks.size() + hchunks.size());
       } catch (CudaFail const& e) {
         if (e.err != cudaErrorMemoryAllocation) throw;
         cudaGetLastError();
@@ -2284,7 +2299,10 @@ struct Numeric : NumericBase {
       if (hinv_off) return;
       CK(cudaMemcpyAsync(hinv_blocks.p, hblocks.data(), hblocks.size() * sizeof(int2),
                          cudaMemcpyHostToDevice, s));
-      launch_half_inv(d_sn, hinv_blocks.p, (int)hblocks.size(), wave_hinv.p, s);
+      CK(cudaMemcpyAsync(hinv_blocks.p + hblocks.size(), hchunks.data(),
+                         hchunks.size() * sizeof(int2), cudaMemcpyHostToDevice, s));
+      launch_half_inv(d_sn, hinv_blocks.p, (int)hblocks.size(), hinv_blocks.p + hblocks.size(),
+                      (int)hchunks.size(), wave_hinv.p, hinv_exps(), hinv_grown(), s);
       hinv_ready = true;
     }
   }
@@ -2695,6 +2713,7 @@ struct Numeric : NumericBase {
       }
       CK(cudaMemcpy(hfd[f].D, D.data(), D.size() * sizeof(double), cudaMemcpyHostToDevice));
     }
+    hinv_ready = false;  // their balance is D's
   }
 };
 

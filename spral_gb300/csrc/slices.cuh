@@ -12,6 +12,8 @@ namespace ssids300 {
 
 // exponent of a row with Inf or NaN: the products of the row become NaN
 constexpr int kSliceNonFinite = 1 << 19;
+// exponent of a row of zeros
+constexpr int kEmptyExponent = -(1 << 18);
 
 // biased exponent of an entry after its column's balance 2^h
 __device__ __forceinline__ int slice_exponent(unsigned long long bits, int h) {

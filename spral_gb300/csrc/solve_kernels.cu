@@ -203,10 +203,25 @@ __device__ __forceinline__ void solve_in_regs(int jb, const T* Lb, T (&x)[R][2])
 // is rounded once and added to an FP64 accumulator.  The diagonal block is
 // solved as two halves of 32 rows with their inverses (k_half_inv, once per
 // factorisation) and the product between them; those operands' digits are put
-// into shared memory as fragments before the waits too.  One or two columns
-// keep the multiply-adds: the digit work of a tile, padded to eight columns,
-// stays the same while theirs falls (at four columns the two passes of a
-// 6000-row saddle point gain 1.97 -> 1.60 ms only).
+// into shared memory as fragments before the waits too.
+//
+// What the digits cut off is 2^-62 of the largest entry of a tile row times the
+// largest value of a right-hand side.  Three rules keep that, entry by entry, at
+// what the multiply-adds lose.  (1) Entry k of the sum is balanced: L(r, k) is
+// multiplied by 2^h, its value divided by it (backward the other way round),
+// 2^h ~ sqrt|D_k| for a pivot, the largest |L sqrt|D|| of the row for a row
+// below the pivots (k_solve_scale).  So a diagonal scaling of the matrix, which
+// the unknowns follow, changes nothing.  (2) A sum more than 2^kSumGuard below
+// the product of those maxima is formed again with multiply-adds: a value far
+// below its neighbours (a right-hand side whose solution decays) keeps its
+// digits, and random values hardly ever get there.  (3) A pivot block whose
+// inverse has a balanced entry above 2^kHalfGrowth (threshold pivots allow
+// entries of L up to 1/u) is solved by substitution, its items take
+// fwd_block and bwd_block.
+//
+// One or two columns keep the multiply-adds: the digit work of a tile, padded
+// to eight columns, stays the same while theirs falls (at four columns the two
+// passes of a 6000-row saddle point gain 1.97 -> 1.60 ms only).
 // Bound by the chain of pivot blocks at the top of the tree (eight columns:
 // 10 us a block for flag, digits, products of one tile and of the diagonal
 // block; 19 us before) and by the FP64 pipe in the small items below it.
@@ -214,15 +229,21 @@ __device__ __forceinline__ void solve_in_regs(int jb, const T* Lb, T (&x)[R][2])
 // pass (fronts of 4 and more pivot blocks only: 4.3 and 5.0; of 2 and more:
 // 3.8 and 4.3).  Six matrices each of five kinds, 16 columns: errors 0.47 to
 // 0.86 of those of the multiply-adds, which round every product.
+// 48^3 Laplacian, 8 random columns, a solve: 3.29 ms with neither of the three,
+// 3.51 with (1) and (3), 3.64 with (2) as well (3.52 with kSumGuard 16; a
+// 6000-row saddle point, 4 columns: 1.30, 1.39, 1.59, 1.48).
+constexpr int kSumGuard = 12;
+constexpr int kHalfGrowth = 6;
 template <typename T, int NR>
 constexpr bool solve_mma() { return sizeof(T) == 8 && NR >= 4; }
 template <int NR>
 constexpr int mma_cols() { return (NR + 7) / 8 * 8; }  // right-hand sides, padded
 // shared memory of an item: the diagonal block's fragments (3 operands x 2
 // row tiles x 2 k steps x 8 digits x 512 bytes), row exponents, right-hand
-// side exponents, the block's values, the sums (also the values' digits)
+// side exponents, the balance of the block's values, the values, the sums (also
+// a half's digits and values)
 constexpr int kMmaFragBytes = 3 * 2 * 2 * 8 * 512;
-constexpr int kMmaHeadBytes = kMmaFragBytes + 3 * 32 * 4 + 16 * 4 + 64;
+constexpr int kMmaHeadBytes = kMmaFragBytes + 3 * 32 * 4 + 16 * 4 + 64 * 4;
 constexpr int MV = SB + 1;  // stride of the block's values
 template <int NR>
 constexpr size_t mma_smem_bytes() {
@@ -818,62 +839,89 @@ __device__ __forceinline__ void bwd_gather_rows(const SolveNode<T>& sn, const do
   }
 }
 
+// a product of a tile with the right-hand sides: entry (r, k) of the tile at
+// p[r * rs + k * ks], nr rows and nk columns; value k of right-hand side
+// q < nq at y[q * m + k]; the balance exponent of entry k at h[k]
+struct TileRef {
+  const double* p;
+  int64_t rs, ks;
+  int nr, nk, nq;
+  const double* y;
+  int64_t m;
+  const int* h;
+};
 struct TileDigits {
   unsigned d[2][2][8][2];  // [k step][row g or g + 8][digit][register]
   int e[2];                // row exponents
 };
-// tile entry (r, k) at p[r * rs + k * ks], zero past nr rows or nk columns
-// of the 16 rows from r0 and 32 columns from k0
-__device__ __forceinline__ void tile_digits(const double* p, int64_t rs, int64_t ks, int nr, int nk,
-                                            int r0, int k0, TileDigits& t) {
+// digits of the 16 rows from r0 and 32 columns from k0 of a tile, entry k times
+// 2^(sg h[k]) (k < nh, else unchanged)
+__device__ __forceinline__ void tile_digits(const TileRef& s, int r0, int k0, int sg, int nh,
+                                            TileDigits& t) {
   r0 += (threadIdx.x & 31) >> 2;
   k0 += (threadIdx.x & 3) * 2;
   unsigned long long v[2][2][4];
+  int h[2][4];
 #pragma unroll
-  for (int s = 0; s < 2; ++s)
+  for (int st = 0; st < 2; ++st)
 #pragma unroll
-    for (int u = 0; u < 2; ++u)
+    for (int q = 0; q < 4; ++q) {
+      const int k = k0 + 16 * st + (q & 1) + (q >> 1) * 8;
+      h[st][q] = k < nh ? sg * __ldg(s.h + k) : 0;
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int r = r0 + 8 * u, k = k0 + 16 * s + (q & 1) + (q >> 1) * 8;
-        v[s][u][q] = (r < nr && k < nk)
-                         ? (unsigned long long)__double_as_longlong(p[r * rs + k * ks]) : 0ULL;
+      for (int u = 0; u < 2; ++u) {
+        const int r = r0 + 8 * u;
+        v[st][u][q] = (r < s.nr && k < s.nk)
+                          ? (unsigned long long)__double_as_longlong(s.p[r * s.rs + k * s.ks])
+                          : 0ULL;
       }
+    }
 #pragma unroll
   for (int u = 0; u < 2; ++u) {
-    int e = -(1 << 18);
+    int e = kEmptyExponent;
 #pragma unroll
-    for (int s = 0; s < 2; ++s)
+    for (int st = 0; st < 2; ++st)
 #pragma unroll
       for (int q = 0; q < 4; ++q)
-        if ((v[s][u][q] << 1) != 0ULL) e = max(e, slice_exponent(v[s][u][q], 0));
+        if ((v[st][u][q] << 1) != 0ULL) e = max(e, slice_exponent(v[st][u][q], h[st][q]));
     e = max(e, __shfl_xor_sync(0xffffffffu, e, 1));
     e = max(e, __shfl_xor_sync(0xffffffffu, e, 2));
     t.e[u] = e;
-    const int h[4] = {0, 0, 0, 0};
 #pragma unroll
-    for (int s = 0; s < 2; ++s) slice_quad(v[s][u], h, e, t.d[s][u]);
+    for (int st = 0; st < 2; ++st) slice_quad(v[st][u], h[st], e, t.d[st][u]);
   }
 }
-// digits of 64 values of every right-hand side, value k of right-hand side q
-// at p[q * m + k] (another CTA's: read from L2): into yd, exponents into ey.
-// The caller's barriers separate it from the products.
+// this warp's share of a tile
+__device__ __forceinline__ void tile_digits(const TileRef& s, int sg, TileDigits& t) {
+  const int warp = threadIdx.x >> 5;
+  tile_digits(s, (warp & 3) * 16, (warp >> 2) * 32, sg, s.nk, t);
+}
+// the balance of this thread's values in rhs_digits
+__device__ __forceinline__ void rhs_balance(const TileRef& s, int sg, int (&h)[8]) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int k = (threadIdx.x & 7) * 8 + i;
+    h[i] = k < s.nk ? -sg * __ldg(s.h + k) : 0;
+  }
+}
+// digits of the 64 values of every right-hand side (another CTA's: read from
+// L2), balanced by h, into yd, exponents into ey.  The caller's barriers
+// separate it from the products.
 template <int NR>
-__device__ __forceinline__ void rhs_digits(const double* p, int64_t m, int nk, int nrhs, char* yd,
-                                           int* ey) {
+__device__ __forceinline__ void rhs_digits(const TileRef& s, const int (&h)[8], char* yd, int* ey) {
   constexpr int NP = mma_cols<NR>();
   static_assert(NP * 8 <= kSolveThreads, "a thread per right-hand side and 8 values");
   if ((int)threadIdx.x >= NP * 8) return;  // whole warps
   const int q = threadIdx.x >> 3, o = threadIdx.x & 7;
   unsigned long long v[8];
-  int e[8], em = -(1 << 18);
+  int e[8], em = kEmptyExponent;
 #pragma unroll
   for (int i = 0; i < 8; ++i)
-    v[i] = (q < nrhs && o * 8 + i < nk)
-               ? (unsigned long long)__double_as_longlong(__ldcg(p + q * m + o * 8 + i)) : 0ULL;
+    v[i] = (q < s.nq && o * 8 + i < s.nk)
+               ? (unsigned long long)__double_as_longlong(__ldcg(s.y + q * s.m + o * 8 + i)) : 0ULL;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    e[i] = slice_exponent(v[i], 0);
+    e[i] = slice_exponent(v[i], h[i]);
     if ((v[i] << 1) != 0ULL) em = max(em, e[i]);
   }
 #pragma unroll
@@ -881,10 +929,45 @@ __device__ __forceinline__ void rhs_digits(const double* p, int64_t m, int nk, i
   if (o == 0) ey[q] = em;
   slice_store(v, e, em, yd + o * (NP * 16) + q * 16, 8 * NP * 16);
 }
+// The sum of a tile row with exponent er and a right-hand side with exponent ec
+// from its levels; low: it is more than 2^kSumGuard below the product of the
+// largest entries, where the digits cut off may show, or one of those is not
+// finite (rows and right-hand sides of zeros alone are neither).
+__device__ __forceinline__ double digit_sum(const float (&v)[8], int er, int ec, bool& low) {
+  const double p = levels_to_double(v, slice_product_exponent(er, ec));
+  low = ((__double2hiint(p) >> 20) & 0x7ff) + kSumGuard < er + ec - 1023;
+  return p;
+}
+// The low sums of a warp with multiply-adds, term(l, x, k) the k-th of the 32
+// terms of lane l's sum x (0 past the end): the four lanes of a quad form its
+// lanes' sums one after the other, always in the same order, so that a sum does
+// not depend on the others.  Called by whole warps.
+template <typename Term>
+__device__ __forceinline__ void plain_sums(const bool (&low)[4], double (&p)[4], Term term) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int x = 0; x < 4; ++x) {
+    const unsigned who = __ballot_sync(0xffffffffu, low[x]);
+#pragma unroll 1
+    for (int j = 0; j < 4; ++j) {
+      if (!(who & (0x11111111u << j))) continue;
+      const int l = (lane & ~3) | j;
+      double v = 0.0;
+      if ((who >> l) & 1u) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v += term(l, x, (lane & 3) + 4 * i);
+      }
+      v += __shfl_xor_sync(0xffffffffu, v, 1);
+      v += __shfl_xor_sync(0xffffffffu, v, 2);
+      if (lane == l && low[x]) p[x] = v;
+    }
+  }
+}
 // acc += tile x right-hand sides: acc[nt][x] is row g + 8 (x / 2) of the warp's
 // 16, right-hand side 8 nt + 2 (lane % 4) + x % 2
 template <int NR>
-__device__ __forceinline__ void tile_product(const TileDigits& t, const char* yd, const int* ey,
+__device__ __forceinline__ void tile_product(const TileRef& src, const TileDigits& t,
+                                             const char* yd, const int* ey,
                                              double (&acc)[mma_cols<NR>() / 8][4]) {
   constexpr int NP = mma_cols<NR>();
   const int lane = threadIdx.x & 31, kh = threadIdx.x >> 7;
@@ -909,21 +992,25 @@ __device__ __forceinline__ void tile_product(const TileDigits& t, const char* yd
         }
       }
     }
+    double p[4];
+    bool low[4];
 #pragma unroll
     for (int x = 0; x < 4; ++x) {
       const float v[8] = {f[0][x], f[1][x], f[2][x], f[3][x], f[4][x], f[5][x], f[6][x], f[7][x]};
-      const int ec = ey[nt * 8 + (lane & 3) * 2 + (x & 1)];
-      double p = levels_to_double(v, slice_product_exponent(t.e[x >> 1], ec));
-      if (max(t.e[x >> 1], ec) >= kSliceNonFinite / 2) p = __longlong_as_double(0x7ff8000000000000LL);
-      acc[nt][x] += p;
+      p[x] = digit_sum(v, t.e[x >> 1], ey[nt * 8 + (lane & 3) * 2 + (x & 1)], low[x]);
     }
+    if (__any_sync(0xffffffffu, low[0] || low[1] || low[2] || low[3])) {
+      const int row0 = ((threadIdx.x >> 5) & 3) * 16, q0 = nt * 8, k0 = kh * 32;
+      plain_sums(low, p, [&](int l, int x, int k) {
+        const int row = row0 + (l >> 2) + 8 * (x >> 1), q = q0 + (l & 3) * 2 + (x & 1);
+        k += k0;
+        return row < src.nr && q < src.nq && k < src.nk
+                   ? src.p[row * src.rs + k * src.ks] * __ldcg(src.y + q * src.m + k) : 0.0;
+      });
+    }
+#pragma unroll
+    for (int x = 0; x < 4; ++x) acc[nt][x] += p[x];
   }
-}
-// this warp's share of a tile
-__device__ __forceinline__ void tile_digits(const double* p, int64_t rs, int64_t ks, int nr, int nk,
-                                            TileDigits& t) {
-  const int warp = threadIdx.x >> 5;
-  tile_digits(p, rs, ks, nr, nk, (warp & 3) * 16, (warp >> 2) * 32, t);
 }
 // the two column halves' sums into red[half][q][row]
 template <int NR>
@@ -944,65 +1031,99 @@ struct MmaSpace {  // an item's shared memory (kMmaHeadBytes)
   char* frag;
   int* fexp;
   int* ey;
+  int* hv;      // balance exponents of the block's 64 values
   double* vb;   // vb[q * MV + row]
   double* red;
   char* yd;     // in the sums' space
+  double* vc;   // a half's values, vc[q * 33 + row], after its digits
   __device__ explicit MmaSpace(void* base) {
     frag = static_cast<char*>(base);
     fexp = reinterpret_cast<int*>(frag + kMmaFragBytes);
     ey = fexp + 96;
+    hv = ey + 16;
     vb = reinterpret_cast<double*>(frag + kMmaHeadBytes);
     red = vb + (NR * MV + 1) / 2 * 2;
     yd = reinterpret_cast<char*>(red);
+    vc = red + 4 * 16 * mma_cols<NR>();  // (64 of the 128 columns of red)
   }
 };
 static_assert(kMmaHeadBytes % 16 == 0, "the digits of the values are 16-byte aligned");
 
-// The fragments of the three 32 x 32 operands of a diagonal block's solve
-// (rows and columns [c0, c0 + jb) of L; X: the inverses of its halves):
-// forward X_0, L_10, X_1, backward their transposes from the last.
+// The three 32 x 32 operands of a diagonal block's solve (rows and columns
+// [c0, c0 + jb) of L; X: the inverses of its halves): forward X_0, L_10, X_1,
+// backward their transposes from the last.  half_offset: the block's value that
+// their first column multiplies.
 template <bool TRANS>
-__device__ __forceinline__ void half_operands(const SolveNode<double>& sn, const double* X, int c0,
-                                              int jb, char* frag, int* fexp) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (warp >= 6) return;
-  const int mat = warp >> 1, rt = warp & 1;
-  TileDigits t;
+__device__ __forceinline__ int half_offset(int mat) {
+  return mat == 1 ? (TRANS ? 32 : 0) : ((mat == 2) != TRANS ? 32 : 0);
+}
+template <bool TRANS>
+__device__ __forceinline__ TileRef half_source(const SolveNode<double>& sn, const double* X, int c0,
+                                               int jb, int mat) {
+  TileRef s{};
   if (mat != 1) {
-    const double* p = X + (((mat == 2) != TRANS) ? 32 * 32 : 0);
-    tile_digits(p, TRANS ? 1 : 32, TRANS ? 32 : 1, 32, 32, rt * 16, 0, t);
+    s.p = X + half_offset<TRANS>(mat) * 32;
+    s.rs = TRANS ? 1 : 32;
+    s.ks = TRANS ? 32 : 1;
+    s.nr = s.nk = max(0, min(32, jb - half_offset<TRANS>(mat)));
   } else {
-    const double* p = sn.L + (int64_t)c0 * sn.ld + c0 + 32;
     const int n0 = min(jb, 32), n1 = jb - 32;
-    tile_digits(p, TRANS ? sn.ld : 1, TRANS ? 1 : sn.ld, TRANS ? n0 : n1, TRANS ? n1 : n0, rt * 16,
-                0, t);
+    s.p = sn.L + (int64_t)c0 * sn.ld + c0 + 32;
+    s.rs = TRANS ? sn.ld : 1;
+    s.ks = TRANS ? 1 : sn.ld;
+    s.nr = TRANS ? n0 : n1;
+    s.nk = TRANS ? n1 : n0;
   }
+  return s;
+}
+// their fragments, and the balance of the block's values
+template <bool TRANS>
+__device__ __forceinline__ void half_operands(const SolveNode<double>& sn, const double* X,
+                                              const int* h, int c0, int jb, char* frag, int* fexp,
+                                              int* hv) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (warp >= 6) {
+    const int k = threadIdx.x - 192;
+    hv[k] = k < jb ? (TRANS ? 1 : -1) * h[c0 + k] : 0;
+    return;
+  }
+  const int mat = warp >> 1, rt = warp & 1;
+  const int off = half_offset<TRANS>(mat);
+  TileRef s = half_source<TRANS>(sn, X, c0, jb, mat);
+  s.h = h + c0 + off;
+  TileDigits t;
+  tile_digits(s, rt * 16, 0, TRANS ? -1 : 1, jb - off, t);
 #pragma unroll
-  for (int s = 0; s < 2; ++s)
+  for (int st = 0; st < 2; ++st)
 #pragma unroll
     for (int i = 0; i < 8; ++i)
-      *reinterpret_cast<uint4*>(frag + ((warp * 2 + s) * 8 + i) * 512 + lane * 16) =
-          make_uint4(t.d[s][0][i][0], t.d[s][1][i][0], t.d[s][0][i][1], t.d[s][1][i][1]);
+      *reinterpret_cast<uint4*>(frag + ((warp * 2 + st) * 8 + i) * 512 + lane * 16) =
+          make_uint4(t.d[st][0][i][0], t.d[st][1][i][0], t.d[st][0][i][1], t.d[st][1][i][1]);
   if ((lane & 3) == 0) {
     fexp[warp * 16 + (lane >> 2)] = t.e[0];
     fexp[warp * 16 + 8 + (lane >> 2)] = t.e[1];
   }
 }
-// digits of half h of the block's values
+// digits of half h of the block's values, and the values beside them
 template <int NR>
 __device__ __forceinline__ void half_digits(const MmaSpace<NR>& sp, int h) {
   constexpr int NP = mma_cols<NR>();
   if ((int)threadIdx.x >= NP * 4) return;  // whole warps
   const int q = threadIdx.x >> 2, o = threadIdx.x & 3;
+  const int4* hp = reinterpret_cast<const int4*>(sp.hv + h * 32 + o * 8);
+  const int4 h0 = hp[0], h1 = hp[1];
+  const int hv[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
   unsigned long long v[8];
-  int e[8], em = -(1 << 18);
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-    v[i] = q < NR ? (unsigned long long)__double_as_longlong(sp.vb[q * MV + h * 32 + o * 8 + i])
-                  : 0ULL;
+  int e[8], em = kEmptyExponent;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    e[i] = slice_exponent(v[i], 0);
+    const double w = q < NR ? sp.vb[q * MV + h * 32 + o * 8 + i] : 0.0;
+    sp.vc[q * 33 + o * 8 + i] = w;
+    v[i] = (unsigned long long)__double_as_longlong(w);
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    e[i] = slice_exponent(v[i], hv[i]);
     if ((v[i] << 1) != 0ULL) em = max(em, e[i]);
   }
   em = max(em, __shfl_xor_sync(0xffffffffu, em, 1));
@@ -1010,9 +1131,11 @@ __device__ __forceinline__ void half_digits(const MmaSpace<NR>& sp, int h) {
   if (o == 0) sp.ey[q] = em;
   slice_store(v, e, em, sp.yd + o * (NP * 16) + q * 16, 4 * NP * 16);
 }
-// half h of the values = operand mat times the digits (sub: minus it)
-template <int NR>
-__device__ __forceinline__ void half_product(const MmaSpace<NR>& sp, int mat, int h, bool sub) {
+// half h of the values = operand mat (half_source) times the digits (sub: minus it)
+template <int NR, bool TRANS>
+__device__ __forceinline__ void half_product(const MmaSpace<NR>& sp, const SolveNode<double>& sn,
+                                             const double* X, int c0, int jb, int mat, int h,
+                                             bool sub) {
   constexpr int NP = mma_cols<NR>();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rt = warp & 1, nt = warp >> 1;
@@ -1038,57 +1161,127 @@ __device__ __forceinline__ void half_product(const MmaSpace<NR>& sp, int mat, in
       for (int j = 0; j < 8 - i; ++j) mma_f16(f[i + j], a, b[j]);
     }
   }
+  double p[4];
+  bool low[4];
+#pragma unroll
+  for (int x = 0; x < 4; ++x) {
+    const int row = rt * 16 + (lane >> 2) + 8 * (x >> 1), q = nt * 8 + (lane & 3) * 2 + (x & 1);
+    const float v[8] = {f[0][x], f[1][x], f[2][x], f[3][x], f[4][x], f[5][x], f[6][x], f[7][x]};
+    p[x] = digit_sum(v, sp.fexp[mat * 32 + row], sp.ey[q], low[x]);
+  }
+  if (__any_sync(0xffffffffu, low[0] || low[1] || low[2] || low[3])) {
+    const TileRef src = half_source<TRANS>(sn, X, c0, jb, mat);
+    plain_sums(low, p, [&](int l, int x, int k) {
+      const int row = rt * 16 + (l >> 2) + 8 * (x >> 1), q = nt * 8 + (l & 3) * 2 + (x & 1);
+      return row < src.nr && k < src.nk ? src.p[row * src.rs + k * src.ks] * sp.vc[q * 33 + k]
+                                        : 0.0;
+    });
+  }
 #pragma unroll
   for (int x = 0; x < 4; ++x) {
     const int row = rt * 16 + (lane >> 2) + 8 * (x >> 1), q = nt * 8 + (lane & 3) * 2 + (x & 1);
     if (q >= NR) continue;
-    const float v[8] = {f[0][x], f[1][x], f[2][x], f[3][x], f[4][x], f[5][x], f[6][x], f[7][x]};
-    const int er = sp.fexp[mat * 32 + row], ec = sp.ey[q];
-    double p = levels_to_double(v, slice_product_exponent(er, ec));
-    if (max(er, ec) >= kSliceNonFinite / 2) p = __longlong_as_double(0x7ff8000000000000LL);
     double& t = sp.vb[q * MV + h * 32 + row];
-    t = sub ? t - p : p;
+    t = sub ? t - p[x] : p[x];
   }
 }
-// the diagonal block's solve, from half `first` (0 forward, 1 backward) on
-template <int NR>
-__device__ __forceinline__ void half_solves(const MmaSpace<NR>& sp, int first) {
+// the diagonal block's solve: forward from half 0, backward from half 1
+template <int NR, bool TRANS>
+__device__ __forceinline__ void half_solves(const MmaSpace<NR>& sp, const SolveNode<double>& sn,
+                                            const double* X, int c0, int jb) {
+  constexpr int first = TRANS ? 1 : 0;
 #pragma unroll 1
   for (int st = 0; st < 3; ++st) {
     __syncthreads();
     half_digits<NR>(sp, st == 2 ? 1 - first : first);
     __syncthreads();
-    half_product<NR>(sp, st, st == 0 ? first : 1 - first, st == 1);
+    half_product<NR, TRANS>(sp, sn, X, c0, jb, st, st == 0 ? first : 1 - first, st == 1);
   }
   __syncthreads();
+}
+
+// Balance exponents of the fronts' rows for the products above, rows [64 w.y,
+// 64 w.y + 64) of front w.x = blocks[i].x: a pivot's from D^{-1}, another row's
+// the exponent of its largest |L(r, k)| 2^h_k (0 for a row of zeros).  Bound by
+// reading L21 once per factorisation.
+__global__ void __launch_bounds__(256) k_solve_scale(const SolveNode<double>* sns,
+                                                     const int2* blocks, int* out) {
+  constexpr int KC = 1024;
+  __shared__ short hs[KC];
+  __shared__ int em4[4][SB];
+  const int2 w = blocks[blockIdx.x];
+  const SolveNode<double>& sn = sns[w.x];
+  const int r = threadIdx.x & (SB - 1), g = threadIdx.x / SB;
+  const int row0 = w.y * SB, row = row0 + r, nelim = sn.nelim;
+  int* o = out + sn.eoff;
+  if (g == 0 && row < nelim) o[row] = slice_balance(sn.D, row, nelim);
+  if (row0 + SB <= nelim) return;
+  const bool mine = row >= nelim && row < sn.m;
+  int em = INT_MIN;
+  for (int kb = 0; kb < nelim; kb += KC) {
+    const int kn = min(KC, nelim - kb);
+    __syncthreads();
+    for (int k = threadIdx.x; k < kn; k += blockDim.x)
+      hs[k] = (short)slice_balance(sn.D, kb + k, nelim);
+    __syncthreads();
+    if (!mine) continue;
+    const double* p = sn.L + (int64_t)kb * sn.ld + row;
+    for (int k0 = g; k0 < kn; k0 += 32) {
+      unsigned long long v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int k = k0 + 4 * u;
+        v[u] = k < kn ? (unsigned long long)__double_as_longlong(p[(int64_t)k * sn.ld]) : 0ULL;
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if ((v[u] << 1) != 0ULL)
+          em = max(em, min((int)((v[u] >> 52) & 0x7ff), 0x7fe) - 1023 + hs[k0 + 4 * u]);
+    }
+  }
+  em4[g][r] = em;
+  __syncthreads();
+  if (g == 0 && mine) {
+    em = max(max(em4[0][r], em4[1][r]), max(em4[2][r], em4[3][r]));
+    o[row] = em == INT_MIN ? 0 : em;
+  }
 }
 
 // Inverses of the two 32 x 32 unit lower halves on the diagonal of pivot
 // block blocks[i] = (front, block) of the FP64 factors, row-major, into
 // X[hoff + block]; a warp per half, lane c column c by substitution (496
-// FP64 multiply-adds: 20 us, once per factorisation).
+// FP64 multiply-adds: 20 us, once per factorisation).  grown[hoff + block]: an
+// entry, balanced as the products are, is above 2^kHalfGrowth or not finite.
 __global__ void __launch_bounds__(64) k_half_inv(const SolveNode<double>* sns, const int2* blocks,
-                                                 double* X) {
+                                                 double* X, unsigned char* grown) {
   __shared__ double Ls[2][32][33];
   const int2 w = blocks[blockIdx.x];
   const SolveNode<double>& sn = sns[w.x];
-  const int h = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int c0 = w.y * SB + 32 * h, jb = sn.nelim - c0;  // rows left (may be <= 0)
+  const int half = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int c0 = w.y * SB + 32 * half, jb = sn.nelim - c0;  // rows left (may be <= 0)
   for (int c = 0; c < 32; ++c)
-    Ls[h][lane][c] =
+    Ls[half][lane][c] =
         (lane > c && lane < jb) ? sn.L[(int64_t)(c0 + c) * sn.ld + c0 + lane] : 0.0;
+  const int h = lane < jb ? slice_balance(sn.D, c0 + lane, sn.nelim) : 0;
   __syncwarp();
   double x[32];
 #pragma unroll
   for (int i = 0; i < 32; ++i) {
     double acc = i == lane ? 1.0 : 0.0;
 #pragma unroll
-    for (int k = 0; k < i; ++k) acc -= Ls[h][i][k] * x[k];
+    for (int k = 0; k < i; ++k) acc -= Ls[half][i][k] * x[k];
     x[i] = acc;
   }
-  double* out = X + ((size_t)(sn.hoff + w.y) * 2 + h) * 32 * 32;
+  double* out = X + ((size_t)(sn.hoff + w.y) * 2 + half) * 32 * 32;
+  bool big = false;
 #pragma unroll
-  for (int i = 0; i < 32; ++i) out[i * 32 + lane] = x[i];
+  for (int i = 0; i < 32; ++i) {
+    out[i * 32 + lane] = x[i];
+    const int e = (__double2hiint(x[i]) >> 20) & 0x7ff, hi = __shfl_sync(0xffffffffu, h, i);
+    if (e == 0x7ff || e - 1023 + h - hi >= kHalfGrowth) big = true;
+  }
+  const int any = __syncthreads_or(big);
+  if (threadIdx.x == 0) grown[sn.hoff + w.y] = any ? 1 : 0;
 }
 
 // fwd_block on the tensor cores
@@ -1110,18 +1303,22 @@ __device__ bool fwd_block_mma(const SolveNode<double>& sn, int code, int nrhs, d
     const int q = q0 + 4 * k;
     own[k] = (row < rows && q < nrhs) ? __ldcg(&sn.xloc[(int64_t)q * m + r0 + row]) : 0.0;
   }
-  if (piv)
-    half_operands<false>(sn, wl.hinv + (size_t)(sn.hoff + code) * 2 * 32 * 32, r0, rows, sp.frag,
-                         sp.fexp);
+  const int* h = wl.hexp + sn.eoff;
+  const double* X = wl.hinv + (size_t)(sn.hoff + code) * 2 * 32 * 32;  // (a pivot block's)
+  if (piv) half_operands<false>(sn, X, h, r0, rows, sp.frag, sp.fexp, sp.hv);
   double acc[mma_cols<NR>() / 8][4] = {};
   for (int j = 0; j < ncb; ++j) {
     const int c0 = j * SB, jb = min(SB, nelim - c0);
+    const TileRef src{sn.L + (int64_t)c0 * sn.ld + r0, 1, sn.ld, rows, jb, nrhs, sn.xloc + c0, m,
+                      h + c0};
     TileDigits td;
-    tile_digits(sn.L + (int64_t)c0 * sn.ld + r0, 1, sn.ld, rows, jb, td);
+    int hy[8];
+    tile_digits(src, 1, td);
+    rhs_balance(src, 1, hy);
     if (!wave_wait(&sn.flag[j], status, s_fail)) return false;
-    rhs_digits<NR>(sn.xloc + c0, m, jb, nrhs, sp.yd, sp.ey);
+    rhs_digits<NR>(src, hy, sp.yd, sp.ey);
     __syncthreads();
-    tile_product<NR>(td, sp.yd, sp.ey, acc);
+    tile_product<NR>(src, td, sp.yd, sp.ey, acc);
     __syncthreads();
   }
   wave_stamp(wl, it, 1);
@@ -1135,7 +1332,7 @@ __device__ bool fwd_block_mma(const SolveNode<double>& sn, int code, int nrhs, d
     else if (row < rows && q < nrhs) sn.xloc[(int64_t)q * m + r0 + row] = own[k];
   }
   if (!piv) return true;
-  half_solves<NR>(sp, 0);
+  half_solves<NR, false>(sp, sn, X, r0, rows);
 #pragma unroll
   for (int k = 0; k < E; ++k) {
     const int q = q0 + 4 * k;
@@ -1153,19 +1350,23 @@ __device__ bool fwd_block_mma(const SolveNode<double>& sn, int code, int nrhs, d
 
 // bwd_l21_item on the tensor cores
 template <int NR>
-__device__ void bwd_l21_mma(const SolveNode<double>& sn, int t, int nrhs, void* base) {
+__device__ void bwd_l21_mma(const SolveNode<double>& sn, int t, int nrhs, void* base,
+                            const WaveLevel& wl) {
   const MmaSpace<NR> sp(base);
   const int m = sn.m, b = t / sn.nch, c = t - b * sn.nch;
   const int c0 = b * SB, jb = min(SB, sn.nelim - c0);
   const int R0 = sn.nelim + c * kWaveL21Rows, nr = min(kWaveL21Rows, m - R0);
   double acc[mma_cols<NR>() / 8][4] = {};
   for (int k0 = 0; k0 < nr; k0 += SB) {
-    const int nk = min(SB, nr - k0);
+    const TileRef src{sn.L + (int64_t)c0 * sn.ld + R0 + k0, sn.ld, 1, jb, min(SB, nr - k0), nrhs,
+                      sn.xloc + R0 + k0, m, wl.hexp + sn.eoff + R0 + k0};
     TileDigits td;
-    tile_digits(sn.L + (int64_t)c0 * sn.ld + R0 + k0, sn.ld, 1, jb, nk, td);
-    rhs_digits<NR>(sn.xloc + R0 + k0, m, nk, nrhs, sp.yd, sp.ey);
+    int hy[8];
+    tile_digits(src, -1, td);
+    rhs_balance(src, -1, hy);
+    rhs_digits<NR>(src, hy, sp.yd, sp.ey);
     __syncthreads();
-    tile_product<NR>(td, sp.yd, sp.ey, acc);
+    tile_product<NR>(src, td, sp.yd, sp.ey, acc);
     __syncthreads();
   }
   tile_sums<NR>(acc, sp.red);
@@ -1193,7 +1394,9 @@ __device__ bool bwd_block_mma(const SolveNode<double>& sn, int b, int nrhs, doub
     const int q = q0 + 4 * k;
     own[k] = (col < jb && q < nrhs) ? __ldcg(&sn.xloc[(int64_t)q * m + c0 + col]) : 0.0;
   }
-  half_operands<true>(sn, wl.hinv + (size_t)(sn.hoff + b) * 2 * 32 * 32, c0, jb, sp.frag, sp.fexp);
+  const int* h = wl.hexp + sn.eoff;
+  const double* X = wl.hinv + (size_t)(sn.hoff + b) * 2 * 32 * 32;
+  half_operands<true>(sn, X, h, c0, jb, sp.frag, sp.fexp, sp.hv);
   if (sn.nch > 0 && !wave_wait_count(wave_l21done(sn, b), sn.nch, status, s_fail)) return false;
   const double* pp = sn.l21p + (size_t)b * sn.nch * SB * kSolveRhs;
   for (int e = tid; e < SB * NR; e += kSolveThreads) {
@@ -1205,13 +1408,17 @@ __device__ bool bwd_block_mma(const SolveNode<double>& sn, int b, int nrhs, doub
   }
   double acc[mma_cols<NR>() / 8][4] = {};
   for (int j = sn.nblk - 1; j > b; --j) {
-    const int R0 = j * SB, nr = min(SB, nelim - R0);
+    const int R0 = j * SB;
+    const TileRef src{sn.L + (int64_t)c0 * sn.ld + R0, sn.ld, 1, jb, min(SB, nelim - R0), nrhs,
+                      sn.xloc + R0, m, h + R0};
     TileDigits td;
-    tile_digits(sn.L + (int64_t)c0 * sn.ld + R0, sn.ld, 1, jb, nr, td);
+    int hy[8];
+    tile_digits(src, -1, td);
+    rhs_balance(src, -1, hy);
     if (!wave_wait(&sn.flag[j], status, s_fail)) return false;
-    rhs_digits<NR>(sn.xloc + R0, m, nr, nrhs, sp.yd, sp.ey);
+    rhs_digits<NR>(src, hy, sp.yd, sp.ey);
     __syncthreads();
-    tile_product<NR>(td, sp.yd, sp.ey, acc);
+    tile_product<NR>(src, td, sp.yd, sp.ey, acc);
     __syncthreads();
   }
   wave_stamp(wl, it, 1);
@@ -1223,7 +1430,7 @@ __device__ bool bwd_block_mma(const SolveNode<double>& sn, int b, int nrhs, doub
     double& v = sp.vb[q * MV + col];
     v = own[k] - (v + sp.red[q * SB + col] + sp.red[(NR + q) * SB + col]);
   }
-  half_solves<NR>(sp, 1);
+  half_solves<NR, true>(sp, sn, X, c0, jb);
 #pragma unroll
   for (int k = 0; k < E; ++k) {
     const int q = q0 + 4 * k;
@@ -1687,7 +1894,7 @@ __global__ void __launch_bounds__(kSolveThreads, CPS)
       if (ok) {
         bool done = false;
         if constexpr (solve_mma<T, NR>()) {
-          if (wl.hinv && sn.hoff >= 0) {
+          if (wl.hinv && sn.hoff >= 0 && !(code < kWaveContrib && wl.grown[sn.hoff + code])) {
             ok = fwd_block_mma<NR>(sn, code, nrhs, x, ldx, scale_sqrt, status, solve_smem, &s_fail,
                                    wl, it);
             done = true;
@@ -2188,7 +2395,7 @@ __global__ void __launch_bounds__(kSolveThreads, CPS)
         bool done = false;
         if constexpr (solve_mma<T, NR>()) {
           if (wl.hinv && sn.hoff >= 0) {
-            bwd_l21_mma<NR>(sn, t, nrhs, solve_smem);
+            bwd_l21_mma<NR>(sn, t, nrhs, solve_smem, wl);
             done = true;
           }
         }
@@ -2212,7 +2419,7 @@ __global__ void __launch_bounds__(kSolveThreads, CPS)
       if (ok) {
         bool done = false;
         if constexpr (solve_mma<T, NR>()) {
-          if (wl.hinv && sn.hoff >= 0) {
+          if (wl.hinv && sn.hoff >= 0 && !wl.grown[sn.hoff + code]) {
             ok = bwd_block_mma<NR>(sn, code, nrhs, x, ldx, status, solve_smem, &s_fail, wl, it);
             done = true;
           }
@@ -2414,11 +2621,13 @@ void launch_diag_inv(const SolveNode<T>* sn, const int2* blocks, int nblocks, cu
   }
 }
 
-void launch_half_inv(const SolveNode<double>* sn, const int2* blocks, int nblocks, double* X,
+void launch_half_inv(const SolveNode<double>* sn, const int2* blocks, int nblocks,
+                     const int2* rows, int nrows, double* X, int* h, unsigned char* grown,
                      cudaStream_t s) {
   if (nblocks <= 0) return;
-  k_half_inv<<<nblocks, 64, 0, s>>>(sn, blocks, X);
-  note_launches(1);
+  k_half_inv<<<nblocks, 64, 0, s>>>(sn, blocks, X, grown);
+  k_solve_scale<<<nrows, 256, 0, s>>>(sn, rows, h);
+  note_launches(2);
 }
 
 template <typename T>

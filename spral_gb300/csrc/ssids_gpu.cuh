@@ -324,6 +324,7 @@ struct SolveNode {
   int nitf, nitb;    // items of the forward and of the backward pass
   int parent;        // front index of the parent, -1 at a root
   int64_t hoff;      // first pivot block in WaveLevel::hinv, -1: none
+  int64_t eoff;      // first row in WaveLevel::hexp (hoff >= 0)
 };
 
 // Wavefront solves: one persistent launch per pass over the whole tree.
@@ -378,6 +379,10 @@ struct WaveLevel {
   // unit lower halves on the diagonal of the pivot blocks of the fronts that
   // are not one small item (SolveNode::hoff), [block][half][32][32]; or nullptr
   const double* hinv;
+  // with hinv: the balance exponents of those fronts' rows (SolveNode::eoff),
+  // and per pivot block whether its inverses are too large to multiply by
+  const int* hexp;
+  const unsigned char* grown;
 };
 
 constexpr int kSolveBlk = 64;   // diagonal block of the blocked triangular solves
@@ -416,10 +421,14 @@ void launch_bwd_tree(const SolveNode<T>* sn, const WaveLevel& wl, double* x, int
                      int diag_mode, int* status, cudaStream_t s);
 // the inverses of the 64 x 64 unit lower diagonal blocks blocks[i] =
 // (front, block) into each front's SolveNode::binv
-void launch_half_inv(const SolveNode<double>* sn, const int2* blocks, int nblocks, double* X,
-                     cudaStream_t s);
 template <typename T>
 void launch_diag_inv(const SolveNode<T>* sn, const int2* blocks, int nblocks, cudaStream_t s);
+// what WaveLevel holds for FP64 factors: hinv and grown of the pivot blocks
+// blocks[i] = (front, block), hexp of the rows [64 c, 64 c + 64) of rows[i] =
+// (front, c)
+void launch_half_inv(const SolveNode<double>* sn, const int2* blocks, int nblocks,
+                     const int2* rows, int nrows, double* X, int* h, unsigned char* grown,
+                     cudaStream_t s);
 // failure-detection probe of the wavefront solves' bounded flag wait
 // (solve_kernels.cu): -51 when the wait gave up
 int wave_timeout_probe(int rounds);

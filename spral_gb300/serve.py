@@ -74,8 +74,9 @@ def estimate_bytes(akeep, precision=ssids.PRECISION_FP64, nrhs=1):
         # or the largest front alone
         sl = 32 * (cm + 128) * np.minimum(ncol, 2048)
         work += max(sl.max(), min(sl.sum(), 256 << 20))
-        # inverses of the diagonal half blocks (passes of several columns)
-        work += 16384 * ((ncol + 63) // 64).sum()
+        # inverses of the diagonal half blocks and the rows' balance exponents
+        # (passes of several columns)
+        work += 16384 * ((ncol + 63) // 64).sum() + 4 * nrow.sum()
     solve = 4 * akeep.n * max(nrhs, 16) * 8
     return int(factors + contrib + work + solve + (192 << 20))
 
