@@ -2362,19 +2362,36 @@ __global__ void __launch_bounds__(kTppTallThreads) k_tpp(FrontDesc<T>* fds, Fron
 // launch, an LD launch and a contribution launch, and small fronts run many
 // CTAs per SM (the tiny class launches one warp per CTA).
 // ------------------------------------------------------------------------
+// alpha = x / det, beta = -b / det of the 2x2 block with determinant det = x y -
+// b^2: by the reciprocal where that is a normal number, else from the block
+// scaled by its largest entry (pivots of some 1e154: det is a denormal number,
+// its reciprocal infinite)
+__device__ __forceinline__ void two_by_two_column(double x, double b, double y, double& alpha,
+                                                  double& beta) {
+  const double det = x * y - b * b;
+  const int e = (__double2hiint(det) >> 20) & 0x7ff;
+  if (e > 64 && e < 1982) {
+    const double r = recip_nr(det);
+    alpha = x * r;
+    beta = -b * r;
+  } else {
+    const double m = 1.0 / tpps::max_mag(x, tpps::max_mag(b, y)), xs = x * m, bs = b * m;
+    const double d = xs * y - bs * b;
+    alpha = xs / d;
+    beta = -bs / d;
+  }
+}
 // (alpha, beta, partner) of eliminated column c: column c of D = (D^{-1})^{-1}
 // is alpha e_c + beta e_partner (1x1: partner = c, beta = 0)
 __device__ __forceinline__ void d_column(const double* D, int c, int nel, double& alpha,
                                          double& beta, int& partner) {
   const double d11 = D[2 * c];
   if (isinf(d11)) {  // second column of a 2x2
-    const double a = D[2 * (c - 1)], b = D[2 * (c - 1) + 1], d = D[2 * c + 1];
-    const double rdet = recip_nr(a * d - b * b);
-    alpha = a * rdet; beta = -b * rdet; partner = c - 1;
+    two_by_two_column(D[2 * (c - 1)], D[2 * (c - 1) + 1], D[2 * c + 1], alpha, beta);
+    partner = c - 1;
   } else if (c + 1 < nel && isinf(D[2 * c + 2])) {  // first column of a 2x2
-    const double b = D[2 * c + 1], d = D[2 * c + 3];
-    const double rdet = recip_nr(d11 * d - b * b);
-    alpha = d * rdet; beta = -b * rdet; partner = c + 1;
+    two_by_two_column(D[2 * c + 3], D[2 * c + 1], d11, alpha, beta);
+    partner = c + 1;
   } else {
     alpha = (d11 != 0.0) ? recip_nr(d11) : 0.0; beta = 0.0; partner = c;
   }

@@ -1,0 +1,25 @@
+"""Fronts of small leaf subtrees at the ends of the FP64 range and beyond the
+sizes that the default subtree rule gives them."""
+import numpy as np
+import pytest
+
+from spral_gb300 import matrices as M, ssids
+from test_gpu_tpp_search import _saddles
+
+pytestmark = pytest.mark.gpu
+
+
+# 2^0: the fast reciprocals; 2^505: outside their range; 2^525 and 2^-525: the
+# determinant of a 2x2 pivot's inverse is a denormal number, or overflows
+@pytest.mark.parametrize("e", [0, 505, 525, -525])
+def test_gpu_two_by_two_pivots_at_the_ends_of_the_range(e):
+    p, r, v = _saddles(3, 40, 15, 20, seed=1)
+    n = len(p) - 1
+    ak = ssids.analyse(p, r, np.arange(n, dtype=np.int32))
+    b = M.sym_matvec(p, r, v, np.random.default_rng(2).standard_normal((n, 2)))
+    fk, inf = ssids.factor(ak, np.ldexp(v, e), ssids.Options(small=1e-300))
+    assert inf.num_two > 0
+    x = fk.solve(b)
+    # x 2^e solves the matrix with right-hand side b: the fixtures' bound
+    assert M.scaled_bwd_error(p, r, v, np.ldexp(x, e), b).max() <= 5e-14
+    fk.free()
