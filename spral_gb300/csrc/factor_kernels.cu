@@ -274,8 +274,8 @@ __global__ void __launch_bounds__(kDiagThreads) k_app_diag(FrontDesc<T>* fds, Fr
       if (POSDEF) {
         i1 = q;  // no pivoting
         if (!((double)blk[q][q] > 0.0)) pivsiz = -1;
-      } else if (kF64 ? ((gk & 0x7fffffffffffffffULL) | 0x3ffULL) <
-                             (unsigned long long)__double_as_longlong(small)
+      } else if (kF64 ? (long long)((gk & 0x7fffffffffffffffULL) | 0x3ffULL) <
+                             __double_as_longlong(small)  // (signed: no entry is below -0.0)
                       : bv < small) {
         pivsiz = 0;
       } else if (bi != bj) {

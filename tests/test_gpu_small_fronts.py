@@ -23,3 +23,18 @@ def test_gpu_two_by_two_pivots_at_the_ends_of_the_range(e):
     # x 2^e solves the matrix with right-hand side b: the fixtures' bound
     assert M.scaled_bwd_error(p, r, v, np.ldexp(x, e), b).max() <= 5e-14
     fk.free()
+
+
+def test_gpu_zero_threshold_of_either_sign():
+    """small = -0.0 finds no entry below it, as small = 0.0."""
+    k = 12
+    p, r, v = M.laplacian_3d(k, shift=-0.3)
+    ak = ssids.analyse(p, r, M.nd_order_grid(k, k, k))
+    b = np.random.default_rng(1).standard_normal(k ** 3)
+    xs = []
+    for small in (0.0, -0.0):
+        fk, inf = ssids.factor(ak, v, ssids.Options(small=small))
+        assert (inf.flag, inf.matrix_rank) == (0, k ** 3)
+        xs.append(fk.solve(b))
+        fk.free()
+    assert np.array_equal(xs[0], xs[1])
