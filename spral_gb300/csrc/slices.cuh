@@ -21,17 +21,32 @@ __device__ __forceinline__ int slice_exponent(unsigned long long bits, int h) {
   return e == 0x7ff ? kSliceNonFinite : max(e, 1) + h;
 }
 
-// Column balance 2^h ~ sqrt|D| of pivot column c from D^{-1}: a 1x1 pivot by
-// its entry, a 2x2 pivot by its off-diagonal entry (exponents only); dlast
-// ends the pivots.
+// exponent of |v|, far below all others for a zero
+__device__ __forceinline__ int slice_log2(double v) {
+  const int e = (int)(((unsigned)__double2hiint(v) >> 20) & 0x7ff);
+  return e ? e - 1023 : -4096;
+}
+// Column balance 2^h of pivot column c from D^{-1} (dlast ends the pivots), h
+// half the exponent of the largest entry in the column of D, so that the
+// columns of L 2^h and of L D 2^-h are of one size: 1 / d of a 1x1 pivot; of a
+// 2x2 pivot with D^{-1} = [a b; b d], det = a d - b^2, the larger of d / det (a /
+// det in its second column) and b / det, by exponents: no 2x2 pivot's det is
+// much smaller than the larger of its products.  (The off-diagonal entry alone
+// is no measure: threshold pivoting takes 2x2 pivots with any entry there.)
 __device__ __forceinline__ int slice_balance(const double* D, int c, int dlast) {
-  const unsigned long long inf = 0x7ff0000000000000ULL;
-  unsigned long long v = (unsigned long long)__double_as_longlong(D[2 * c]);
-  if (v == inf) v = (unsigned long long)__double_as_longlong(D[2 * c - 1]);
-  else if (c + 1 < dlast && (unsigned long long)__double_as_longlong(D[2 * c + 2]) == inf)
-    v = (unsigned long long)__double_as_longlong(D[2 * c + 1]);
-  const int e = (int)((v >> 52) & 0x7ff);
-  return (e > 0 && e < 0x7ff) ? (1023 - e) >> 1 : 0;
+  const long long inf = 0x7ff0000000000000LL;
+  // all loads at once
+  const double v0 = D[2 * c], v1 = D[2 * c + 1];
+  const double p0 = c > 0 ? D[2 * c - 2] : 0.0, p1 = c > 0 ? D[2 * c - 1] : 0.0;
+  const double n0 = c + 1 < dlast ? D[2 * c + 2] : 0.0, n1 = c + 1 < dlast ? D[2 * c + 3] : 0.0;
+  const bool second = __double_as_longlong(v0) == inf;
+  int h = -slice_log2(v0);
+  if (second || __double_as_longlong(n0) == inf) {
+    const int a = slice_log2(second ? p0 : v0), b = slice_log2(second ? p1 : v1);
+    const int d = slice_log2(second ? v1 : n1);
+    h = max(second ? a : d, b) - max(a + d, 2 * b);
+  }
+  return h > -2048 && h < 2048 ? h >> 1 : 0;
 }
 
 // The eight balanced digits of an entry (exponent e after the balance, row

@@ -38,3 +38,37 @@ def test_gpu_zero_threshold_of_either_sign():
         xs.append(fk.solve(b))
         fk.free()
     assert np.array_equal(xs[0], xs[1])
+
+
+@pytest.mark.parametrize("tiny", [0.0, 1e-12, 1e-30, 1e-90])
+@pytest.mark.parametrize("nrhs", [1, 4])
+def test_gpu_two_by_two_pivots_of_any_off_diagonal_entry(tiny, nrhs):
+    """Pairs of columns coupled by a tiny entry, or by 0.5, and by nothing else: the pivot search
+    takes them as 2x2 pivots (the 2x2 test comes first and asks nothing of that
+    entry), whose contribution has to keep its digits whatever its size."""
+    w, border = 40, 30
+    rng = np.random.default_rng(3)
+    n = 2 * w + border
+    ptr, row, val = [0], [], []
+    for j in range(n):
+        b, k = divmod(j, w)
+        rows = np.arange(j, n) if j >= 2 * w else np.concatenate(
+            [np.arange(j, (b + 1) * w), np.arange(2 * w, n)])
+        vals = rng.uniform(-1, 1, len(rows))
+        vals[0] = rng.uniform(1, 2) * (n if j >= 2 * w else 10)
+        if j < 2 * w:
+            vals[1:w - k] = 0.0
+            if k % 2 == 0:  # pairs of either kind, which share a row's digits
+                vals[1] = tiny if k % 4 == 0 else 0.5
+        row.append(rows.astype(np.int32))
+        val.append(vals)
+        ptr.append(ptr[-1] + len(rows))
+    p, r, v = np.array(ptr, np.int64), np.concatenate(row), np.concatenate(val)
+    ak = ssids.analyse(p, r, np.arange(n, dtype=np.int32))
+    fk, inf = ssids.factor(ak, v)
+    assert inf.flag == 0 and inf.num_two >= 2 * w // 2
+    x0 = rng.standard_normal((n, nrhs))
+    b = M.sym_matvec(p, r, v, x0)
+    # a diagonally dominant matrix: rounding, n terms a sum
+    assert M.scaled_bwd_error(p, r, v, fk.solve(b), b).max() <= n * 2.0 ** -52
+    fk.free()
