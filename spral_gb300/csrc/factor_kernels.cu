@@ -2590,7 +2590,9 @@ __global__ void __launch_bounds__(kTppThreads) k_tpp_level(FrontDesc<T>* fds, Fr
 // ------------------------------------------------------------------------
 constexpr int kSmallContribThreads = 128;
 
-constexpr int kSmallBalance = 512;  // balanced columns of a front; later ones keep their scale
+// a front's balance exponents held in shared memory (the default subtree rule
+// allows some 220 columns; those of larger fronts are formed where they are used)
+constexpr int kSmallBalance = 512;
 
 __global__ void __launch_bounds__(kSmallContribThreads, 2)
     k_small_contrib_f64(FrontDesc<double>* fds, const FrontState* sts, const int* fronts) {
@@ -2641,7 +2643,7 @@ __global__ void __launch_bounds__(kSmallContribThreads, 2)
 #pragma unroll
       for (int q = 0; q < 8; ++q) {
         const int k = k0 + (q >> 2) * 16 + t2 + (q & 1) + ((q >> 1) & 1) * 8;
-        h[q] = k < min(nel, kSmallBalance) ? hs[k] : 0;
+        h[q] = k >= nel ? 0 : k < kSmallBalance ? hs[k] : slice_balance(fd.D, k, nel);
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
           if ((a[u][q] << 1) != 0) er[u] = max(er[u], slice_exponent(a[u][q], h[q]));

@@ -40,13 +40,9 @@ def test_gpu_zero_threshold_of_either_sign():
     assert np.array_equal(xs[0], xs[1])
 
 
-@pytest.mark.parametrize("tiny", [0.0, 1e-12, 1e-30, 1e-90])
-@pytest.mark.parametrize("nrhs", [1, 4])
-def test_gpu_two_by_two_pivots_of_any_off_diagonal_entry(tiny, nrhs):
-    """Pairs of columns coupled by a tiny entry, or by 0.5, and by nothing else: the pivot search
-    takes them as 2x2 pivots (the 2x2 test comes first and asks nothing of that
-    entry), whose contribution has to keep its digits whatever its size."""
-    w, border = 40, 30
+def _pairs(w, border, tiny):
+    """Two blocks of w columns under a border, diagonally dominant: in a block,
+    pairs of columns are coupled by `tiny` and by 0.5 in turn."""
     rng = np.random.default_rng(3)
     n = 2 * w + border
     ptr, row, val = [0], [], []
@@ -58,17 +54,55 @@ def test_gpu_two_by_two_pivots_of_any_off_diagonal_entry(tiny, nrhs):
         vals[0] = rng.uniform(1, 2) * (n if j >= 2 * w else 10)
         if j < 2 * w:
             vals[1:w - k] = 0.0
-            if k % 2 == 0:  # pairs of either kind, which share a row's digits
+            if k % 2 == 0:
                 vals[1] = tiny if k % 4 == 0 else 0.5
         row.append(rows.astype(np.int32))
         val.append(vals)
         ptr.append(ptr[-1] + len(rows))
-    p, r, v = np.array(ptr, np.int64), np.concatenate(row), np.concatenate(val)
+    return np.array(ptr, np.int64), np.concatenate(row), np.concatenate(val)
+
+
+@pytest.mark.parametrize("tiny", [0.0, 1e-12, 1e-30, 1e-90])
+@pytest.mark.parametrize("nrhs", [1, 4])
+def test_gpu_two_by_two_pivots_of_any_off_diagonal_entry(tiny, nrhs):
+    """Pairs of columns coupled by a tiny entry, or by 0.5, and by nothing else: the pivot search
+    takes them as 2x2 pivots (the 2x2 test comes first and asks nothing of that
+    entry), whose contribution has to keep its digits whatever its size."""
+    p, r, v = _pairs(40, 30, tiny)
+    n = len(p) - 1
     ak = ssids.analyse(p, r, np.arange(n, dtype=np.int32))
     fk, inf = ssids.factor(ak, v)
-    assert inf.flag == 0 and inf.num_two >= 2 * w // 2
-    x0 = rng.standard_normal((n, nrhs))
-    b = M.sym_matvec(p, r, v, x0)
+    assert inf.flag == 0 and inf.num_two >= 40
+    b = M.sym_matvec(p, r, v, np.random.default_rng(4).standard_normal((n, nrhs)))
     # a diagonally dominant matrix: rounding, n terms a sum
     assert M.scaled_bwd_error(p, r, v, fk.solve(b), b).max() <= n * 2.0 ** -52
+    fk.free()
+
+
+def test_gpu_balance_of_a_small_subtree_front_of_many_columns():
+    """560 columns in a front that the caller's subtree rule makes a small one,
+    pairs of the last ones scaled by 2^30 and 2^-30 in turn: its contribution
+    keeps the border's entries."""
+
+    class Wide(ssids.Options):
+        def cpu_options(self):
+            c = super().cpu_options()
+            c.small_subtree_threshold = 10 ** 9
+            return c
+
+    w = 560
+    p, r, v = _pairs(w, 30, 0.25)
+    n = len(p) - 1
+    s = np.ones(n)
+    for b in range(2):
+        s[b * w + 512:(b + 1) * w] = np.ldexp(1.0, np.where(np.arange(w - 512) % 4 < 2, 30, -30))
+    b = M.sym_matvec(p, r, v, np.random.default_rng(5).standard_normal((n, 2)))
+    ak = ssids.analyse(p, r, np.arange(n, dtype=np.int32))
+    cols = np.repeat(np.arange(n), np.diff(p))
+    # a threshold that takes the scaled columns (pairs by themselves) in any order
+    fk, inf = ssids.factor(ak, v * s[r] * s[cols], Wide(u=1e-13))
+    assert (inf.flag, inf.num_neg, inf.num_delay) == (0, 0, 0)
+    x = s[:, None] * fk.solve(s[:, None] * b)
+    # the unscaled matrix is diagonally dominant: rounding, n terms a sum
+    assert M.scaled_bwd_error(p, r, v, x, b).max() <= n * 2.0 ** -52
     fk.free()
