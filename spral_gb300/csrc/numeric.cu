@@ -988,16 +988,27 @@ struct Numeric : NumericBase {
     w.nitems = fwd ? wave_nfwd : wave_nbwd;
     w.counter = wave_ints.p + (fwd ? 1 : 2);
     w.trace = nullptr;
-    // many small-front items: more CTAs in flight; otherwise the widest
-    // fronts' chains set the time and keep their registers
-    // (FP64 tensor-core items spill in the registers of three: they keep two
-    // unless they are a few among many small ones.  A 6000-row saddle point,
-    // 4 columns: forward and backward 1.60 ms with two, 1.82 ms with three)
     w.hinv = q > 2 && hinv_ready ? wave_hinv.p : nullptr;
     w.hexp = w.hinv ? hinv_exps() : nullptr;
     w.grown = w.hinv ? hinv_grown() : nullptr;
-    const bool tc = w.hinv && 64 * (long long)hblocks.size() > wave_nsmall;
-    w.ctas_per_sm = 2 * wave_nsmall > wave_nfwd && !tc ? 3 : 2;
+    // Digits for up to four columns only in fronts of five and more pivot
+    // blocks: in smaller ones the multiply-adds take no longer (a solve of three
+    // columns with digits from 1, 3 and 5 blocks on: 6000-row saddle point 1.51,
+    // 1.42, 1.43 ms; 48^3 grid 3.23, 3.17, 3.15; 600^2 grid 2.20, 2.15, 2.14; 320
+    // small grids 2.89, 2.82, 2.76).  By the front and the number of columns
+    // alone, so that a matrix has the same bits alone and in a batch.
+    w.mma_blk = q <= 4 ? 5 : 1;
+    // Three CTAs per SM where small-front items are most of the work, else the
+    // widest fronts' chains set the time and two keep their registers.  The digit
+    // items spill in the registers of three: with them only up to eight columns,
+    // and where the small items are ten times the pivot blocks of the other fronts
+    // and sixteen for each CTA (two and three CTAs, ms: 320 small grids, 30,540
+    // small items to 1,277 blocks, 3 columns 3.67 and 2.86, 8: 5.51 and 4.53, 16:
+    // 9.68 and 9.93; 600^2 grid, 9,969 to 816, 3: 2.14 and 2.03, 8: 2.88 and 2.82,
+    // 16: 4.73 and 5.09; 300^2 grid, 2,505 to 199, 3: 0.89 and 0.99; 30,000-row
+    // saddle point, 2,516 to 290, 4: 7.25 and 8.83).
+    const bool many = wave_nsmall > 10 * (long long)hblocks.size() && wave_nsmall > 16 * 2 * 152;
+    w.ctas_per_sm = 2 * wave_nsmall > wave_nfwd && (!w.hinv || (q <= 8 && many)) ? 3 : 2;
     w.front_group = S->d_front_group;
     w.active = S->d_front_group ? group_active.p : nullptr;
     if (!wave_trace.empty()) {

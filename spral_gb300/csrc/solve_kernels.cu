@@ -219,9 +219,9 @@ __device__ __forceinline__ void solve_in_regs(int jb, const T* Lb, T (&x)[R][2])
 // entries of L up to 1/u) is solved by substitution, its items take
 // fwd_block and bwd_block.
 //
-// One or two columns keep the multiply-adds: the digit work of a tile, padded
-// to eight columns, stays the same while theirs falls (at four columns the two
-// passes of a 6000-row saddle point gain 1.97 -> 1.60 ms only).
+// One or two columns keep the multiply-adds, and up to four in the smaller of
+// these fronts (WaveLevel::mma_blk): the digit work of a tile, padded to eight
+// columns, stays the same while theirs falls.
 // Bound by the chain of pivot blocks at the top of the tree (eight columns:
 // 10 us a block for flag, digits, products of one tile and of the diagonal
 // block; 19 us before) and by the FP64 pipe in the small items below it.
@@ -1284,6 +1284,11 @@ __global__ void __launch_bounds__(64) k_half_inv(const SolveNode<double>* sns, c
   if (threadIdx.x == 0) grown[sn.hoff + w.y] = any ? 1 : 0;
 }
 
+// whether a front's items multiply digits in this pass
+__device__ __forceinline__ bool wave_mma(const SolveNode<double>& sn, const WaveLevel& wl) {
+  return wl.hinv && sn.hoff >= 0 && sn.nblk >= wl.mma_blk;
+}
+
 // fwd_block on the tensor cores
 template <int NR>
 __device__ bool fwd_block_mma(const SolveNode<double>& sn, int code, int nrhs, double* x, int ldx,
@@ -1894,7 +1899,7 @@ __global__ void __launch_bounds__(kSolveThreads, CPS)
       if (ok) {
         bool done = false;
         if constexpr (solve_mma<T, NR>()) {
-          if (wl.hinv && sn.hoff >= 0 && !(code < kWaveContrib && wl.grown[sn.hoff + code])) {
+          if (wave_mma(sn, wl) && !(code < kWaveContrib && wl.grown[sn.hoff + code])) {
             ok = fwd_block_mma<NR>(sn, code, nrhs, x, ldx, scale_sqrt, status, solve_smem, &s_fail,
                                    wl, it);
             done = true;
@@ -2394,7 +2399,7 @@ __global__ void __launch_bounds__(kSolveThreads, CPS)
       if (ok) {
         bool done = false;
         if constexpr (solve_mma<T, NR>()) {
-          if (wl.hinv && sn.hoff >= 0) {
+          if (wave_mma(sn, wl)) {
             bwd_l21_mma<NR>(sn, t, nrhs, solve_smem, wl);
             done = true;
           }
@@ -2419,7 +2424,7 @@ __global__ void __launch_bounds__(kSolveThreads, CPS)
       if (ok) {
         bool done = false;
         if constexpr (solve_mma<T, NR>()) {
-          if (wl.hinv && sn.hoff >= 0 && !wl.grown[sn.hoff + code]) {
+          if (wave_mma(sn, wl) && !wl.grown[sn.hoff + code]) {
             ok = bwd_block_mma<NR>(sn, code, nrhs, x, ldx, status, solve_smem, &s_fail, wl, it);
             done = true;
           }

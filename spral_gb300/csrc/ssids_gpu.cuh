@@ -368,7 +368,7 @@ struct WaveLevel {
   // optional trace (nullptr: off): per item, the global timer when a CTA
   // took it, when its last wait was over, when it finished, and the SM
   unsigned long long* trace;
-  int ctas_per_sm;  // persistent CTAs per SM: 3 when small fronts dominate, else 2
+  int ctas_per_sm;  // persistent CTAs per SM, 2 or 3 (Numeric::wave_pass)
   // optional mask (nullptr: every front): the items of front f run only when
   // active[front_group[f]] != 0; a group is one matrix of a batch stacked as
   // a forest, so the skipped fronts are whole trees that no other item waits
@@ -383,6 +383,7 @@ struct WaveLevel {
   // and per pivot block whether its inverses are too large to multiply by
   const int* hexp;
   const unsigned char* grown;
+  int mma_blk;  // the fronts of this many pivot blocks and more multiply digits
 };
 
 constexpr int kSolveBlk = 64;   // diagonal block of the blocked triangular solves
