@@ -335,8 +335,8 @@ int spral_ssids_gpu_tune_table(int* out, int nout);
 
 /* The scaled backward error of each row group (spral_ssids_gpu_set_row_groups:
  * e.g. the matrices of a batch) after the last refined solve of the handle,
- * the largest over the right-hand sides of its last chunk of 16.  out holds
- * ngroups values.  Returns 0, -1 without row groups or refined solve, -51 on
+ * the largest over the right-hand sides of its last chunk of 16 (infinite for
+ * a group with a NaN or Inf).  out holds ngroups values.  Returns 0, -1 without row groups or refined solve, -51 on
  * a CUDA error.  No reference counterpart. */
 int spral_ssids_gpu_group_bwd_errors(const void* numeric, double* out, int ngroups);
 

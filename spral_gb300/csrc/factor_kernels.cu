@@ -925,7 +925,10 @@ __global__ void __launch_bounds__(kApplyRows) k_app_apply(FrontDesc<float>* fds,
 // Laplacian 22.2 -> 15.9 us a launch, saddle point n = 6000 26.3 -> 10.9 us.
 // ------------------------------------------------------------------------
 constexpr int kApplyF64Threads = 128;
-constexpr int kApplySms = 2 * 152;  // CTAs of 16 rows that run at once without slowing each other
+// CTAs of 16 rows that run at once without slowing each other: two on each of a
+// GB300's 152 SMs (a constant, so that the variant, whose sums are the same, does
+// not cost a device query per launch)
+constexpr int kApplySms = 2 * 152;
 
 template <int RP>
 __global__ void __launch_bounds__(kApplyF64Threads)
@@ -1610,32 +1613,36 @@ __global__ void k_app_finish(FrontDesc<T>* fds, FrontState* sts, const int* fron
 
 // ------------------------------------------------------------------------
 // k_tpp: threshold partial pivoting on the failed columns [nelim, n)
-// (ldlt_tpp.cxx:166-270).  One CTA per front; FP64 arithmetic.
+// (ldlt_tpp.cxx:166-270) by tpp_fast, one CTA per front, in place.
 // ------------------------------------------------------------------------
 constexpr int kTppThreads = 256;
 // threads of k_tpp on tall FP32 fronts: its one CTA per front scans and updates
 // lines of global memory, bound by their latency (seven fronts of some 7,000
 // rows: 3.0 ms with 256 threads, 0.95 with 1,024; FP64 is bound by the SM's
 // FP64 pipe and gains nothing)
+// (Both types are compiled for 1,024 threads, 64 registers each; k_tpp<double>,
+// which always runs 256, spills 32 bytes under that bound, none under its own.)
 constexpr int kTppTallThreads = 1024;
 
-
 // ------------------------------------------------------------------------
-// k_tpp_small: the fronts of small leaf subtrees, factored with TPP from
-// their first column as the reference's CPU path does for every node of a
-// subtree below small_subtree_threshold flops (SymbolicSubtree.hxx:56-82;
+// TPP (tpp_fast): the failed columns of APP fronts (k_tpp) and, from their
+// first column, the fronts of small leaf subtrees (k_tpp_level), as the
+// reference's CPU path does for every node of a subtree below
+// small_subtree_threshold flops (SymbolicSubtree.hxx:56-82;
 // SmallLeafNumericSubtree.hxx:345-375 calls ldlt_tpp_factor on the whole
-// front).  One CTA per front, the front (m x n), two workspace columns and
-// its perm/opos held in shared memory.  The TPP itself (tpp_fast, which
-// k_tpp also runs on the failed columns of APP fronts): each pivot, warp 0
-// alone runs the pivot search of ldlt_tpp_factor (ldlt_tpp.cxx:166-270;
-// every reduction a warp shuffle), performs the symmetric swaps, writes
-// D^{-1} and keeps unscaled copies of the pivot column(s); after one barrier
-// every warp scales the pivot column(s) and updates the trailing
-// fully-summed columns (rows of the front's contribution part included);
-// one more barrier ends the pivot.  A front too large for the launch's
-// shared memory (delays can grow one) is factored the same way in global
-// memory.  step = 0 records that no APP pass ran.
+// front).  Per pivot:
+//   * the search of ldlt_tpp_factor (ldlt_tpp.cxx:166-270).  The first
+//     candidate is examined by warp 0, which shares its verdict through shared
+//     memory, or by all warps where more than kTppWideRows rows are left; the
+//     others, when it is not taken, by all warps (decide_cta; a CTA of one warp:
+//     decide_rest).  FP64 verdicts come from FP32 where no rounding could
+//     decide;
+//   * a barrier wherever all warps read pivot entries from the front, so that
+//     each has its verdict before an entry changes;
+//   * warp 0 swaps, writes D^{-1} and keeps unscaled copies of the pivot
+//     column(s); a barrier; every warp scales the pivot column(s); a barrier;
+//     every warp updates the trailing fully-summed columns (rows of the front's
+//     contribution part included); a barrier ends the pivot.
 // ------------------------------------------------------------------------
 namespace tpps {
 // kTwoRaw: an accepted 2x2 whose D^{-1} is still to be formed (FP64 factors);
@@ -2355,12 +2362,13 @@ __global__ void __launch_bounds__(kTppTallThreads) k_tpp(FrontDesc<T>* fds, Fron
 // i = blockIdx.x, blockIdx.x + gridDim.x, ... of the class's list (largest
 // first); per front: the TPP factorisation (in shared memory when the front
 // fits the launch's dynamic shared memory, else in place in global memory),
-// then, fused, the front's contribution: LD = L21 D (the front's LD
-// workspace) and C -= L21 LD^T on the lower triangle of its contribution
-// block, warp per column of C and lane per row, k in increasing order.  So
-// a level set of small fronts takes one or two launches instead of a TPP
-// launch, an LD launch and a contribution launch, and small fronts run many
-// CTAs per SM (the tiny class launches one warp per CTA).
+// then, fused, LD = L21 D (FP64: into the front's LD workspace) and, for FP32
+// factors, C -= L21 LD^T on the lower triangle of its contribution block; FP64
+// factors leave that to k_small_contrib_f64, one launch after each class's.  So a
+// level set of small fronts takes one or two launches per size class (up to
+// six, on side streams) instead of a TPP launch, an LD launch and a
+// contribution launch, and small fronts run many CTAs per SM (the tiny class
+// launches one warp per CTA).  step = 0 records that no APP pass ran.
 // ------------------------------------------------------------------------
 // alpha = x / det, beta = -b / det of the 2x2 block with determinant det = x y -
 // b^2: by the reciprocal where that is a normal number, else from the block
@@ -2415,17 +2423,15 @@ __device__ __forceinline__ void d_column_raw(const double* D, int c, int nel, fl
 // the fused contribution of one front whose factor is at S (leading
 // dimension ldS); all threads of the CTA.  Column c of D, (alpha, beta,
 // partner), is formed once per column into shared memory: FP64 factors
-// from D^{-1} (d_column, FP64 divisions), FP32 factors from the recorded
+// from D^{-1} (d_column), FP32 factors from the recorded
 // pivot blocks (d_column_raw, before tpp_finish_d) with LD in FP32
 // arithmetic (compensated for 2x2 columns), so the FP32 contribution issues
 // no FP64 instruction per entry.  LD goes to ldsm (shared memory, cm x nel)
 // when given, else to the front's LD workspace.  C -= L21 LD^T on the lower
-// triangle: FP32 factors in 32 x 16 tiles, one per warp at a time, lane
-// (lr, lc) = (lane % 8, lane / 8) holding rows lr + 8i and columns lc + 4j,
-// i, j < 4, so each k takes 8 loads for 16 FMAs; FP64 factors a warp per
-// column and a lane per row (their FMAs, not the loads, bound it, and the
-// tile's registers would cost a CTA per SM).  Either way every entry sums
-// its products in increasing k, one FMA each.
+// triangle for FP32 factors (FP64: k_small_contrib_f64), in 32 x 16 tiles, one
+// per warp at a time, lane (lr, lc) = (lane % 8, lane / 8) holding rows lr + 8i
+// and columns lc + 4j, i, j < 4, so each k takes 8 loads for 16 FMAs; every
+// entry sums its products in increasing k, one FMA each.
 template <typename T>
 __device__ void tpp_front_contrib(const FrontDesc<T>& fd, const T* S, int ldS, int nel, T* ldsm) {
   const int n = fd.n, cm = fd.m - fd.n;
@@ -2974,7 +2980,7 @@ void launch_tpp(FrontDesc<T>* fd, FrontState* st, const int* fronts, int nf, int
   { k_tpp<T><<<nf, threads, 0, s>>>(fd, st, fronts, action, u, small, all_fronts); note_launches(1); }
 }
 
-// Largest dynamic shared memory of k_tpp_small: the fronts of small leaf
+// Largest dynamic shared memory of k_tpp_level: the fronts of small leaf
 // subtrees hold m * n < ~26k entries (their flops are below 4e6), about
 // 205 KB in FP64.
 // dynamic shared memory ceiling of k_tpp_level: the 227 KB per CTA less its

@@ -1277,8 +1277,6 @@ struct Numeric : NumericBase {
     slice_enqueue(b, slice_tab.p, s);
   }
 
-  // shared-memory staging of a small leaf front (k_tpp_small): the front,
-  // two workspace columns, perm and opos, bytes
   // shared memory of a front in k_tpp_level: the front with two workspace
   // columns, perm and opos, then (FP32 factors, 16-byte aligned) its LD
   // block for the fused contribution

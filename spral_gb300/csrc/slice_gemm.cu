@@ -13,8 +13,8 @@
 //   * every row of A and of B is scaled by a power of two so that its
 //     largest entry lies in [1/2, 1), truncated to a 62-bit integer and cut
 //     into kSlices = 8 balanced base-256 digits in [-128, 128], each exact in
-//     FP16.  Entries within a factor 2^10 of the row's largest keep all 53
-//     bits;
+//     FP16.  Entries within a factor 2^9 of the row's largest keep all 53
+//     bits, smaller ones what is left of the 62;
 //   * the digit products of equal weight (levels l = 0..7 of the two digits'
 //     indices) are summed by tcgen05.mma in FP32 accumulators in TMEM.  A
 //     product is at most 2^14 and a level has at most 8 of them per column,
@@ -27,11 +27,16 @@
 // about 2^-62 sqrt(K) of (row maximum of A) x (row maximum of B) in all; an
 // FP64 accumulation over K columns loses about 2^-54 sqrt(K) of the size of
 // its partial sums.  (Seven digits, 2^-55, were up to three times less exact
-// than FP64 on rows whose entries spread over e^6.)  Columns are balanced before that: column k of A is
-// multiplied by 2^h and column k of B divided by it, 2^h ~ sqrt|D_k|, so
-// both rows are those of L sqrt|D| and the loss follows a diagonal scaling of
-// the matrix exactly.  The result of an entry depends on nothing but its two
-// rows, so a front gives the same bits alone and in a batch.
+// than FP64 on rows whose entries spread over e^6.)  Columns are balanced before
+// that: column k of A is multiplied by 2^h and column k of B divided by it, 2^h
+// ~ sqrt|D_k| (slice_balance), so both rows are those of L sqrt|D| and the loss
+// follows a diagonal scaling of the matrix, exactly for 1x1 pivots; the two
+// columns of a 2x2 pivot without diagonal entries share a scale.  The loss
+// goes by the size of two rows of L sqrt|D|, as the error bound of a
+// factorisation does, and lies below that bound; a C(r, c) far smaller than
+// both keeps fewer bits than multiply-adds would leave it.  The result of an
+// entry depends on nothing but its two rows, so a front gives the same bits
+// alone and in a batch.
 //
 // Bound: 36 FP16 products of 16 columns per tile (128 x 64, so that the eight
 // level accumulators fit the 512 TMEM columns) at 6 KiB of shared-memory

@@ -223,12 +223,13 @@ __device__ __forceinline__ void solve_in_regs(int jb, const T* Lb, T (&x)[R][2])
 // these fronts (WaveLevel::mma_blk): the digit work of a tile, padded to eight
 // columns, stays the same while theirs falls.
 // Bound by the chain of pivot blocks at the top of the tree (eight columns:
-// 10 us a block for flag, digits, products of one tile and of the diagonal
-// block; 19 us before) and by the FP64 pipe in the small items below it.
-// 57^3 Laplacian, 16 columns: forward 7.2 -> 3.6 ms, backward 8.5 -> 4.0 ms a
-// pass (fronts of 4 and more pivot blocks only: 4.3 and 5.0; of 2 and more:
-// 3.8 and 4.3).  Six matrices each of five kinds, 16 columns: errors 0.47 to
-// 0.86 of those of the multiply-adds, which round every product.
+// 12 us a block for flag, digits, products of one tile and of the diagonal
+// block; 19 us with multiply-adds) and by the FP64 pipe in the small items below
+// it.  57^3 Laplacian, 16 columns, without the three rules: forward 7.2 -> 3.6
+// ms, backward 8.5 -> 4.0 ms a pass (fronts of 4 and more pivot blocks only: 4.3
+// and 5.0; of 2 and more: 3.8 and 4.3); the rules add 11%.  Eight 48^3 and eight
+// 57^3 matrices, four saddle points, 16, 16 and 4 columns: errors 0.41, 0.46 and
+// 0.36 of those of the multiply-adds, which round every product.
 // 48^3 Laplacian, 8 random columns, a solve: 3.29 ms with neither of the three,
 // 3.51 with (1) and (3), 3.64 with (2) as well (3.52 with kSumGuard 16; a
 // 6000-row saddle point, 4 columns: 1.30, 1.39, 1.59, 1.48).

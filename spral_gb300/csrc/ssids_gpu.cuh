@@ -180,11 +180,12 @@ template <typename T>
 void launch_tpp(FrontDesc<T>* fd, FrontState* st, const int* fronts, int nf, int max_m,
                 bool action, double u, double small, bool root_only_or_all, cudaStream_t s);
 // fronts of small leaf subtrees, one persistent launch: TPP from the first
-// column, then each front's contribution block (LD and C -= L21 LD^T);
-// max_bytes is the dynamic shared memory of the launch (fronts whose
-// staging, ((m + 1) & ~1) * (n + 2) * sizeof(T) + 8 n bytes, exceeds it
-// are factored in place); threads: 32 (one warp per front) or 256; max_cm:
-// the largest contribution block
+// column, then each front's contribution block (LD and C -= L21 LD^T; FP64
+// factors the product in a second launch); max_bytes is the dynamic shared
+// memory of the launch (fronts whose staging, ((m + 1) & ~1) * (n + 2) *
+// sizeof(T) + 8 n bytes, exceeds it are factored in place); threads per front:
+// 32, 64 or 256, raised to 128 where the level has no more fronts than the GPU
+// has SMs; max_cm: the largest contribution block
 template <typename T>
 void launch_tpp_level(FrontDesc<T>* fd, FrontState* st, const int* fronts, int nf, bool action,
                       double u, double small, int max_bytes, int threads, int max_cm,
